@@ -10,6 +10,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -17,7 +18,7 @@ LIB = os.path.join(HERE, "libcatabra_b200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = os.environ.get("NVCC", "nvcc")
 
-DEVICE_SOURCES = ["kernels.cu", "queue.cu", "noalloc.cu", "tables.cu", "real.cu"]
+DEVICE_SOURCES = ["kernels.cu", "queue.cu", "passes32.cu", "passes64.cu", "noalloc.cu", "tables.cu", "real.cu"]
 HOST_SOURCES = ["plan.cpp"]
 
 
@@ -63,13 +64,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     os.makedirs(os.path.join(HERE, "_build"), exist_ok=True)
     common = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-I", CSRC]
-    for s in todo:
+    def compile_one(s: str) -> None:
         cmd = [NVCC, *ARCH, *common, "-c", os.path.join(CSRC, s), "-o", _obj(s)]
         if s in DEVICE_SOURCES:
             cmd.insert(3, "-lineinfo")
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
         subprocess.run(cmd, check=True)
+
+    # one nvcc per source, a few at a time (the generic kernels take minutes each)
+    with ThreadPoolExecutor(min(8, os.cpu_count() or 1)) as ex:
+        list(ex.map(compile_one, todo))
     objs = [_obj(s) for s in DEVICE_SOURCES + HOST_SOURCES]
     tmp = LIB + ".tmp"
     subprocess.run([NVCC, *ARCH, "-shared", "-o", tmp, *objs, "-lcudart"], check=True)

@@ -2,15 +2,13 @@
 //
 // One transform (or a tile of sub-transforms) is staged in shared memory and
 // every radix pass runs there; HBM is touched once on the way in and once on
-// the way out.  Four work shapes share the same in-place Stockham core:
+// the way out.  Two work shapes share the same in-place Stockham core:
 //
 //   ROWS     V whole transforms per CTA (small n), one row each.
 //   FOUR     one transform of length M = N1*N2 split over a thread-block
 //            cluster of C CTAs: column FFTs (length N1) in each CTA, twiddle
 //            w_M^(i2*k1), exchange through distributed shared memory, row
 //            FFTs (length N2).  C = 1 is the single-CTA four-step.
-//   COLPASS  / ROWPASS: the two HBM passes of the four-step for lengths that
-//            exceed a cluster (tiles of adjacent columns / rows).
 //
 // Rader (prime n) and Bluestein (other non-smooth n) are fused into ROWS and
 // FOUR: the prologue builds the zero-padded convolution input (generator
@@ -144,10 +142,6 @@ template <> __device__ __forceinline__ float2 store_out<float2>(const KParams& p
 __device__ __forceinline__ int fdiv(unsigned n, unsigned long long m) {
     return (int)(((unsigned long long)n * m) >> 40);
 }
-__device__ __forceinline__ unsigned long long fdiv_magic(int d) {
-    return ((1ULL << 40) + (unsigned long long)d - 1) / (unsigned long long)d;
-}
-
 // ------------------------------------------------ asynchronous global->smem
 // cp.async (sm_80+ LDGSTS): the copy lands in shared memory without passing
 // through registers, so the next transform's input streams in while the
@@ -1086,186 +1080,21 @@ __device__ __forceinline__ void four_body(const KParams& p, unsigned char* smem)
     four_transform<V, EMAX, K>(p, buf, bufC, nullptr, xs, red, twA, twC, t4, t, -1, c);
 }
 
-// ------------------------------------------------------- COLPASS / ROWPASS
-// COLPASS: tile of V adjacent columns c0..c0+V of the N1 x N2 view of one
-// transform; column FFTs; store the w^(i2 k1)-scaled result to scratch
-// row-major.  ROWPASS: tile of V adjacent rows r0..r0+V of the scratch; row
-// FFTs; store X[k1 + N1 k2] (natural order), optionally with the Bluestein
-// epilogue.  A tile streams into shared memory with cp.async (all of its
-// copies in flight at once); pre-multiplications (conjugation, chirp,
-// spectrum) are applied in shared memory once it has arrived.  The
-// sub-transform twiddle table is staged in shared memory when small.
+// ---- batched entry points: each block finds its parameter block, stages it
+// in shared memory with the launch's base pointers and direction applied, and
+// runs the same body as the single-plan kernels.
 template <typename V>
-__device__ __forceinline__ void colpass_issue(const KParams& p, int tile, V* dst) {
-    const int T = blockDim.x, tid = opaque_tid();
-    const int tiles = p.N2 / p.V, t = tile / tiles, c0 = (tile - t * tiles) * p.V;
-    const int N1 = p.N1, N2 = p.N2, Vw = p.V, PA = p.PA;
-    const long long lim = (p.pre == PRE_CHIRP) ? (long long)p.nx : (1LL << 62);
-    // the first ks Vw threads (ks = T / Vw) each take one column j of the
-    // tile, rows i1 = k0, k0 + ks, ...: no per-element division; a warp
-    // still reads runs of Vw consecutive elements of consecutive rows
-    const int ks = T / Vw;
-    if (tid >= ks * Vw) return;
-    const int j = tid % Vw, k0 = tid / Vw;
-    if (p.in_fmt == IO_PLAIN) {
-        const V* in = (const V*)p.in + (long long)t * p.in_dist + c0 + j;
-        for (int i1 = k0; i1 < N1; i1 += ks) {
-            const long long jj = (long long)i1 * N2 + c0 + j;
-            if (jj < lim) cp_async_elem(dst + i1 * PA + j, in + (long long)i1 * N2);
-        }
-    } else {
-        for (int i1 = k0; i1 < N1; i1 += ks) {
-            const long long jj = (long long)i1 * N2 + c0 + j;
-            if (jj < lim) dst[i1 * PA + j] = user_ld<V>(p, t, jj);
-        }
+__device__ __forceinline__ const KParams& stage_params(const BatchLaunch& L, KParams* sp) {
+    if (threadIdx.x == 0) {
+        KParams p = L.desc[L.block_desc[blockIdx.x]];
+        if (p.in_user) p.in = (const V*)L.in_base + p.in_off;
+        if (p.out_user) p.out = (V*)L.out_base + p.out_off;
+        if (L.dir >= 0) {                 // one direction for the launch
+            p.dir = L.dir;
+            if (L.dir != 1) p.scale = 1.0;
+        }                                 // else: per-block direction and scale
+        *sp = p;
     }
-}
-// prologue on the arrived tile; returns whether it wrote (caller syncs)
-template <typename V>
-__device__ __forceinline__ bool colpass_fix(const KParams& p, int tile, V* buf) {
-    if (p.pre == PRE_NONE && !p.dir) return false;
-    const int T = blockDim.x, tid = opaque_tid();
-    const int tiles = p.N2 / p.V, t = tile / tiles, c0 = (tile - t * tiles) * p.V;
-    const int N1 = p.N1, N2 = p.N2, Vw = p.V, PA = p.PA;
-    // one column per thread, as in colpass_issue (the caller synchronises)
-    const int ks = T / Vw;
-    if (tid >= ks * Vw) return true;
-    const int j = tid % Vw;
-#pragma unroll 4
-    for (int i1 = tid / Vw; i1 < N1; i1 += ks) {
-        const long long jj = (long long)i1 * N2 + c0 + j;
-        V* e = buf + i1 * PA + j;
-        if (p.pre == PRE_NONE) {
-            *e = conjv(*e);
-        } else if (p.pre == PRE_CHIRP) {
-            *e = (jj < p.nx) ? fromd<V>(cmul(tod(load_in(p, *e)), __ldg(p.chirp + jj))) : zero<V>();
-        } else {
-            *e = conjv(fromd<V>(cmul(tod(*e), __ldg(p.spec + jj))));
-        }
-    }
-    return true;
-}
-// column FFTs and the twiddled store; (c0 + j) * k1 < N2 * N1 = M, so the
-// exponent needs no reduction
-template <typename V, int EMAX>
-__device__ __forceinline__ void colpass_finish(const KParams& p, int tile, V* buf, const V* tw,
-                                               const TwoLevel& t4) {
-    const int T = blockDim.x, tid = opaque_tid();
-    const int tiles = p.N2 / p.V, t = tile / tiles, c0 = (tile - t * tiles) * p.V;
-    V* out = (V*)p.out + (long long)t * p.out_dist;
-    const int N1 = p.N1, N2 = p.N2, Vw = p.V, PA = p.PA;
-    run_subffts<V, EMAX, 2>(buf, p.pa, tw, Vw, PA, 1);
-    // the first ks Vw threads (ks = T / Vw; all of them when Vw divides T)
-    // each keep one column: no per-element division, and the twiddles
-    // w^(c k1), k1 = k0, k0 + ks, ..., are FP64 products with the step
-    // w^(c ks), re-seeded from the table every 16 steps (the error stays near
-    // 1e-15; the same FP64 work per element as a table product, a sixteenth
-    // of its table reads)
-    const int ks = T / Vw;
-    if (tid < ks * Vw) {
-        const int j = tid % Vw, k0 = tid / Vw;
-        const unsigned c = (unsigned)(c0 + j);
-        V* o = out + c0 + j;
-        const double2 st = tw_two(t4, c * (unsigned)ks);
-        double2 w = make_double2(1, 0);
-        int i = 0;
-#pragma unroll 4
-        for (int k1 = k0; k1 < N1; k1 += ks, i++) {
-            if ((i & 15) == 0) w = tw_two(t4, c * (unsigned)k1);
-            o[(long long)k1 * N2] = cmul(buf[k1 * PA + j], fromd<V>(w));
-            w = cmul(w, st);
-        }
-    }
-}
-
-template <typename V>
-__device__ __forceinline__ void rowpass_issue(const KParams& p, int tile, V* dst) {
-    const int T = blockDim.x, tid = opaque_tid();
-    const int tiles = p.N1 / p.V, t = tile / tiles, r0 = (tile - t * tiles) * p.V;
-    const int N2 = p.N2, PC = p.PC;
-    const V* src = (const V*)p.in + (long long)t * p.in_dist + (long long)r0 * N2;
-    for (int idx = tid; idx < p.V * N2; idx += T) {
-        const int r = fdiv(idx, p.mN2), i2 = idx - r * N2;
-        cp_async_elem(dst + r * PC + i2, src + idx);
-    }
-}
-template <typename V, int EMAX>
-__device__ __forceinline__ void rowpass_finish(const KParams& p, int tile, V* buf, const V* tw) {
-    const int T = blockDim.x, tid = opaque_tid();
-    const int tiles = p.N1 / p.V, t = tile / tiles, r0 = (tile - t * tiles) * p.V;
-    V* out = (V*)p.out + (long long)t * p.out_dist;
-    const int N1 = p.N1, N2 = p.N2, Vw = p.V, PC = p.PC;
-    run_subffts<V, EMAX, 2>(buf, p.pc, tw, Vw, 1, PC);
-    // the first ks Vw threads (ks = T / Vw) each store one row r of the
-    // tile, k2 = k0, k0 + ks, ...: no per-element division; a warp still
-    // writes runs of Vw consecutive outputs
-    const int ks = T / Vw;
-    if (tid >= ks * Vw) return;
-    const int r = tid % Vw, k0 = tid / Vw;
-    if (p.out_fmt != IO_PLAIN) {
-        // the caller's strided or ComplexF16 layout (the last stage of a fused plan)
-        for (int k2 = k0; k2 < N2; k2 += ks) {
-            const long long k = (long long)(r0 + r) + (long long)N1 * k2;
-            const V v = buf[r * PC + k2];
-            if (p.post == POST_CHIRP) {
-                if (k < p.nx) user_st(p, t, k, store_out(p, fromd<V>(cmul(tod(conjv(v)), __ldg(p.chirp + k)))));
-            } else {
-                user_st(p, t, k, store_out(p, v));
-            }
-        }
-        return;
-    }
-#pragma unroll 4
-    for (int k2 = k0; k2 < N2; k2 += ks) {
-        const long long k = (long long)(r0 + r) + (long long)N1 * k2;
-        V v = buf[r * PC + k2];
-        if (p.post == POST_CHIRP) {
-            if (k < p.nx) stg_stream(out + k, store_out(p, fromd<V>(cmul(tod(conjv(v)), __ldg(p.chirp + k)))));
-        } else if (p.post == POST_RAW) {
-            out[k] = v;                       // intermediate of a convolution
-        } else {
-            stg_stream(out + k, store_out(p, v));
-        }
-    }
-}
-
-// one tile per CTA
-template <typename V, int EMAX>
-__device__ __forceinline__ void colpass_body(const KParams& p, unsigned char* smem) {
-    const int T = blockDim.x, tid = opaque_tid();
-    const int tile = block_id(p);
-    if (tile >= p.batch * (p.N2 / p.V)) return;
-    const int lt = cfft_pass_tw_elems(p.pa.twlen, (int)sizeof(V));
-    const int nt = cfft_pass_t4_elems(p.t4.bits, p.t4.N), nlo = 1 << p.t4.bits;
-    V* tws = (V*)smem;
-    double2* t4s = after16(tws + lt);
-    V* buf = (V*)(t4s + nt);
-    colpass_issue<V>(p, tile, buf);
-    cp_async_commit();
-    for (int i = tid; i < lt; i += T) tws[i] = ((const V*)p.pa.tw)[i];
-    for (int i = tid; i < nt; i += T) t4s[i] = (i < nlo) ? p.t4.lo[i] : p.t4.hi[i - nlo];
-    TwoLevel t4 = p.t4;
-    if (nt) {
-        t4.lo = t4s;
-        t4.hi = t4s + nlo;
-    }
-    cp_async_wait_all();
     __syncthreads();
-    if (colpass_fix<V>(p, tile, buf)) __syncthreads();
-    colpass_finish<V, EMAX>(p, tile, buf, lt ? (const V*)tws : (const V*)p.pa.tw, t4);
-}
-template <typename V, int EMAX>
-__device__ __forceinline__ void rowpass_body(const KParams& p, unsigned char* smem) {
-    const int T = blockDim.x, tid = opaque_tid();
-    const int tile = block_id(p);
-    if (tile >= p.batch * (p.N1 / p.V)) return;
-    const int lt = cfft_pass_tw_elems(p.pc.twlen, (int)sizeof(V));
-    V* tws = (V*)smem;
-    V* buf = tws + lt;
-    rowpass_issue<V>(p, tile, buf);
-    cp_async_commit();
-    for (int i = tid; i < lt; i += T) tws[i] = ((const V*)p.pc.tw)[i];
-    cp_async_wait_all();
-    __syncthreads();
-    rowpass_finish<V, EMAX>(p, tile, buf, lt ? (const V*)tws : (const V*)p.pc.tw);
+    return *sp;
 }

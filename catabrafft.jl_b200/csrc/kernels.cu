@@ -31,40 +31,6 @@ __global__ void __launch_bounds__(CFFT_THREADS, MB) k_four_mb(KParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     four_body<V, EMAX, K>(p, smem);
 }
-// the pass kernels keep three ComplexF32 CTAs resident per SM (80 registers
-// suffice for their radix-16 codelets)
-template <typename V> struct PassBlocks { static constexpr int value = 3; };
-template <> struct PassBlocks<double2> { static constexpr int value = 2; };
-
-template <typename V, int EMAX>
-__global__ void __launch_bounds__(CFFT_THREADS, PassBlocks<V>::value) k_colpass(KParams p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    colpass_body<V, EMAX>(p, smem);
-}
-template <typename V, int EMAX>
-__global__ void __launch_bounds__(CFFT_THREADS, PassBlocks<V>::value) k_rowpass(KParams p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    rowpass_body<V, EMAX>(p, smem);
-}
-
-// ---- batched entry points: each block finds its parameter block, stages it
-// in shared memory with the launch's base pointers and direction applied, and
-// runs the same body as the single-plan kernels.
-template <typename V>
-__device__ __forceinline__ const KParams& stage_params(const BatchLaunch& L, KParams* sp) {
-    if (threadIdx.x == 0) {
-        KParams p = L.desc[L.block_desc[blockIdx.x]];
-        if (p.in_user) p.in = (const V*)L.in_base + p.in_off;
-        if (p.out_user) p.out = (V*)L.out_base + p.out_off;
-        if (L.dir >= 0) {                 // one direction for the launch
-            p.dir = L.dir;
-            if (L.dir != 1) p.scale = 1.0;
-        }                                 // else: per-block direction and scale
-        *sp = p;
-    }
-    __syncthreads();
-    return *sp;
-}
 template <typename V, int EMAX>
 __global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) kb_rows(BatchLaunch L) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -78,35 +44,20 @@ __global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) kb_four(Bat
     four_body<V, EMAX, K>(stage_params<V>(L, &sp), smem);
 }
 
-template <typename V, int EMAX>
-__global__ void __launch_bounds__(CFFT_THREADS, PassBlocks<V>::value) kb_colpass(BatchLaunch L) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ KParams sp;
-    colpass_body<V, EMAX>(stage_params<V>(L, &sp), smem);
-}
-template <typename V, int EMAX>
-__global__ void __launch_bounds__(CFFT_THREADS, PassBlocks<V>::value) kb_rowpass(BatchLaunch L) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ KParams sp;
-    rowpass_body<V, EMAX>(stage_params<V>(L, &sp), smem);
-}
-
 const void* cfft_batch_kernel_for(int mode, int dtype) {
+    if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS)
+        return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, true) : cfft_pass_kernel32(mode, true);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {
             case MODE_ROWS: return (const void*)kb_rows<double2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)kb_four<double2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)kb_four<double2, CFFT_EMAX, DynK<1>>;
-            case MODE_COLPASS: return (const void*)kb_colpass<double2, CFFT_EMAX>;
-            case MODE_ROWPASS: return (const void*)kb_rowpass<double2, CFFT_EMAX>;
         }
     } else {
         switch (mode) {
             case MODE_ROWS: return (const void*)kb_rows<float2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)kb_four<float2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)kb_four<float2, CFFT_EMAX, DynK<1>>;
-            case MODE_COLPASS: return (const void*)kb_colpass<float2, CFFT_EMAX>;
-            case MODE_ROWPASS: return (const void*)kb_rowpass<float2, CFFT_EMAX>;
         }
     }
     return nullptr;
@@ -505,21 +456,19 @@ int cfft_mixc_lookup(long long n, int dtype, int variant, const void** fn, int* 
 }
 
 const void* cfft_kernel_for(int mode, int dtype) {
+    if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS)
+        return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, false) : cfft_pass_kernel32(mode, false);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {
             case MODE_ROWS: return (const void*)k_rows<double2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)k_four<double2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)k_four<double2, CFFT_EMAX, DynK<1>>;
-            case MODE_COLPASS: return (const void*)k_colpass<double2, CFFT_EMAX>;
-            case MODE_ROWPASS: return (const void*)k_rowpass<double2, CFFT_EMAX>;
         }
     } else {
         switch (mode) {
             case MODE_ROWS: return (const void*)k_rows<float2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)k_four<float2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)k_four<float2, CFFT_EMAX, DynK<1>>;
-            case MODE_COLPASS: return (const void*)k_colpass<float2, CFFT_EMAX>;
-            case MODE_ROWPASS: return (const void*)k_rowpass<float2, CFFT_EMAX>;
         }
     }
     return nullptr;

@@ -13,6 +13,10 @@
 
 // generic kernel for a mode, or nullptr
 const void* cfft_kernel_for(int mode, int dtype);
+// the HBM-pass kernels (passes32.cu, passes64.cu): COLPASS, ROWPASS, MIDPASS,
+// for one plan or descriptor driven
+const void* cfft_pass_kernel32(int mode, bool batched);
+const void* cfft_pass_kernel64(int mode, bool batched);
 // statically shaped FOUR kernel matching (N1, N2, C, radix multiplicities), or
 // nullptr; *single (if given) = 1 when it keeps one buffer for both layouts
 const void* cfft_static_four(int dtype, int N1, int N2, int C, const unsigned char* ca,
@@ -99,6 +103,8 @@ cudaError_t cfft_gen_rader_b(double2* b, const int* iperm, long long n, long lon
                              double2 winv, cudaStream_t st);
 cudaError_t cfft_scale(double2* v, long long M, double s, cudaStream_t st);
 cudaError_t cfft_spec_rowmajor(double2* dst, const double2* src, long long N1, long long N2, cudaStream_t st);
+cudaError_t cfft_spec_center(double2* dst, const double2* src, long long N1, const SfPlan& S, double scale,
+                             cudaStream_t st);
 // real-input transforms (real.cu)
 cudaError_t cfft_r2c_post(void* out, long long N, long long n, long long batch, long long dist, int dtype,
                           cudaStream_t st);

@@ -36,6 +36,7 @@
 #include "../../include/catabra_b200.h"
 #include "engine_types.h"
 #include "kernels.h"
+#include "passplan.h"
 
 static constexpr size_t kScratchBytes = 32u << 20;   // intermediate between the passes
 static constexpr size_t kTableBytes = 256u << 10;    // sub-transform + four-step twiddles
@@ -74,79 +75,26 @@ __device__ double2 omega_dev(long long m, long long L) {
     sincospi(-2.0 * (double)m / (double)L, &s, &c);
     return make_double2(c, s);
 }
-// per-pass twiddle blocks of one sub-transform (layout of SubPlan.tw)
-struct PassTable {
-    int L, np, twlen;
-    int r[CFFT_MAXP], s[CFFT_MAXP], off[CFFT_MAXP];
-};
+// forward twiddle blocks of both sub-transforms (SfPlan.off) and the two-level table of w_M
 template <typename V>
-__global__ void k_noalloc_tables(V* twA, PassTable A, V* twC, PassTable Cc, double2* lo, int nlo,
-                                 double2* hi, int nhi, int M) {
+__global__ void k_noalloc_tables(V* twA, SfPlan A, V* twC, SfPlan Cc, double2* lo, int nlo, double2* hi, int nhi,
+                                 int M) {
     const int stride = gridDim.x * blockDim.x;
     const int total = max(max(A.twlen, Cc.twlen), max(nlo, nhi));
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         for (int w = 0; w < 2; w++) {
-            const PassTable& T = w ? Cc : A;
+            const SfPlan& T = w ? Cc : A;
             V* dst = w ? twC : twA;
             if (i >= T.twlen) continue;
-            int p = 0;
-            while (p + 1 < T.np && T.off[p + 1] <= i) p++;
-            const int n1 = T.L / (T.s[p] * T.r[p]), k = i - T.off[p];
-            const int j = k / n1 + 1, q = k - (j - 1) * n1;
-            const double2 v = omega_dev((long long)j * q * T.s[p], T.L);
+            long long e;
+            int N;
+            sf_tw_entry(T, i, &e, &N);
+            const double2 v = omega_dev(e, N);
             dst[i] = round_to<V>(v.x, v.y);
         }
         if (i < nlo) lo[i] = omega_dev(i, M);
         if (i < nhi) hi[i] = omega_dev((long long)i * nlo, M);
     }
-}
-
-// greedy radix split (largest codelet first), passes stored in CFFT_EXEC_ORDER
-const int kRad[8] = {16, 9, 8, 7, 5, 4, 3, 2};
-const int kExec[8] = CFFT_EXEC_ORDER;
-bool split_canonical(long long L, SubPlan& sp) {
-    sp.L = (int)L;
-    sp.np = 0;
-    for (int i = 0; i < 8; i++) sp.cnt[i] = 0;
-    long long rem = L;
-    while (rem > 1) {
-        int k = -1;
-        for (int i = 0; i < 8; i++)
-            if (rem % kRad[i] == 0) { k = i; break; }
-        if (k < 0 || sp.np >= CFFT_MAXP) return false;
-        for (int i = 0; i < 8; i++)
-            if (kExec[i] == kRad[k]) sp.cnt[i]++;
-        sp.np++;
-        rem /= kRad[k];
-    }
-    int k = 0;
-    for (int i = 0; i < 8; i++)
-        for (int c = 0; c < sp.cnt[i]; c++) sp.radix[k++] = (unsigned char)kExec[i];
-    // block-wide waves only: G sub-transforms per wave fit 256 threads x 16 elements
-    long long g = 1 << 20;
-    for (int i = 0; i < sp.np; i++) {
-        const int r = sp.radix[i];
-        g = std::min<long long>(g, (long long)CFFT_THREADS * (CFFT_EMAX / r) * r / sp.L);
-    }
-    sp.G = (int)std::max<long long>(1, std::min<long long>(g, 1 << 20));
-    sp.Gwarp = 0;
-    return sp.np == 0 || g >= 1;
-}
-void pass_table(const SubPlan& sp, PassTable& T) {
-    T.L = sp.L;
-    T.np = sp.np;
-    long long s = 1, off = 0;
-    for (int i = 0; i < sp.np; i++) {
-        T.r[i] = sp.radix[i];
-        T.s[i] = (int)s;
-        T.off[i] = (int)off;
-        off += (long long)(sp.radix[i] - 1) * (sp.L / (s * sp.radix[i]));
-        s *= sp.radix[i];
-    }
-    T.twlen = (int)off;
-}
-unsigned long long magic(long long d) {
-    return ((1ULL << 40) + (unsigned long long)d - 1) / (unsigned long long)d;
 }
 }  // namespace
 
@@ -163,18 +111,18 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
                             "n exceeds the fixed scratch (2^21 ComplexF64 / 2^22 ComplexF32 elements)");
     if (((uintptr_t)d_in % e) || ((uintptr_t)d_out % e))
         return noalloc_fail(CFFT_ERR_INVALID, "buffers must be aligned to the element size");
-    // balanced split with both factors <= 4096 and 7-smooth
+    // the planner's split rule (factors <= 4096 and 7-smooth, best score)
     long long N1 = -1;
-    double best = 1e30;
-    SubPlan pa, pc;
+    double best = 1e8;
+    SfPlan pa, pc;
     for (long long a = 2; a <= 4096; a++) {
         if (n % a) continue;
         const long long b = n / a;
         if (b < 2 || b > 4096) continue;
-        SubPlan ta, tc;
-        if (!split_canonical(a, ta) || !split_canonical(b, tc)) continue;
-        const double bal = std::fabs(std::log2((double)a / (double)b));
-        if (bal < best) { best = bal; N1 = a; pa = ta; pc = tc; }
+        SfPlan ta, tc;
+        if (!sf_plan((int)a, ta) || !sf_plan((int)b, tc)) continue;
+        const double sc = sf_pass_cost(ta, b, a, e) + sf_pass_cost(tc, a, sf_qw(tc), e);
+        if (sc < best) { best = sc; N1 = a; pa = ta; pc = tc; }
     }
     if (N1 < 0)
         return noalloc_fail(CFFT_ERR_UNSUPPORTED,
@@ -214,23 +162,18 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
     while ((1LL << (2 * bits)) < n) bits++;
     const int nlo = 1 << bits, nhi = (int)((n + nlo - 1) / nlo + 1);
     unsigned char* tab = arena + kScratchBytes;
-    PassTable TA, TC;
-    pass_table(pa, TA);
-    pass_table(pc, TC);
-    pa.twlen = TA.twlen;
-    pc.twlen = TC.twlen;
     void* twA = tab;
-    void* twC = tab + (size_t)TA.twlen * e;
-    size_t off = (size_t)((TA.twlen + TC.twlen) * e + 255) & ~(size_t)255;
+    void* twC = tab + (size_t)pa.twlen * e;
+    size_t off = (size_t)((pa.twlen + pc.twlen) * e + 255) & ~(size_t)255;
     double2* lo = (double2*)(tab + off);
     double2* hi = lo + nlo;
     if (off + (size_t)(nlo + nhi) * sizeof(double2) > kTableBytes)
         return noalloc_fail(CFFT_ERR_UNSUPPORTED, "twiddle tables exceed the fixed table region");
     if (dtype == CFFT_C128)
-        k_noalloc_tables<double2><<<32, 256, 0, st>>>((double2*)twA, TA, (double2*)twC, TC, lo, nlo, hi,
+        k_noalloc_tables<double2><<<32, 256, 0, st>>>((double2*)twA, pa, (double2*)twC, pc, lo, nlo, hi,
                                                         nhi, (int)n);
     else
-        k_noalloc_tables<float2><<<32, 256, 0, st>>>((float2*)twA, TA, (float2*)twC, TC, lo, nlo, hi,
+        k_noalloc_tables<float2><<<32, 256, 0, st>>>((float2*)twA, pa, (float2*)twC, pc, lo, nlo, hi,
                                                        nhi, (int)n);
     ce = cudaGetLastError();
     if (ce != cudaSuccess) return noalloc_fail(CFFT_ERR_CUDA, "table kernel launch", ce);
@@ -251,27 +194,20 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
     kp.t4.N = (int)n;
     pa.tw = twA;
     pc.tw = twC;
-    const long long PC = N2 + ((N2 % 2 == 0) ? 1 : 0);
-    // the planner's tile rule: widths within the per-CTA shared-memory budget
-    // (staged tables included), power-of-two widths preferred
-    long long Vc = 1, Vr = 1;
-    cfft_pass_tiles(N1, N2, PC, pa.twlen, pc.twlen, bits, (int)n, e, &Vc, &Vr);
+    kp.sa = pa;
+    kp.sc = pc;
+    kp.qp = sf_qp(pc);
+    kp.qw = sf_qw(pc);
     KParams col = kp, row = kp;
     col.mode = MODE_COLPASS;
-    col.V = (int)Vc;
-    col.PA = (int)Vc;
-    col.pa = pa;
-    col.mV = magic(Vc);
+    col.V = sf_tile(N2, N1, e);
+    col.lw = sf_lg(col.V);
     col.pre = PRE_NONE;
+    col.post = POST_TWIDDLE;
     row.mode = MODE_ROWPASS;
-    row.V = (int)Vr;
-    row.PC = (int)PC;
-    row.pc = pc;
-    row.mV = magic(Vr);
-    row.mN2 = magic(N2);
-    row.post = POST_OUT;
-    const size_t smem_col = cfft_colpass_smem(pa.twlen, bits, (int)n, (int)(N1 * Vc), (int)e);
-    const size_t smem_row = (size_t)(cfft_pass_tw_elems(pc.twlen, (int)e) + Vr * PC) * e + 16;
+    row.V = sf_tile(N1, kp.qw, e);
+    row.lw = sf_lg(row.V);
+    const size_t smem_col = sf_col_smem(pa, col.V, e), smem_row = sf_row_smem(pc, row.V, e);
 
     const long long chunk = std::max<long long>(1, (long long)(kScratchBytes / ((size_t)n * e)));
     for (long long b0 = 0; b0 < batch; b0 += chunk) {
@@ -285,9 +221,9 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
         row.out = (char*)d_out + (size_t)b0 * n * e;
         row.in_dist = n;
         row.out_dist = n;
-        ce = cfft_launch_fn(fcol, col, (unsigned)(nb * (N2 / Vc)), CFFT_THREADS, smem_col, 1, st);
+        ce = cfft_launch_fn(fcol, col, (unsigned)(nb * ((N2 + col.V - 1) / col.V)), CFFT_THREADS, smem_col, 1, st);
         if (ce == cudaSuccess)
-            ce = cfft_launch_fn(frow, row, (unsigned)(nb * (N1 / Vr)), CFFT_THREADS, smem_row, 1, st);
+            ce = cfft_launch_fn(frow, row, (unsigned)(nb * ((N1 + row.V - 1) / row.V)), CFFT_THREADS, smem_row, 1, st);
         if (ce != cudaSuccess) return noalloc_fail(CFFT_ERR_CUDA, "kernel launch", ce);
     }
     return CFFT_OK;

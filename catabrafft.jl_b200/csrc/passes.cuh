@@ -1,0 +1,400 @@
+// passes.cuh -- the HBM passes of lengths that exceed a CTA (or cluster):
+//
+//   COLPASS  a tile of V adjacent columns of the N1 x N2 view of a transform:
+//            N1-point DFTs down the columns, then either the four-step
+//            twiddle w_M^(c k1) into the intermediate (POST_TWIDDLE) or the
+//            Bluestein chirp into the caller's output (POST_CHIRP)
+//   ROWPASS  a tile of V adjacent rows of the intermediate: N2-point DFTs,
+//            X[k1 + N1 k2] into the caller's output
+//   MIDPASS  the middle of a convolution, in place on V rows of the
+//            intermediate: N2-point DFT, product with the FP64 spectrum,
+//            conjugation, N2-point DFT that takes the digits in reverse
+//            order, four-step twiddle w_M^(k1 j2)
+//
+// A smooth length is COLPASS + ROWPASS; a Bluestein convolution is COLPASS
+// (chirp) + MIDPASS + COLPASS (chirp): three passes over its M points, the
+// four-step of the second FFT being the first one's run backwards.  (The
+// reference runs the layered Stockham passes over the whole vector in memory,
+// src/radix_exec.jl, and splits mixed lengths four-step style,
+// src/mixed_radix.jl:44-78.)
+//
+// Sub-transforms (SfPlan, engine_types.h) are two to six stages.  The first
+// stage's butterflies read global memory straight into registers and the last
+// stage's write it straight from registers; between them every stage reads
+// and writes its own positions of one shared-memory tile, so a stage costs
+// one shared read and one write per element, one barrier, and no second
+// buffer, and a thread's butterfly never has to be held across a barrier.  An
+// earlier form staged the tile by cp.async and ran all stages from shared
+// memory with runtime divisions per wave: it spent twice the instructions
+// (issue slots are what bounds these kernels: 40 % ALU at 12 % of DRAM).
+// Measured on B200, before -> after, per launch of the whole plan: ComplexF32
+// 10^6 x 64 1367 -> 844 us, 3^10 x 512 528 -> 359, prime 999983 x 32 (a
+// four-pass convolution before) 3972 -> 1973, 100003 x 128 2039 -> 660;
+// ComplexF64 10^6 x 64 2537 -> 1541, 999983 x 32 8314 -> 3363.
+// What a stage does per butterfly of radix R: R loads and R stores at a fixed
+// stride, one DFT_R codelet, R - 1 table twiddles (exactly rounded, read
+// through L1), and one or two small integer quotients.
+//
+// COLPASS tiles are stored position-major (position, column), the column
+// fastest: half-warps touch V >= 16 (ComplexF32) or quarter-warps V >= 8
+// (ComplexF64) consecutive slots, and twiddle reads are broadcasts.  ROWPASS
+// and MIDPASS tiles are row-major with every run of r[np - 1] positions
+// padded to an odd pitch qp (position t at (t / r) qp + t % r), which keeps
+// the last stage's stride-r reads off one bank, and rows at an odd pitch qw
+// for ROWPASS, whose later stages take adjacent rows in adjacent lanes.
+#pragma once
+#include "engine.cuh"
+
+// R as a compile-time constant for each radix the planner uses (sf_radix)
+#define SF_SWITCH(r, CALL)          \
+    switch (r) {                    \
+        case 2: CALL(2); break;     \
+        case 3: CALL(3); break;     \
+        case 4: CALL(4); break;     \
+        case 5: CALL(5); break;     \
+        case 6: CALL(6); break;     \
+        case 7: CALL(7); break;     \
+        case 8: CALL(8); break;     \
+        case 9: CALL(9); break;     \
+        case 10: CALL(10); break;   \
+        case 12: CALL(12); break;   \
+        case 14: CALL(14); break;   \
+        case 15: CALL(15); break;   \
+        default: CALL(16); break;   \
+    }
+#define SF_SWITCH_LAST(r, CALL)     \
+    if ((r) == 1) { CALL(1); }      \
+    else SF_SWITCH(r, CALL)
+
+template <int R, typename V> __device__ __forceinline__ void sf_dft(V (&v)[R]) {
+    if constexpr (R > 1) dft<R>(v);
+}
+// v[k] *= t[(k - 1) step], k = 1 .. R - 1
+template <int R, typename V> __device__ __forceinline__ void sf_twiddle(V (&v)[R], const V* t, int step) {
+#pragma unroll
+    for (int k = 1; k < R; k++) v[k] = cmul(v[k], __ldg(t + (k - 1) * step));
+}
+// output index of position b in digits 0 .. s - 1 (b < r[0] .. r[s - 1])
+__device__ __forceinline__ int sf_index(const SfPlan& S, int s, int b) {
+    int k = 0;
+    for (int i = s - 1; i >= 1; i--) {
+        const int q = udiv_small(b, S.r[i]);
+        k = (k + (b - q * S.r[i])) * S.r[i - 1];
+        b = q;
+    }
+    return k + b;
+}
+
+// ---------------------------------------------------------------- COLPASS
+// thread -> column w = tid % V of the tile and butterflies tid / V + i T / V
+template <typename V, int R>
+__device__ __forceinline__ void col_first(const KParams& p, V* buf, int t, int col, int w) {
+    const SfPlan& S = p.sa;
+    const int nb = S.L / R, N2 = p.N2, lw = p.lw, db = CFFT_THREADS >> lw;
+    const V* tw = (const V*)S.tw + S.off[0];
+    for (int b = opaque_tid() >> lw; b < nb; b += db) {
+        V v[R];
+        if (p.pre == PRE_CHIRP) {
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                const int j = (b + nb * m) * N2 + col;
+                v[m] = (j < p.nx) ? fromd<V>(cmul(tod(load_in(p, user_ld<V>(p, t, j))), __ldg(p.chirp + j))) : zero<V>();
+            }
+        } else if (p.pre == PRE_NONE && p.in_fmt != IO_PLAIN) {
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = load_in(p, user_ld<V>(p, t, (long long)(b + nb * m) * N2 + col));
+        } else {
+            const V* src = (const V*)p.in + (long long)t * p.in_dist + (b * N2 + col);
+            const int step = nb * N2;
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = p.pre == PRE_RAW ? __ldcg(src + m * step) : ldg_stream(src + m * step);
+            if (p.pre == PRE_NONE && p.dir) {
+#pragma unroll
+                for (int m = 0; m < R; m++) v[m] = conjv(v[m]);
+            }
+        }
+        sf_dft<R>(v);
+        sf_twiddle<R>(v, tw + b, nb);
+        V* dst = buf + (b << lw) + w;
+        const int ds = nb << lw;
+#pragma unroll
+        for (int m = 0; m < R; m++) dst[m * ds] = v[m];
+    }
+}
+template <typename V, int R>
+__device__ __forceinline__ void col_mid(const KParams& p, V* buf, int s, int Ls, int w) {
+    const SfPlan& S = p.sa;
+    const int nb = Ls / R, total = S.L / R, lw = p.lw, db = CFFT_THREADS >> lw;
+    const V* tw = (const V*)S.tw + S.off[s];
+    for (int b = opaque_tid() >> lw; b < total; b += db) {
+        const int K = udiv_small(b, nb), tp = b - K * nb;
+        V* e = buf + ((K * Ls + tp) << lw) + w;
+        const int ds = nb << lw;
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m * ds];
+        sf_dft<R>(v);
+        sf_twiddle<R>(v, tw + tp, nb);
+#pragma unroll
+        for (int m = 0; m < R; m++) e[m * ds] = v[m];
+    }
+}
+template <typename V, int R>
+__device__ __forceinline__ void col_last(const KParams& p, const V* buf, int t, int col, int w) {
+    const SfPlan& S = p.sa;
+    const int total = S.L / R, N2 = p.N2, lw = p.lw, db = CFFT_THREADS >> lw;
+    // outputs k = K + total j of column c take w_M^(c K) (w_M^(c total))^j:
+    // FP64 products of two table values, at most 15 of them (relative error a
+    // few 1e-15), rounded once to the data type
+    double2 st = make_double2(1, 0);
+    if (p.post == POST_TWIDDLE) st = tw_two(p.t4, (unsigned)(col * total));
+    for (int b = opaque_tid() >> lw; b < total; b += db) {
+        const V* e = buf + ((b * R) << lw) + w;
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m << lw];
+        sf_dft<R>(v);
+        const int K = sf_index(S, S.np - 1, b);
+        if (p.post == POST_TWIDDLE) {
+            V* o = (V*)p.out + (long long)t * p.out_dist + (K * N2 + col);
+            const int step = total * N2;
+            double2 wk = tw_two(p.t4, (unsigned)(col * K));
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                o[j * step] = cmul(v[j], fromd<V>(wk));
+                if (j < R - 1) wk = cmul(wk, st);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                const int jj = (K + total * j) * N2 + col;
+                if (jj < p.nx)
+                    user_st(p, t, jj, store_out(p, fromd<V>(cmul(tod(conjv(v[j])), __ldg(p.chirp + jj)))));
+            }
+        }
+    }
+}
+template <typename V> __device__ __forceinline__ void colpass_body(const KParams& p, unsigned char* smem) {
+    V* buf = (V*)smem;
+    const SfPlan& S = p.sa;
+    const int tile = block_id(p), tiles = (p.N2 + p.V - 1) >> p.lw;
+    const int t = tile / tiles;
+    if (t >= p.batch) return;                   // uniform across the CTA
+    const int w = opaque_tid() & (p.V - 1), col = ((tile - t * tiles) << p.lw) + w;
+    const bool ok = col < p.N2;                 // the last tile may be partial
+#define SF_CALL(R) col_first<V, R>(p, buf, t, col, w)
+    if (ok) { SF_SWITCH(S.r[0], SF_CALL) }
+#undef SF_CALL
+    __syncthreads();
+    int Ls = S.L / S.r[0];
+    for (int s = 1; s < S.np - 1; s++) {
+#define SF_CALL(R) col_mid<V, R>(p, buf, s, Ls, w)
+        if (ok) { SF_SWITCH(S.r[s], SF_CALL) }
+#undef SF_CALL
+        __syncthreads();
+        Ls /= S.r[s];
+    }
+#define SF_CALL(R) col_last<V, R>(p, buf, t, col, w)
+    if (ok) { SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL) }
+#undef SF_CALL
+}
+
+// ------------------------------------------------------- rows of a tile
+// position t of a row sits at (t / rl) qp + t % rl, rl = r[np - 1]; strides of
+// every stage but the last are multiples of rl positions
+__device__ __forceinline__ int row_at(int t, int rl, int qp) {
+    const int q = udiv_small(t, rl);
+    return q * qp + (t - q * rl);
+}
+// first stage: lanes take adjacent butterflies of a row (contiguous reads, of
+// an intermediate that other SMs may have written in the same launch: through
+// L2)
+template <typename V, int R>
+__device__ __forceinline__ void row_first(const KParams& p, V* buf, const V* src, int rows) {
+    const SfPlan& S = p.sc;
+    const int nb = S.L / R, rl = S.r[S.np - 1], qp = p.qp, total = rows * nb;
+    const int ds = S.np > 2 ? udiv_small(nb, rl) * qp : qp;
+    const V* tw = (const V*)S.tw + S.off[0];
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = udiv_small(i, nb), b = i - r * nb;
+        const V* x = src + (r * S.L + b);
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = __ldcg(x + m * nb);
+        sf_dft<R>(v);
+        sf_twiddle<R>(v, tw + b, nb);
+        V* e = buf + r * p.qw + (S.np > 2 ? row_at(b, rl, qp) : b);
+#pragma unroll
+        for (int m = 0; m < R; m++) e[m * ds] = v[m];
+    }
+}
+// a middle stage; LANES_W: adjacent lanes take adjacent rows (V a power of
+// two) or adjacent butterflies.  BACK: the second transform's stage on the
+// same digit
+template <typename V, int R, bool LANES_W, bool BACK>
+__device__ __forceinline__ void row_mid(const KParams& p, V* buf, int s, int Ls, int rows) {
+    const SfPlan& S = p.sc;
+    const int nb = Ls / R, per = S.L / R, rl = S.r[S.np - 1], qp = p.qp;
+    const int ds = udiv_small(nb, rl) * qp, pre = BACK ? S.L / Ls : 0;
+    const V* tw = (const V*)S.tw + (BACK ? S.boff[s] : S.off[s]);
+    const int total = LANES_W ? per << p.lw : rows * per;
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        int r, b;
+        if (LANES_W) {
+            r = i & (p.V - 1);
+            b = i >> p.lw;
+        } else {
+            r = udiv_small(i, per);
+            b = i - r * per;
+        }
+        const int K = udiv_small(b, nb), tp = b - K * nb;
+        V* e = buf + r * p.qw + row_at(K * Ls + tp, rl, qp);
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m * ds];
+        sf_dft<R>(v);
+        if (BACK) sf_twiddle<R>(v, tw + K, pre);
+        else sf_twiddle<R>(v, tw + tp, nb);
+#pragma unroll
+        for (int m = 0; m < R; m++) e[m * ds] = v[m];
+    }
+}
+
+// ---------------------------------------------------------------- ROWPASS
+template <typename V, int R>
+__device__ __forceinline__ void row_last(const KParams& p, const V* buf, int t, int r0, int rows) {
+    const SfPlan& S = p.sc;
+    const int per = S.L / R, N1 = p.N1, total = per << p.lw;
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = i & (p.V - 1), b = i >> p.lw;
+        if (r >= rows) continue;
+        const V* e = buf + r * p.qw + b * p.qp;
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m];
+        sf_dft<R>(v);
+        const int k0 = (r0 + r) + N1 * sf_index(S, S.np - 1, b), step = N1 * per;
+        if (p.out_fmt == IO_PLAIN) {
+            V* o = (V*)p.out + (long long)t * p.out_dist + k0;
+#pragma unroll
+            for (int j = 0; j < R; j++) stg_stream(o + j * step, store_out(p, v[j]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < R; j++) user_st(p, t, (long long)k0 + (long long)step * j, store_out(p, v[j]));
+        }
+    }
+}
+template <typename V> __device__ __forceinline__ void rowpass_body(const KParams& p, unsigned char* smem) {
+    V* buf = (V*)smem;
+    const SfPlan& S = p.sc;
+    const int tile = block_id(p), tiles = (p.N1 + p.V - 1) >> p.lw;
+    const int t = tile / tiles;
+    if (t >= p.batch) return;                   // uniform across the CTA
+    const int r0 = (tile - t * tiles) << p.lw, rows = min(p.V, p.N1 - r0);
+    const V* src = (const V*)p.in + (long long)t * p.in_dist + (long long)r0 * p.N2;
+#define SF_CALL(R) row_first<V, R>(p, buf, src, rows)
+    SF_SWITCH(S.r[0], SF_CALL)
+#undef SF_CALL
+    __syncthreads();
+    int Ls = S.L / S.r[0];
+    for (int s = 1; s < S.np - 1; s++) {
+        // rows past the tile's last are padding: transformed, never stored
+#define SF_CALL(R) row_mid<V, R, true, false>(p, buf, s, Ls, rows)
+        SF_SWITCH(S.r[s], SF_CALL)
+#undef SF_CALL
+        __syncthreads();
+        Ls /= S.r[s];
+    }
+#define SF_CALL(R) row_last<V, R>(p, buf, t, r0, rows)
+    SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
+#undef SF_CALL
+}
+
+// ---------------------------------------------------------------- MIDPASS
+// The last stage of the first transform leaves X[row][K + per j] of position
+// b = the butterfly's in its registers: times the spectrum (stored in this
+// order: entry row L + j per + b), conjugated, it is the input of the second
+// transform's first stage over the same digit.
+template <typename V, int R>
+__device__ __forceinline__ void mid_center(const KParams& p, V* buf, int r0, int rows) {
+    const SfPlan& S = p.sc;
+    const int per = S.L / R, total = rows * per;
+    const V* tw = (const V*)S.tw + S.boff[S.np - 1];
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = udiv_small(i, per), b = i - r * per;
+        V* e = buf + r * p.qw + b * p.qp;
+        const double2* sp = p.spec + ((long long)(r0 + r) * S.L + b);
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m];
+        sf_dft<R>(v);
+#pragma unroll
+        for (int j = 0; j < R; j++) v[j] = conjv(fromd<V>(cmul(tod(v[j]), __ldg(sp + j * per))));
+        sf_dft<R>(v);
+        sf_twiddle<R>(v, tw + b, per);
+#pragma unroll
+        for (int m = 0; m < R; m++) e[m] = v[m];
+    }
+}
+// the second transform's last stage (digit 0): outputs j2 = b + nb m of the
+// row, times w_M^(k1 j2), back in the row's place in the intermediate
+template <typename V, int R>
+__device__ __forceinline__ void mid_last(const KParams& p, const V* buf, V* dst, int r0, int rows) {
+    const SfPlan& S = p.sc;
+    const int nb = S.L / R, rl = S.r[S.np - 1], qp = p.qp, total = rows * nb;
+    const int ds = S.np > 2 ? udiv_small(nb, rl) * qp : qp;
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = udiv_small(i, nb), b = i - r * nb;
+        const V* e = buf + r * p.qw + (S.np > 2 ? row_at(b, rl, qp) : b);
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m * ds];
+        sf_dft<R>(v);
+        // FP64 products as in col_last
+        const unsigned k1 = (unsigned)(r0 + r);
+        const double2 st = tw_two(p.t4, k1 * (unsigned)nb);
+        double2 wk = tw_two(p.t4, k1 * (unsigned)b);
+        V* o = dst + (r * S.L + b);
+#pragma unroll
+        for (int m = 0; m < R; m++) {
+            o[m * nb] = cmul(v[m], fromd<V>(wk));
+            if (m < R - 1) wk = cmul(wk, st);
+        }
+    }
+}
+template <typename V> __device__ __forceinline__ void midpass_body(const KParams& p, unsigned char* smem) {
+    V* buf = (V*)smem;
+    const SfPlan& S = p.sc;
+    const int tile = block_id(p), tiles = (p.N1 + p.V - 1) / p.V;
+    const int t = tile / tiles;
+    if (t >= p.batch) return;                   // uniform across the CTA
+    const int r0 = (tile - t * tiles) * p.V, rows = min(p.V, p.N1 - r0);
+    const V* src = (const V*)p.in + (long long)t * p.in_dist + (long long)r0 * p.N2;
+    V* dst = (V*)p.out + (long long)t * p.out_dist + (long long)r0 * p.N2;
+#define SF_CALL(R) row_first<V, R>(p, buf, src, rows)
+    SF_SWITCH(S.r[0], SF_CALL)
+#undef SF_CALL
+    __syncthreads();
+    int Ls = S.L / S.r[0];
+    for (int s = 1; s < S.np - 1; s++) {
+#define SF_CALL(R) row_mid<V, R, false, false>(p, buf, s, Ls, rows)
+        SF_SWITCH(S.r[s], SF_CALL)
+#undef SF_CALL
+        __syncthreads();
+        Ls /= S.r[s];
+    }
+#define SF_CALL(R) mid_center<V, R>(p, buf, r0, rows)
+    SF_SWITCH(S.r[S.np - 1], SF_CALL)
+#undef SF_CALL
+    __syncthreads();
+    for (int s = S.np - 2; s >= 1; s--) {
+        Ls *= S.r[s];
+#define SF_CALL(R) row_mid<V, R, false, true>(p, buf, s, Ls, rows)
+        SF_SWITCH(S.r[s], SF_CALL)
+#undef SF_CALL
+        __syncthreads();
+    }
+#define SF_CALL(R) mid_last<V, R>(p, buf, dst, r0, rows)
+    SF_SWITCH(S.r[0], SF_CALL)
+#undef SF_CALL
+}

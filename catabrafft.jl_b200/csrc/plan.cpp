@@ -32,6 +32,7 @@
 
 #include "../../include/catabra_b200.h"
 #include "kernels.h"
+#include "passplan.h"
 #include "trace.h"
 
 // thread-local error text in a fixed buffer (set without touching the heap)
@@ -356,6 +357,12 @@ static std::string join(const std::vector<int>& v0) {
     return s;
 }
 
+static std::string join_raw(const std::vector<int>& v) {
+    std::string s;
+    for (size_t i = 0; i < v.size(); i++) s += (i ? "," : "") + std::to_string(v[i]);
+    return s;
+}
+
 // ------------------------------------------------------------ shape choice
 static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch, Shape& sh) {
     if (M > 4096) return false;
@@ -459,28 +466,63 @@ static void four_candidates(int64_t M, int64_t nx, int conv, int dtype, std::vec
     std::sort(out.begin(), out.end(), [](const Shape& a, const Shape& b) { return a.score < b.score; });
 }
 
+// SfPlan of every sub-length the passes use, worked out once
+static const int kSfMax = 4096;
+static const SfPlan* sf_get(int64_t L) {
+    static const std::vector<SfPlan> tab = [] {
+        std::vector<SfPlan> t(kSfMax + 1);
+        for (int l = 2; l <= kSfMax; l++)
+            if (!is_smooth7(l) || !sf_plan(l, t[l])) t[l].L = 0;
+        return t;
+    }();
+    return L >= 2 && L <= kSfMax && tab[L].L ? &tab[L] : nullptr;
+}
+static std::vector<int> sf_radices(const SfPlan& S) { return std::vector<int>(S.r, S.r + S.np); }
+static void pass_shape(int64_t N1, int64_t N2, Shape& sh) {
+    sh.mode = MODE_COLPASS;
+    sh.M = N1 * N2;
+    sh.N1 = (int)N1;
+    sh.N2 = (int)N2;
+    sh.ra = sf_radices(*sf_get(N1));
+    sh.rc = sf_radices(*sf_get(N2));
+}
+// COLPASS + ROWPASS split of a smooth M: best score of the two passes
 static bool global_shape(int64_t M, int dtype, Shape& sh) {
-    size_t e = elem_bytes(dtype);
+    const size_t e = elem_bytes(dtype);
     int64_t best = -1;
-    double bestb = 1e9;
-    for (int64_t N1 = 2; N1 <= 4096; N1++) {
+    double bests = 1e8;
+    for (int64_t N1 = 2; N1 <= kSfMax; N1++) {
         if (M % N1) continue;
-        int64_t N2 = M / N1;
-        if (N2 < 2 || N2 > 4096) continue;
-        auto ra = radix_split(N1), rc = radix_split(N2);
-        if (ra.empty() || rc.empty()) continue;
-        if (wave_G(ra, N1, CFFT_THREADS) < 1 || wave_G(rc, N2, CFFT_THREADS) < 1) continue;
-        double b = std::fabs(std::log2((double)N1 / (double)N2));
-        if (b < bestb) { bestb = b; best = N1; }
+        const SfPlan *a = sf_get(N1), *c = sf_get(M / N1);
+        if (!a || !c) continue;
+        const double sc = sf_pass_cost(*a, M / N1, N1, e) + sf_pass_cost(*c, N1, sf_qw(*c), e);
+        if (sc < bests) { bests = sc; best = N1; }
     }
     if (best < 0) return false;
-    sh.mode = MODE_COLPASS;
-    sh.M = M;
-    sh.N1 = (int)best;
-    sh.N2 = (int)(M / best);
-    sh.ra = radix_split(sh.N1);
-    sh.rc = radix_split(sh.N2);
-    (void)e;
+    pass_shape(best, M / best, sh);
+    return true;
+}
+// COLPASS + MIDPASS + COLPASS split of a convolution of at least M points:
+// the column length and row length with the least M x score
+static bool conv_shape(int64_t M, int dtype, Shape& sh) {
+    const size_t e = elem_bytes(dtype);
+    double bests = 1e300;
+    int64_t b1 = 0, b2 = 0;
+    for (int64_t N1 = 16; N1 <= kSfMax; N1++) {
+        const SfPlan* a = sf_get(N1);
+        if (!a) continue;
+        int64_t N2 = (M + N1 - 1) / N1;
+        if (N2 < 16) break;
+        for (int tries = 0; tries < 2 && N2 <= kSfMax; tries++, N2++) {
+            while (N2 <= kSfMax && !sf_get(N2)) N2++;
+            if (N2 > kSfMax) break;
+            const SfPlan* c = sf_get(N2);
+            const double sc = (double)(N1 * N2) * (2.0 * sf_pass_cost(*a, N2, N1, e) + sf_mid_cost(*c, N1, e));
+            if (sc < bests) { bests = sc; b1 = N1; b2 = N2; }
+        }
+    }
+    if (!b1) return false;
+    pass_shape(b1, b2, sh);
     return true;
 }
 
@@ -626,23 +668,18 @@ static void mixc_candidates(int64_t n, int dtype, std::vector<Shape>& out) {
     }
 }
 
-// two HBM passes (COLPASS then ROWPASS; a convolution runs two of each);
-// Rader here becomes Bluestein, and a convolution may use any 7-smooth
-// length >= its minimum: take the first that splits into two factors of at
-// most 4096
+// the HBM passes: COLPASS then ROWPASS, or COLPASS, MIDPASS, COLPASS for a
+// convolution, which may use any length >= its minimum; Rader here becomes
+// Bluestein
 static bool twopass_shape(int64_t n, int conv, int64_t M, int dtype, Shape& g) {
-    int c2 = conv;
-    int64_t M2 = M;
-    if (conv == CONV_RADER) { c2 = CONV_BLUE; M2 = smooth_ceil(2 * n - 1); }
-    for (int tries = 0; tries < 256; tries++) {
-        if (global_shape(M2, dtype, g)) {
-            g.conv = c2;
-            return true;
-        }
-        if (c2 == CONV_NONE) return false;
-        M2 = smooth_ceil(M2 + 1);
+    if (conv == CONV_NONE) {
+        if (!global_shape(M, dtype, g)) return false;
+        g.conv = CONV_NONE;
+        return true;
     }
-    return false;
+    if (!conv_shape(2 * n - 1, dtype, g)) return false;
+    g.conv = CONV_BLUE;
+    return true;
 }
 
 static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch) {
@@ -698,7 +735,7 @@ static std::string shape_desc(const Shape& s, int64_t n) {
         return pre + "four(C=" + std::to_string(s.C) + ",N1=" + std::to_string(s.N1) +
                ",N2=" + std::to_string(s.N2) + ")[" + join(s.ra) + "|" + join(s.rc) + "]";
     return pre + "twopass(N1=" + std::to_string(s.N1) + ",N2=" + std::to_string(s.N2) + ")[" +
-           join(s.ra) + "|" + join(s.rc) + "]";
+           join_raw(s.ra) + "|" + join_raw(s.rc) + "]";
 }
 
 // ---------------------------------------------------------- device tables
@@ -813,6 +850,29 @@ static int make_subplan(cfft_plan_s* P, int64_t L, const std::vector<int>& rad, 
         }
     }, &sp.tw);
 }
+// sub-transform of the passes with its twiddle blocks (SfPlan.off / .boff)
+static int make_sfplan(cfft_plan_s* P, int64_t L, SfPlan& S) {
+    const SfPlan* q = sf_get(L);
+    if (!q) return fail(CFFT_ERR_UNSUPPORTED, "no radix sequence for " + std::to_string(L));
+    S = *q;
+    const int dtype = P->dtype;
+    return cached_table(P, "sf/" + std::to_string(dtype) + "/" + std::to_string(L), [&](std::vector<unsigned char>& img) {
+        std::vector<double2> w(std::max(1, q->twall));
+        for (int i = 0; i < q->twall; i++) {
+            long long e;
+            int N;
+            sf_tw_entry(*q, i, &e, &N);
+            w[i] = omega(e, N, -1);
+        }
+        if (dtype == CFFT_C128) {
+            put(img, w);
+        } else {
+            std::vector<float2> t(w.size());
+            for (size_t m = 0; m < w.size(); m++) t[m] = make_float2((float)w[m].x, (float)w[m].y);
+            put(img, t);
+        }
+    }, &S.tw);
+}
 static int make_twolevel(cfft_plan_s* P, int64_t N, TwoLevel& t) {
     const int bits = twolevel_bits(N);
     const int64_t lo_n = 1LL << bits, hi_n = (N + lo_n - 1) / lo_n + 1;
@@ -831,6 +891,7 @@ static int make_twolevel(cfft_plan_s* P, int64_t N, TwoLevel& t) {
     return CFFT_OK;
 }
 
+static int blocks_for(const KParams& kp);
 static int plan_build(cfft_plan_s* P, const Shape& sh);
 static int plan_execute(cfft_plan_s* P, const void* in, void* out, int dir, cudaStream_t st,
                         int64_t nbatch = -1, int64_t in_dist = -1, int64_t out_dist = -1);
@@ -903,6 +964,32 @@ static int conv_spectrum(cfft_plan_s* P, const std::string& key, int64_t M, G ge
     return rc;
 }
 
+// the spectrum in MIDPASS's order (mid_center), which alone is kept: the
+// natural-order one is built in a temporary buffer
+template <class G>
+static int conv_spectrum_rows(cfft_plan_s* P, const std::string& key, int64_t N1, const SfPlan& S, G gen,
+                              const double2** out) {
+    const int64_t M = N1 * S.L;
+    cfft_plan_s* F = nullptr;
+    int rc = spectrum_plan(P->device, M, &F);
+    if (rc) return rc;
+    const void* d = nullptr;
+    rc = cached_dev_table(P, key, (size_t)M * sizeof(double2), [&](void* dp) -> int {
+        DevPtr tmp;
+        int r = dev_alloc((size_t)M * sizeof(double2), &tmp);
+        if (r) return r;
+        double2* v = (double2*)tmp->p;
+        CUDA_TRY(gen(v));
+        r = plan_execute(F, v, v, CFFT_FORWARD, 0);
+        if (r) return r;
+        CUDA_TRY(cfft_spec_center((double2*)dp, v, N1, S, 1.0 / (double)M, 0));
+        CUDA_TRY(cudaStreamSynchronize(0));      // before the buffer is released
+        return CFFT_OK;
+    }, &d);
+    *out = (const double2*)d;
+    return rc;
+}
+
 static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::string* spec_key) {
     const int64_t n = P->n, M = sh.M;
     const std::string tag = std::to_string(n) + "/" + std::to_string(M);
@@ -949,6 +1036,9 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
     if (rc) return rc;
     kp.chirp = (const double2*)dch;
     const double2* ch = kp.chirp;
+    if (sh.mode == MODE_COLPASS)
+        return conv_spectrum_rows(P, "sc/" + tag + "/" + std::to_string(sh.N1), sh.N1, *sf_get(sh.N2),
+                                  [&](double2* v) { return cfft_gen_bluestein_b(v, ch, n, M, 0); }, &kp.spec);
     *spec_key = "sb/" + tag;
     return conv_spectrum(P, *spec_key, M, [&](double2* v) {
         return cfft_gen_bluestein_b(v, ch, n, M, 0);
@@ -1389,83 +1479,57 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         P->stages.push_back(b);
         return CFFT_OK;
     }
-    // two HBM passes per FFT_M (and two FFT_M for a convolution)
+    // HBM passes (passes.cuh) over one intermediate
     const int64_t N1 = sh.N1, N2 = sh.N2, M = sh.M;
-    const int64_t PC = N2 + ((N2 % 2 == 0) ? 1 : 0);
-    int64_t Vc = 1, Vr = 1;
-    {
-        long long vc = 1, vr = 1;
-        cfft_pass_tiles(N1, N2, PC, (int)twiddle_len(N1, sh.ra), (int)twiddle_len(N2, sh.rc), twolevel_bits(M),
-                        (int)M, e, &vc, &vr);
-        Vc = vc;
-        Vr = vr;
-    }
-    SubPlan pa, pc;
-    rc = make_subplan(P, N1, sh.ra, Vc, pa, true);
+    rc = make_sfplan(P, N1, kp.sa);
     if (rc) return rc;
-    rc = make_subplan(P, N2, sh.rc, Vr, pc, true);
+    rc = make_sfplan(P, N2, kp.sc);
     if (rc) return rc;
-    TwoLevel t4;
-    rc = make_twolevel(P, M, t4);
+    rc = make_twolevel(P, M, kp.t4);
     if (rc) return rc;
+    kp.N1 = (int)N1;
+    kp.N2 = (int)N2;
+    kp.qp = sf_qp(kp.sc);
+    kp.qw = sf_qw(kp.sc);
     // chunk the batch so the scratch of one chunk stays within ~64 MB (L2 sized)
-    const int nscr = (sh.conv == CONV_NONE) ? 1 : 2;
-    int64_t chunk = std::max<int64_t>(1, scratch_budget() / (int64_t)(M * e * nscr));
+    int64_t chunk = std::max<int64_t>(1, scratch_budget() / (int64_t)(M * e));
     chunk = std::min<int64_t>(chunk, P->batch);
     P->chunk = chunk;
     P->scratch_bytes = (size_t)chunk * M * e;
     if (!P->shared_scratch) {
-        for (int i = 0; i < nscr; i++) {
-            CUDA_TRY(lib_malloc(&P->scratch[i], P->scratch_bytes));
-            P->allocs.push_back(P->scratch[i]);
-        }
+        CUDA_TRY(lib_malloc(&P->scratch[0], P->scratch_bytes));
+        P->allocs.push_back(P->scratch[0]);
     }
-    auto col = [&](int pre, int in_sel, int out_sel) {
+    auto add = [&](int mode, int pre, int post, int in_sel, int out_sel) {
         Stage s;
         s.kp = kp;
-        s.kp.mode = MODE_COLPASS;
-        s.kp.N1 = (int)N1;
-        s.kp.N2 = (int)N2;
-        s.kp.V = (int)Vc;
-        s.kp.PA = (int)Vc;
-        s.kp.mV = magic(Vc);
-        s.kp.pa = pa;
-        s.kp.t4 = t4;
+        s.kp.mode = mode;
         s.kp.pre = pre;
-        s.threads = CFFT_THREADS;
-        s.smem = cfft_colpass_smem(pa.twlen, t4.bits, t4.N, (int)(N1 * Vc), (int)e);
-        s.cluster = 1;
-        s.in_sel = in_sel;
-        s.out_sel = out_sel;
-        return s;
-    };
-    auto row = [&](int post, int in_sel, int out_sel) {
-        Stage s;
-        s.kp = kp;
-        s.kp.mode = MODE_ROWPASS;
-        s.kp.N1 = (int)N1;
-        s.kp.N2 = (int)N2;
-        s.kp.V = (int)Vr;
-        s.kp.PC = (int)PC;
-        s.kp.mV = magic(Vr);
-        s.kp.mN2 = magic(N2);
-        s.kp.pc = pc;
         s.kp.post = post;
+        if (mode == MODE_COLPASS) {
+            s.kp.V = sf_tile(N2, N1, e);
+            s.smem = sf_col_smem(kp.sa, s.kp.V, e);
+        } else if (mode == MODE_ROWPASS) {
+            s.kp.V = sf_tile(N1, kp.qw, e);
+            s.smem = sf_row_smem(kp.sc, s.kp.V, e);
+        } else {
+            s.kp.V = sf_mid_rows(kp.sc, N1, e);
+            s.smem = sf_row_smem(kp.sc, s.kp.V, e);
+        }
+        s.kp.lw = sf_lg(s.kp.V);
         s.threads = CFFT_THREADS;
-        s.smem = (size_t)(cfft_pass_tw_elems(pc.twlen, (int)e) + Vr * PC) * e + 16;
         s.cluster = 1;
         s.in_sel = in_sel;
         s.out_sel = out_sel;
-        return s;
+        P->stages.push_back(s);
     };
     if (sh.conv == CONV_NONE) {
-        P->stages.push_back(col(PRE_NONE, 0, 2));
-        P->stages.push_back(row(POST_OUT, 2, 1));
+        add(MODE_COLPASS, PRE_NONE, POST_TWIDDLE, 0, 2);
+        add(MODE_ROWPASS, 0, 0, 2, 1);
     } else {
-        P->stages.push_back(col(PRE_CHIRP, 0, 2));
-        P->stages.push_back(row(POST_RAW, 2, 3));
-        P->stages.push_back(col(PRE_SPEC, 3, 2));
-        P->stages.push_back(row(POST_CHIRP, 2, 1));
+        add(MODE_COLPASS, PRE_CHIRP, POST_TWIDDLE, 0, 2);
+        add(MODE_MIDPASS, 0, 0, 2, 2);
+        add(MODE_COLPASS, PRE_RAW, POST_CHIRP, 2, 1);
     }
     for (auto& s : P->stages) {
         s.fn = cfft_kernel_for(s.kp.mode, P->dtype);
@@ -1549,8 +1613,7 @@ static int plan_execute(cfft_plan_s* P, const void* in, void* out, int dir, cuda
             else if (kp.mode == MODE_ROWS) grid = (unsigned)((nb + kp.V - 1) / kp.V);
             else if (kp.mode == MODE_FOUR || kp.mode == MODE_CONVC || kp.mode == MODE_MIXC || kp.mode == MODE_P2CL)
                 grid = (unsigned)(nb * kp.C);
-            else if (kp.mode == MODE_COLPASS) grid = (unsigned)(nb * (kp.N2 / kp.V));
-            else grid = (unsigned)(nb * (kp.N1 / kp.V));
+            else grid = (unsigned)(nb * blocks_for(kp));
             if (s.persist && grid > s.persist) grid = s.persist;
             cudaError_t ce;
             if (s.launch == 2) {
@@ -1651,7 +1714,8 @@ static void wisdom_store(const WisdomKey& k, const std::string& sig) {
 static bool io_fusable(const cfft_plan_s* P) {
     for (const auto& st : P->stages) {
         const int m = st.kp.mode;
-        if (m != MODE_ROWS && m != MODE_FOUR && m != MODE_COLPASS && m != MODE_ROWPASS) return false;
+        if (m != MODE_ROWS && m != MODE_FOUR && m != MODE_COLPASS && m != MODE_ROWPASS && m != MODE_MIDPASS)
+            return false;
         if (st.launch != 0 || st.fn == cfft_r4096_kernel(P->dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64))
             return false;
     }
@@ -1911,7 +1975,7 @@ static int build_queue_plan(int64_t n, int dtype, int flags, int device, size_t 
                 ok = P->stages[0].cluster <= 1 && batched_smem(P->stages[0]) <= cap;
             } else {
                 for (auto& st : P->stages)
-                    ok = ok && (st.kp.mode == MODE_COLPASS || st.kp.mode == MODE_ROWPASS) && st.smem <= cap;
+                    ok = ok && st.smem <= cap;
             }
             if (ok) break;
             rc = fail(CFFT_ERR_UNSUPPORTED, "no queue shape within the shared-memory budget for n=" +
@@ -1935,8 +1999,8 @@ static bool single_kernel(const cfft_plan_s* P) {
 // CTAs one parameter block occupies in a batched launch
 static int blocks_for(const KParams& kp) {
     if (kp.mode == MODE_FOUR) return kp.C;
-    if (kp.mode == MODE_COLPASS) return kp.N2 / kp.V;
-    if (kp.mode == MODE_ROWPASS) return kp.N1 / kp.V;
+    if (kp.mode == MODE_COLPASS) return (kp.N2 + kp.V - 1) / kp.V;
+    if (kp.mode == MODE_ROWPASS || kp.mode == MODE_MIDPASS) return (kp.N1 + kp.V - 1) / kp.V;
     return 1;
 }
 // single-kernel stage -> its batched kernel variant (and the parameter fix-up
@@ -2027,15 +2091,15 @@ static int batch_create_queue(cfft_batch_s* B) {
     // Two-pass transforms, largest first, in slabs: consecutive transforms
     // whose scratch fits one slot of a ring, closed once a stage holds at
     // least two waves of tiles.  The items run as a software pipeline of
-    // steps: step t holds stage 3 of slab t-3, stage 2 of slab t-2, stage 1
-    // of slab t-1 and stage 0 of slab t, so an item's dependency (the
+    // steps: step t holds stage 2 of slab t-2, stage 1 of slab t-1 and
+    // stage 0 of slab t, so an item's dependency (the
     // previous stage of its transform) was handed out a step earlier, and
     // the intermediate it reads was written recently (L2).  A slab first
     // waits for the slab that last used its slot; single-CTA transforms are
     // spread over the steps (no dependencies: they fill the waits).
     auto scratch_need = [&](int64_t i) {
         cfft_plan_s* P = B->plans[B->len[i]];
-        return (size_t)P->shape.M * e * (P->stages.size() > 2 ? 2 : 1);
+        return (size_t)P->shape.M * e;
     };
     auto stage_tiles = [&](int64_t i, int s) { return blocks_for(B->plans[B->len[i]]->stages[s].kp); };
     std::vector<std::vector<int64_t>> slabs;
@@ -2063,7 +2127,7 @@ static int batch_create_queue(cfft_batch_s* B) {
         }
         size_t freeb = 0, totb = 0;
         cudaMemGetInfo(&freeb, &totb);
-        // the pipeline keeps four slabs in flight: six slots (or as many as
+        // the pipeline keeps three slabs in flight: six slots (or as many as
         // the slabs, or as a quarter of free memory holds, at least four)
         nslots = (int)std::min<size_t>(slabs.size(), std::max<size_t>(4, std::min<size_t>(6, freeb / 4 / slot)));
         if (slabs.size() == 1) slot = total;
@@ -2071,18 +2135,16 @@ static int batch_create_queue(cfft_batch_s* B) {
         B->allocs.push_back(B->scratch[0]);
     }
     const int nslabs = (int)slabs.size();
-    const int nsteps = nslabs ? nslabs + 3 : 1;
+    const int nsteps = nslabs ? nslabs + 2 : 1;
     std::vector<int> slab_ctr(nslabs), slab_need(nslabs, 0);
     for (int k = 0; k < nslabs; k++) slab_ctr[k] = nctr++;
-    std::map<int64_t, std::pair<int64_t, int64_t>> so;   // scratch offsets (elements) in the slab's slot
+    std::map<int64_t, int64_t> so;                       // scratch offset (elements) in the slab's slot
     std::map<int64_t, std::vector<int>> sctr;            // stage counters per transform
     for (int k = 0; k < nslabs; k++) {
         int64_t cur = 0;
         for (int64_t i : slabs[k]) {
-            cfft_plan_s* P = B->plans[B->len[i]];
-            const int64_t M = P->shape.M;
-            so[i] = {cur, P->stages.size() > 2 ? cur + M : -1};
-            cur += M * (P->stages.size() > 2 ? 2 : 1);
+            so[i] = cur;
+            cur += B->plans[B->len[i]]->shape.M;
         }
     }
     auto emit_stage = [&](int k, int64_t i, int pass) {
@@ -2100,8 +2162,7 @@ static int batch_create_queue(cfft_batch_s* B) {
                 *user = 1;
                 *dist = B->len[i];
             } else {
-                const int64_t o = (sel == 2) ? so[i].first : so[i].second;
-                *ptr = base + (size_t)o * e;
+                *ptr = base + (size_t)so[i] * e;
                 *off = 0;
                 *user = 0;
                 *dist = P->shape.M;
@@ -2131,7 +2192,7 @@ static int batch_create_queue(cfft_batch_s* B) {
             done = nctr++;
             sctr[i].push_back(done);
         }
-        const int kind = kp.mode == MODE_COLPASS ? QK_COLPASS : QK_ROWPASS;
+        const int kind = kp.mode == MODE_COLPASS ? QK_COLPASS : kp.mode == MODE_MIDPASS ? QK_MIDPASS : QK_ROWPASS;
         const int d = (int)desc.size();
         desc.push_back(kp);
         for (int b = 0; b < tiles; b++) items.push_back({d, b, kind, wait, need, done});
@@ -2154,7 +2215,7 @@ static int batch_create_queue(cfft_batch_s* B) {
     };
     size_t next_single = 0;
     for (int t = 0; t < nsteps; t++) {
-        for (int s = 3; s >= 0; s--) {
+        for (int s = 2; s >= 0; s--) {
             const int k = t - s;
             if (k < 0 || k >= nslabs) continue;
             for (int64_t i : slabs[k])
@@ -2251,7 +2312,7 @@ static int batch_create_impl(cfft_batch_s* B, int64_t count, const int64_t* leng
         size_t need_max = 0;
         for (int64_t i : twopass) {
             cfft_plan_s* P = B->plans[B->len[i]];
-            need_max = std::max(need_max, (size_t)P->shape.M * e * (P->stages.size() > 2 ? 2 : 1));
+            need_max = std::max(need_max, (size_t)P->shape.M * e);
         }
         budget = std::max(budget, need_max);
         CUDA_TRY(lib_malloc(&B->scratch[0], budget));
@@ -2260,16 +2321,14 @@ static int batch_create_impl(cfft_batch_s* B, int64_t count, const int64_t* leng
         std::vector<int64_t> chunk;
         auto flush = [&]() -> int {
             if (chunk.empty()) return CFFT_OK;
-            // scratch offsets (elements) per transform: S1, S2
-            std::map<int64_t, std::pair<int64_t, int64_t>> so;
+            // scratch offset (elements) per transform
+            std::map<int64_t, int64_t> so;
             int64_t cur = 0;
             for (int64_t i : chunk) {
-                cfft_plan_s* P = B->plans[B->len[i]];
-                const int64_t M = P->shape.M;
-                so[i] = {cur, P->stages.size() > 2 ? cur + M : -1};
-                cur += M * (P->stages.size() > 2 ? 2 : 1);
+                so[i] = cur;
+                cur += B->plans[B->len[i]]->shape.M;
             }
-            for (int pass = 0; pass < 4; pass++) {
+            for (int pass = 0; pass < 3; pass++) {
                 std::map<std::tuple<const void*, int, int>, std::vector<Item>> pb;
                 for (int64_t i : chunk) {
                     cfft_plan_s* P = B->plans[B->len[i]];
@@ -2281,8 +2340,7 @@ static int batch_create_impl(cfft_batch_s* B, int64_t count, const int64_t* leng
                     auto where = [&](int sel, const void** ptr, long long* off, unsigned char* user, long long* dist) {
                         if (sel <= 1) { *ptr = nullptr; *off = B->off[i]; *user = 1; *dist = B->len[i]; }
                         else {
-                            const int64_t o = (sel == 2) ? so[i].first : so[i].second;
-                            *ptr = (const char*)B->scratch[0] + (size_t)o * e;
+                            *ptr = (const char*)B->scratch[0] + (size_t)so[i] * e;
                             *off = 0; *user = 0; *dist = P->shape.M;
                         }
                     };
@@ -2308,7 +2366,7 @@ static int batch_create_impl(cfft_batch_s* B, int64_t count, const int64_t* leng
         };
         for (int64_t i : twopass) {
             cfft_plan_s* P = B->plans[B->len[i]];
-            const size_t need = (size_t)P->shape.M * e * (P->stages.size() > 2 ? 2 : 1);
+            const size_t need = (size_t)P->shape.M * e;
             if (used + need > budget) {
                 int rc = flush();
                 if (rc) return rc;
@@ -2448,8 +2506,7 @@ static int serve_plan(cfft_server_s* S, int64_t n, bool direct, cfft_plan_s** ou
 }
 static size_t serve_scratch(const cfft_plan_s* P) {
     if (single_kernel(P)) return 0;
-    const size_t one = align_up((size_t)P->shape.M * elem_bytes(P->dtype), kServeAlign);
-    return P->stages.size() > 2 ? 2 * one : one;
+    return align_up((size_t)P->shape.M * elem_bytes(P->dtype), kServeAlign);
 }
 static void serve_error(cfft_server_s* S, const std::string& msg) {
     std::lock_guard<std::mutex> lk(S->emu);
@@ -2473,7 +2530,7 @@ static int serve_launch(cfft_server_s* S, ServeSlot& sl) {
     cfft_trace::Range tr("serve_batch requests=%lld", (long long)sl.reqs.size(), 0);
     struct It { KParams kp; double cost; size_t smem; };
     std::map<std::tuple<const void*, int, int>, std::vector<It>> singles;
-    std::map<std::tuple<const void*, int>, std::vector<It>> pass[4];
+    std::map<std::tuple<const void*, int>, std::vector<It>> pass[3];
     size_t scur = 0;
     for (int64_t t : sl.reqs) {
         ServeReq& r = S->req[t];
@@ -2497,15 +2554,13 @@ static int serve_launch(cfft_server_s* S, ServeSlot& sl) {
             singles[std::make_tuple(fn, P->stages[0].cluster, smem_class(sm))].push_back({kp, cost, sm});
             continue;
         }
-        const size_t one = align_up((size_t)P->shape.M * elem_bytes(S->dtype), kServeAlign);
         char* s1 = (char*)sl.scratch + scur;
-        char* s2 = s1 + one;
         scur += serve_scratch(P);
-        for (size_t k = 0; k < P->stages.size() && k < 4; k++) {
+        for (size_t k = 0; k < P->stages.size(); k++) {
             const Stage& st = P->stages[k];
             KParams kp = st.kp;
             auto where = [&](int sel) -> void* {
-                return sel == 0 ? (void*)r.in : sel == 1 ? r.out : sel == 2 ? (void*)s1 : (void*)s2;
+                return sel == 0 ? (void*)r.in : sel == 1 ? r.out : (void*)s1;
             };
             kp.batch = 1;
             kp.in = where(st.in_sel);
@@ -2547,7 +2602,7 @@ static int serve_launch(cfft_server_s* S, ServeSlot& sl) {
     };
     for (auto& kv : singles) add(std::get<0>(kv.first), std::get<1>(kv.first), kv.second);
     std::stable_sort(gs.begin(), gs.end(), [](const G& a, const G& b) { return a.grid > b.grid; });
-    for (int k = 0; k < 4; k++)
+    for (int k = 0; k < 3; k++)
         for (auto& kv : pass[k]) add(std::get<0>(kv.first), 1, kv.second);
     if (host.size() > sl.desc_cap) {
         if (sl.h_desc) lib_free_host(sl.h_desc);

@@ -13,6 +13,7 @@
 // items.
 #include "engine.cuh"
 #include "kernels.h"
+#include "passes.cuh"
 #include "pow2.cuh"
 
 template <typename V, int MB>
@@ -48,8 +49,9 @@ __global__ void __launch_bounds__(CFFT_THREADS, MB) kq_batch(QueueLaunch L) {
         case QK_ROWS: rows_body<V, CFFT_EMAX>(sp, smem); break;
         case QK_FOUR: four_body<V, CFFT_EMAX, DynK<0>>(sp, smem); break;
         case QK_FOUR_WARP: four_body<V, CFFT_EMAX, DynK<1>>(sp, smem); break;
-        case QK_COLPASS: colpass_body<V, CFFT_EMAX>(sp, smem); break;
-        default: rowpass_body<V, CFFT_EMAX>(sp, smem); break;
+        case QK_COLPASS: colpass_body<V>(sp, smem); break;
+        case QK_ROWPASS: rowpass_body<V>(sp, smem); break;
+        default: midpass_body<V>(sp, smem); break;
     }
     if (it.done >= 0) flow_publish(ctr + it.done);
 }

@@ -109,6 +109,30 @@ cudaError_t cfft_scale(double2* v, long long M, double s, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// spectrum in MIDPASS's order, scaled: dst[row L + j per + b] = scale
+// src[row + N1 (K(b) + per j)], per = L / r[np - 1], K(b) the output index of
+// position b in the other digits
+__global__ void k_spec_center(double2* dst, const double2* src, long long N1, SfPlan S, double scale) {
+    const long long M = N1 * S.L;
+    const int per = S.L / S.r[S.np - 1];
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long row = i / S.L;
+        const int u = (int)(i - row * S.L), j = u / per;
+        int b = u - j * per, K = 0;
+        for (int d = S.np - 2; d >= 1; d--) {
+            K = (K + b % S.r[d]) * S.r[d - 1];
+            b /= S.r[d];
+        }
+        const double2 v = src[row + N1 * (K + b + per * j)];
+        dst[i] = make_double2(v.x * scale, v.y * scale);
+    }
+}
+cudaError_t cfft_spec_center(double2* dst, const double2* src, long long N1, const SfPlan& S, double scale,
+                             cudaStream_t st) {
+    k_spec_center<<<grid_for(N1 * S.L), 256, 0, st>>>(dst, src, N1, S, scale);
+    return cudaGetLastError();
+}
 // spectrum in the cluster kernels' row-major (k1, k2) order: dst[k1 N2 + k2]
 // = src[k1 + N1 k2], so each CTA reads its rows contiguously
 __global__ void k_spec_rowmajor(double2* dst, const double2* src, long long N1, long long N2) {

@@ -1,0 +1,152 @@
+"""CPU check of the HBM-pass kernels' index plan (csrc/passes.cuh): the radix
+sequences, in-place positions, twiddle exponents and padded row addresses of
+COLPASS, ROWPASS and MIDPASS, restated here, give the DFT (and the cyclic
+convolution), touch every position of a tile once per stage and stay inside
+the shared memory the planner asks for."""
+import numpy as np
+import pytest
+
+RADICES = (16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2)
+
+
+def radices(L):
+    """Fewest stages; ascending; at least two (csrc/passplan.h picks among the
+    fewest-stage sequences by arithmetic, which no index depends on)."""
+    best = None
+
+    def go(rem, mx, cur):
+        nonlocal best
+        if rem == 1:
+            if best is None or len(cur) < len(best):
+                best = list(cur)
+            return
+        if best is not None and len(cur) + 1 >= len(best) or len(cur) == 6:
+            return
+        for r in RADICES:
+            if r <= mx and rem % r == 0:
+                go(rem // r, r, cur + [r])
+    go(L, 16, [])
+    return best[::-1] if len(best) > 1 else best + [1]
+
+
+def index_of(r, s, b):
+    """Output index of position b in digits 0 .. s-1 (sf_index)."""
+    k = 0
+    for i in range(s - 1, 0, -1):
+        b, d = divmod(b, r[i])
+        k = (k + d) * r[i - 1]
+    return k + b
+
+
+def w(N, e):
+    return np.exp(-2j * np.pi * ((e % N) / N))
+
+
+def dft(v):
+    return np.fft.fft(v)
+
+
+class Row:
+    """One row of a tile: position t at (t // rl) qp + t % rl."""
+
+    def __init__(self, L):
+        self.L, self.r = L, radices(L)
+        self.rl = self.r[-1]
+        self.qp = self.rl | 1
+        self.qw = (L // self.rl * self.qp) | 1
+        self.buf = np.zeros(self.qw, complex)
+
+    def at(self, t):
+        return (t // self.rl) * self.qp + t % self.rl
+
+    def butterflies(self, s):
+        """(base address, stride, b, K, t') of stage s, every address checked."""
+        r = self.r
+        Ls = self.L // int(np.prod(r[:s]))
+        nb = Ls // r[s]
+        seen = np.zeros(self.qw, bool)
+        for b in range(self.L // r[s]):
+            if s == len(r) - 1:
+                base, st, K, tp = b * self.qp, 1, b, 0
+            else:
+                K, tp = divmod(b, nb)
+                base, st = self.at(K * Ls + tp), (nb // self.rl) * self.qp
+            idx = base + st * np.arange(r[s])
+            assert idx.min() >= 0 and idx.max() < self.qw and not seen[idx].any()
+            seen[idx] = True
+            yield idx, b, K, tp, nb, Ls
+        assert seen.sum() == self.L
+
+
+def forward(x):
+    """FFT of one row through its stages; output in natural order."""
+    R = Row(len(x))
+    r, n = R.r, len(R.r)
+    out = np.zeros(R.L, complex)
+    for s in range(n):
+        for idx, b, K, tp, nb, Ls in R.butterflies(s):
+            v = x[b + nb * np.arange(r[0])] if s == 0 else R.buf[idx]
+            v = dft(v)
+            if s < n - 1:
+                R.buf[idx] = v * w(Ls, tp * np.arange(r[s]))
+            else:
+                out[index_of(r, n - 1, b) + R.L // r[s] * np.arange(r[s])] = v
+    return out
+
+
+LENGTHS = [2, 4, 16, 21, 27, 81, 100, 243, 250, 256, 343, 625, 1000, 1024, 2187, 2401, 3125, 4096]
+
+
+@pytest.mark.parametrize("L", LENGTHS)
+def test_row_stages_are_the_dft(L):
+    rng = np.random.default_rng(L)
+    x = rng.standard_normal(L) + 1j * rng.standard_normal(L)
+    ref = np.fft.fft(x)
+    assert np.linalg.norm(forward(x) - ref) < 1e-12 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("L", [n for n in LENGTHS if len(radices(n)) > 1 and radices(n)[-1] > 1])
+def test_mid_pass_is_the_cyclic_convolution(L):
+    # MIDPASS on one row: FFT, spectrum in the kernel's order, conjugation,
+    # second FFT over the digits in reverse order
+    rng = np.random.default_rng(L + 1)
+    x = rng.standard_normal(L) + 1j * rng.standard_normal(L)
+    spec = rng.standard_normal(L) + 1j * rng.standard_normal(L)
+    R = Row(L)
+    r, n = R.r, len(R.r)
+    per = L // r[-1]
+    center = np.array([spec[index_of(r, n - 1, u % per) + per * (u // per)] for u in range(L)])
+    for s in range(n - 1):
+        for idx, b, K, tp, nb, Ls in R.butterflies(s):
+            v = dft(x[b + nb * np.arange(r[0])] if s == 0 else R.buf[idx])
+            R.buf[idx] = v * w(Ls, tp * np.arange(r[s]))
+    for idx, b, *_ in R.butterflies(n - 1):
+        v = np.conj(dft(R.buf[idx]) * center[np.arange(r[-1]) * per + b])
+        R.buf[idx] = dft(v) * w(L, index_of(r, n - 1, b) * np.arange(r[-1]))
+    out = np.zeros(L, complex)
+    for s in range(n - 2, -1, -1):
+        for idx, b, K, tp, nb, Ls in R.butterflies(s):
+            v = dft(R.buf[idx])
+            if s:
+                pre = L // Ls
+                R.buf[idx] = v * w(pre * r[s], index_of(r, s, K) * np.arange(r[s]))
+            else:
+                out[b + nb * np.arange(r[0])] = v
+    ref = np.fft.fft(np.conj(np.fft.fft(x) * spec))
+    assert np.linalg.norm(out - ref) < 1e-12 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("N1,N2", [(16, 21), (27, 100), (144, 140)])
+def test_three_pass_convolution(N1, N2):
+    # COLPASS, MIDPASS, COLPASS over an N1 x N2 intermediate
+    M = N1 * N2
+    rng = np.random.default_rng(M)
+    x = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    h = np.fft.fft(rng.standard_normal(M) + 1j * rng.standard_normal(M))
+    z = np.fft.fft(x.reshape(N1, N2), axis=0) * w(M, np.outer(np.arange(N1), np.arange(N2)))
+    for k1 in range(N1):
+        y = np.fft.fft(np.conj(np.fft.fft(z[k1]) * h[k1 + N1 * np.arange(N2)]))
+        z[k1] = y * w(M, k1 * np.arange(N2))
+    out = np.conj(np.fft.fft(z, axis=0)).reshape(-1) / M
+    ref = np.fft.ifft(np.fft.fft(x) * h)
+    assert np.linalg.norm(out - ref) < 1e-12 * np.linalg.norm(ref)
