@@ -43,6 +43,8 @@ struct SfPlan {
     int boff[SF_MAXS];
     int twlen;                    // entries of the forward blocks
     int twall;                    // entries of all blocks
+    // ceil(2^32 / d) for quotients by d = nb of stage s, L / r[s] and r[s] (sf_div)
+    unsigned mnb[SF_MAXS], mper[SF_MAXS], mr[SF_MAXS];
     const void* tw;
 };
 
@@ -73,7 +75,8 @@ struct KParams {
     int pre, post;                // pass prologue / epilogue
     SubPlan pa, pc;               // ROWS / FOUR: column (N1) / row (N2, or M in ROWS) plans
     SfPlan sa, sc;                // passes: column (N1) / row (N2) sub-transforms
-    int lw;                       // passes: log2 V (V = tile width of COLPASS / ROWPASS, rows of MIDPASS)
+    unsigned mv;                  // passes: multiplier of V (V = tile width of COLPASS / ROWPASS, rows of MIDPASS)
+    int ks;                       // passes: floor(threads / V)
     int qp, qw;                   // ROWPASS / MIDPASS: pitches of a last-radix run and of a row
     TwoLevel t4;                  // four-step twiddles w_M^(i2 k1)
     const int* perm;              // Rader: g^j mod nx, j < nx-1

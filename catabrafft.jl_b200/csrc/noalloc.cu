@@ -121,7 +121,7 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
         if (b < 2 || b > 4096) continue;
         SfPlan ta, tc;
         if (!sf_plan((int)a, ta) || !sf_plan((int)b, tc)) continue;
-        const double sc = sf_pass_cost(ta, b, a, e) + sf_pass_cost(tc, a, sf_qw(tc), e);
+        const double sc = sf_pass_cost(ta, b, e, false) + sf_pass_cost(tc, a, e, true);
         if (sc < best) { best = sc; N1 = a; pa = ta; pc = tc; }
     }
     if (N1 < 0)
@@ -196,18 +196,14 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
     pc.tw = twC;
     kp.sa = pa;
     kp.sc = pc;
-    kp.qp = sf_qp(pc);
-    kp.qw = sf_qw(pc);
     KParams col = kp, row = kp;
     col.mode = MODE_COLPASS;
-    col.V = sf_tile(N2, N1, e);
-    col.lw = sf_lg(col.V);
+    size_t smem_col = 0, smem_row = 0;
+    sf_stage(col, e, &smem_col);
     col.pre = PRE_NONE;
     col.post = POST_TWIDDLE;
     row.mode = MODE_ROWPASS;
-    row.V = sf_tile(N1, kp.qw, e);
-    row.lw = sf_lg(row.V);
-    const size_t smem_col = sf_col_smem(pa, col.V, e), smem_row = sf_row_smem(pc, row.V, e);
+    sf_stage(row, e, &smem_row);
 
     const long long chunk = std::max<long long>(1, (long long)(kScratchBytes / ((size_t)n * e)));
     for (long long b0 = 0; b0 < batch; b0 += chunk) {

@@ -36,8 +36,8 @@
 // through L1), and one or two small integer quotients.
 //
 // COLPASS tiles are stored position-major (position, column), the column
-// fastest: half-warps touch V >= 16 (ComplexF32) or quarter-warps V >= 8
-// (ComplexF64) consecutive slots, and twiddle reads are broadcasts.  ROWPASS
+// fastest: adjacent lanes touch adjacent slots, and twiddle reads are
+// broadcasts.  ROWPASS
 // and MIDPASS tiles are row-major with every run of r[np - 1] positions
 // padded to an odd pitch qp (position t at (t / r) qp + t % r), which keeps
 // the last stage's stride-r reads off one bank, and rows at an odd pitch qw
@@ -74,11 +74,13 @@ template <int R, typename V> __device__ __forceinline__ void sf_twiddle(V (&v)[R
 #pragma unroll
     for (int k = 1; k < R; k++) v[k] = cmul(v[k], __ldg(t + (k - 1) * step));
 }
+// x / d by the host's multiplier (sf_magic): x < 2^20, d <= 2^12
+__device__ __forceinline__ int sf_div(int x, unsigned m) { return m ? (int)__umulhi((unsigned)x, m) : x; }
 // output index of position b in digits 0 .. s - 1 (b < r[0] .. r[s - 1])
 __device__ __forceinline__ int sf_index(const SfPlan& S, int s, int b) {
     int k = 0;
     for (int i = s - 1; i >= 1; i--) {
-        const int q = udiv_small(b, S.r[i]);
+        const int q = sf_div(b, S.mr[i]);
         k = (k + (b - q * S.r[i])) * S.r[i - 1];
         b = q;
     }
@@ -86,26 +88,47 @@ __device__ __forceinline__ int sf_index(const SfPlan& S, int s, int b) {
 }
 
 // ---------------------------------------------------------------- COLPASS
-// thread -> column w = tid % V of the tile and butterflies tid / V + i T / V
+// thread -> column w = tid % V of the tile and butterflies k0, k0 + ks, ...
+// (k0 = tid / V, ks = floor(T / V); the T - ks V threads left over idle)
+struct ColThread {
+    int w, k0, col;
+    bool ok;
+};
 template <typename V, int R>
-__device__ __forceinline__ void col_first(const KParams& p, V* buf, int t, int col, int w) {
+__device__ __forceinline__ void col_first(const KParams& p, V* buf, int t, const ColThread& c) {
     const SfPlan& S = p.sa;
-    const int nb = S.L / R, N2 = p.N2, lw = p.lw, db = CFFT_THREADS >> lw;
+    const int nb = S.L / R, N2 = p.N2, W = p.V, step = nb * N2;
     const V* tw = (const V*)S.tw + S.off[0];
-    for (int b = opaque_tid() >> lw; b < nb; b += db) {
+    for (int b = c.k0; b < nb; b += p.ks) {
         V v[R];
+        const int j0 = b * N2 + c.col;
         if (p.pre == PRE_CHIRP) {
+            // rows past the input's end are zero; their reads go to the
+            // butterfly's first row, so that no branch keeps the loads apart
+            const int j1 = min(j0, p.nx - 1);
+            if (p.in_fmt == IO_PLAIN) {
+                const V* src = (const V*)p.in + (long long)t * p.in_dist;
+#pragma unroll
+                for (int m = 0; m < R; m++) v[m] = ldg_stream(src + (j0 + m * step < p.nx ? j0 + m * step : j1));
+            } else {
+#pragma unroll
+                for (int m = 0; m < R; m++) v[m] = user_ld<V>(p, t, j0 + m * step < p.nx ? j0 + m * step : j1);
+            }
+            if (p.dir) {
+#pragma unroll
+                for (int m = 0; m < R; m++) v[m] = conjv(v[m]);
+            }
 #pragma unroll
             for (int m = 0; m < R; m++) {
-                const int j = (b + nb * m) * N2 + col;
-                v[m] = (j < p.nx) ? fromd<V>(cmul(tod(load_in(p, user_ld<V>(p, t, j))), __ldg(p.chirp + j))) : zero<V>();
+                const int j = j0 + m * step;
+                const V x = fromd<V>(cmul(tod(v[m]), __ldg(p.chirp + (j < p.nx ? j : j1))));
+                v[m] = j < p.nx ? x : zero<V>();
             }
         } else if (p.pre == PRE_NONE && p.in_fmt != IO_PLAIN) {
 #pragma unroll
-            for (int m = 0; m < R; m++) v[m] = load_in(p, user_ld<V>(p, t, (long long)(b + nb * m) * N2 + col));
+            for (int m = 0; m < R; m++) v[m] = load_in(p, user_ld<V>(p, t, (long long)j0 + (long long)m * step));
         } else {
-            const V* src = (const V*)p.in + (long long)t * p.in_dist + (b * N2 + col);
-            const int step = nb * N2;
+            const V* src = (const V*)p.in + (long long)t * p.in_dist + j0;
 #pragma unroll
             for (int m = 0; m < R; m++) v[m] = p.pre == PRE_RAW ? __ldcg(src + m * step) : ldg_stream(src + m * step);
             if (p.pre == PRE_NONE && p.dir) {
@@ -115,21 +138,21 @@ __device__ __forceinline__ void col_first(const KParams& p, V* buf, int t, int c
         }
         sf_dft<R>(v);
         sf_twiddle<R>(v, tw + b, nb);
-        V* dst = buf + (b << lw) + w;
-        const int ds = nb << lw;
+        V* dst = buf + b * W + c.w;
+        const int ds = nb * W;
 #pragma unroll
         for (int m = 0; m < R; m++) dst[m * ds] = v[m];
     }
 }
 template <typename V, int R>
-__device__ __forceinline__ void col_mid(const KParams& p, V* buf, int s, int Ls, int w) {
+__device__ __forceinline__ void col_mid(const KParams& p, V* buf, int s, int Ls, const ColThread& c) {
     const SfPlan& S = p.sa;
-    const int nb = Ls / R, total = S.L / R, lw = p.lw, db = CFFT_THREADS >> lw;
+    const int nb = Ls / R, total = S.L / R, W = p.V;
     const V* tw = (const V*)S.tw + S.off[s];
-    for (int b = opaque_tid() >> lw; b < total; b += db) {
-        const int K = udiv_small(b, nb), tp = b - K * nb;
-        V* e = buf + ((K * Ls + tp) << lw) + w;
-        const int ds = nb << lw;
+    for (int b = c.k0; b < total; b += p.ks) {
+        const int K = sf_div(b, S.mnb[s]), tp = b - K * nb;
+        V* e = buf + (K * Ls + tp) * W + c.w;
+        const int ds = nb * W;
         V v[R];
 #pragma unroll
         for (int m = 0; m < R; m++) v[m] = e[m * ds];
@@ -140,19 +163,19 @@ __device__ __forceinline__ void col_mid(const KParams& p, V* buf, int s, int Ls,
     }
 }
 template <typename V, int R>
-__device__ __forceinline__ void col_last(const KParams& p, const V* buf, int t, int col, int w) {
+__device__ __forceinline__ void col_last(const KParams& p, const V* buf, int t, const ColThread& c) {
     const SfPlan& S = p.sa;
-    const int total = S.L / R, N2 = p.N2, lw = p.lw, db = CFFT_THREADS >> lw;
+    const int total = S.L / R, N2 = p.N2, W = p.V, col = c.col;
     // outputs k = K + total j of column c take w_M^(c K) (w_M^(c total))^j:
     // FP64 products of two table values, at most 15 of them (relative error a
     // few 1e-15), rounded once to the data type
     double2 st = make_double2(1, 0);
     if (p.post == POST_TWIDDLE) st = tw_two(p.t4, (unsigned)(col * total));
-    for (int b = opaque_tid() >> lw; b < total; b += db) {
-        const V* e = buf + ((b * R) << lw) + w;
+    for (int b = c.k0; b < total; b += p.ks) {
+        const V* e = buf + b * R * W + c.w;
         V v[R];
 #pragma unroll
-        for (int m = 0; m < R; m++) v[m] = e[m << lw];
+        for (int m = 0; m < R; m++) v[m] = e[m * W];
         sf_dft<R>(v);
         const int K = sf_index(S, S.np - 1, b);
         if (p.post == POST_TWIDDLE) {
@@ -165,11 +188,22 @@ __device__ __forceinline__ void col_last(const KParams& p, const V* buf, int t, 
                 if (j < R - 1) wk = cmul(wk, st);
             }
         } else {
+            // outputs past the transform's end are dropped
+            const int j0 = K * N2 + col, step = total * N2, j1 = min(j0, p.nx - 1);
 #pragma unroll
             for (int j = 0; j < R; j++) {
-                const int jj = (K + total * j) * N2 + col;
-                if (jj < p.nx)
-                    user_st(p, t, jj, store_out(p, fromd<V>(cmul(tod(conjv(v[j])), __ldg(p.chirp + jj)))));
+                const int jj = j0 + j * step;
+                v[j] = store_out(p, fromd<V>(cmul(tod(conjv(v[j])), __ldg(p.chirp + (jj < p.nx ? jj : j1)))));
+            }
+            if (p.out_fmt == IO_PLAIN) {
+                V* o = (V*)p.out + (long long)t * p.out_dist + j0;
+#pragma unroll
+                for (int j = 0; j < R; j++)
+                    if (j0 + j * step < p.nx) stg_stream(o + j * step, v[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < R; j++)
+                    if (j0 + j * step < p.nx) user_st(p, t, j0 + j * step, v[j]);
             }
         }
     }
@@ -177,34 +211,40 @@ __device__ __forceinline__ void col_last(const KParams& p, const V* buf, int t, 
 template <typename V> __device__ __forceinline__ void colpass_body(const KParams& p, unsigned char* smem) {
     V* buf = (V*)smem;
     const SfPlan& S = p.sa;
-    const int tile = block_id(p), tiles = (p.N2 + p.V - 1) >> p.lw;
+    const int tile = block_id(p), tiles = (p.N2 + p.V - 1) / p.V;
     const int t = tile / tiles;
     if (t >= p.batch) return;                   // uniform across the CTA
-    const int w = opaque_tid() & (p.V - 1), col = ((tile - t * tiles) << p.lw) + w;
-    const bool ok = col < p.N2;                 // the last tile may be partial
-#define SF_CALL(R) col_first<V, R>(p, buf, t, col, w)
-    if (ok) { SF_SWITCH(S.r[0], SF_CALL) }
+    ColThread c;
+    {
+        const int tid = opaque_tid();
+        c.k0 = sf_div(tid, p.mv);
+        c.w = tid - c.k0 * p.V;
+        c.col = (tile - t * tiles) * p.V + c.w;
+        c.ok = c.k0 < p.ks && c.col < p.N2;     // the last tile may be partial
+    }
+#define SF_CALL(R) col_first<V, R>(p, buf, t, c)
+    if (c.ok) { SF_SWITCH(S.r[0], SF_CALL) }
 #undef SF_CALL
     __syncthreads();
     int Ls = S.L / S.r[0];
     for (int s = 1; s < S.np - 1; s++) {
-#define SF_CALL(R) col_mid<V, R>(p, buf, s, Ls, w)
-        if (ok) { SF_SWITCH(S.r[s], SF_CALL) }
+#define SF_CALL(R) col_mid<V, R>(p, buf, s, Ls, c)
+        if (c.ok) { SF_SWITCH(S.r[s], SF_CALL) }
 #undef SF_CALL
         __syncthreads();
         Ls /= S.r[s];
     }
-#define SF_CALL(R) col_last<V, R>(p, buf, t, col, w)
-    if (ok) { SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL) }
+#define SF_CALL(R) col_last<V, R>(p, buf, t, c)
+    if (c.ok) { SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL) }
 #undef SF_CALL
 }
 
 // ------------------------------------------------------- rows of a tile
 // position t of a row sits at (t / rl) qp + t % rl, rl = r[np - 1]; strides of
 // every stage but the last are multiples of rl positions
-__device__ __forceinline__ int row_at(int t, int rl, int qp) {
-    const int q = udiv_small(t, rl);
-    return q * qp + (t - q * rl);
+__device__ __forceinline__ int row_at(const SfPlan& S, int t, int qp) {
+    const int q = sf_div(t, S.mr[S.np - 1]);
+    return q * qp + (t - q * S.r[S.np - 1]);
 }
 // first stage: lanes take adjacent butterflies of a row (contiguous reads, of
 // an intermediate that other SMs may have written in the same launch: through
@@ -212,43 +252,44 @@ __device__ __forceinline__ int row_at(int t, int rl, int qp) {
 template <typename V, int R>
 __device__ __forceinline__ void row_first(const KParams& p, V* buf, const V* src, int rows) {
     const SfPlan& S = p.sc;
-    const int nb = S.L / R, rl = S.r[S.np - 1], qp = p.qp, total = rows * nb;
-    const int ds = S.np > 2 ? udiv_small(nb, rl) * qp : qp;
+    const int nb = S.L / R, qp = p.qp, total = rows * nb;
+    const int ds = sf_div(nb, S.mr[S.np - 1]) * qp;
     const V* tw = (const V*)S.tw + S.off[0];
     for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
-        const int r = udiv_small(i, nb), b = i - r * nb;
+        const int r = sf_div(i, S.mnb[0]), b = i - r * nb;
         const V* x = src + (r * S.L + b);
         V v[R];
 #pragma unroll
         for (int m = 0; m < R; m++) v[m] = __ldcg(x + m * nb);
         sf_dft<R>(v);
         sf_twiddle<R>(v, tw + b, nb);
-        V* e = buf + r * p.qw + (S.np > 2 ? row_at(b, rl, qp) : b);
+        V* e = buf + r * p.qw + row_at(S, b, qp);
 #pragma unroll
         for (int m = 0; m < R; m++) e[m * ds] = v[m];
     }
 }
-// a middle stage; LANES_W: adjacent lanes take adjacent rows (V a power of
-// two) or adjacent butterflies.  BACK: the second transform's stage on the
-// same digit
+// a middle stage; LANES_W: adjacent lanes take adjacent rows (as COLPASS's
+// adjacent columns), else adjacent butterflies of a row.  BACK: the second
+// transform's stage on the same digit
 template <typename V, int R, bool LANES_W, bool BACK>
 __device__ __forceinline__ void row_mid(const KParams& p, V* buf, int s, int Ls, int rows) {
     const SfPlan& S = p.sc;
-    const int nb = Ls / R, per = S.L / R, rl = S.r[S.np - 1], qp = p.qp;
-    const int ds = udiv_small(nb, rl) * qp, pre = BACK ? S.L / Ls : 0;
+    const int nb = Ls / R, per = S.L / R, qp = p.qp;
+    const int ds = sf_div(nb, S.mr[S.np - 1]) * qp, pre = BACK ? S.L / Ls : 0;
     const V* tw = (const V*)S.tw + (BACK ? S.boff[s] : S.off[s]);
-    const int total = LANES_W ? per << p.lw : rows * per;
-    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+    const int tid = opaque_tid(), k0 = LANES_W ? sf_div(tid, p.mv) : 0;
+    const int total = LANES_W ? (k0 < p.ks ? per : 0) : rows * per;
+    for (int i = LANES_W ? k0 : tid; i < total; i += LANES_W ? p.ks : CFFT_THREADS) {
         int r, b;
         if (LANES_W) {
-            r = i & (p.V - 1);
-            b = i >> p.lw;
+            r = tid - k0 * p.V;
+            b = i;
         } else {
-            r = udiv_small(i, per);
+            r = sf_div(i, S.mper[s]);
             b = i - r * per;
         }
-        const int K = udiv_small(b, nb), tp = b - K * nb;
-        V* e = buf + r * p.qw + row_at(K * Ls + tp, rl, qp);
+        const int K = sf_div(b, S.mnb[s]), tp = b - K * nb;
+        V* e = buf + r * p.qw + row_at(S, K * Ls + tp, qp);
         V v[R];
 #pragma unroll
         for (int m = 0; m < R; m++) v[m] = e[m * ds];
@@ -264,10 +305,9 @@ __device__ __forceinline__ void row_mid(const KParams& p, V* buf, int s, int Ls,
 template <typename V, int R>
 __device__ __forceinline__ void row_last(const KParams& p, const V* buf, int t, int r0, int rows) {
     const SfPlan& S = p.sc;
-    const int per = S.L / R, N1 = p.N1, total = per << p.lw;
-    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
-        const int r = i & (p.V - 1), b = i >> p.lw;
-        if (r >= rows) continue;
+    const int per = S.L / R, N1 = p.N1, tid = opaque_tid(), k0 = sf_div(tid, p.mv), r = tid - k0 * p.V;
+    if (k0 >= p.ks || r >= rows) return;
+    for (int b = k0; b < per; b += p.ks) {
         const V* e = buf + r * p.qw + b * p.qp;
         V v[R];
 #pragma unroll
@@ -287,10 +327,10 @@ __device__ __forceinline__ void row_last(const KParams& p, const V* buf, int t, 
 template <typename V> __device__ __forceinline__ void rowpass_body(const KParams& p, unsigned char* smem) {
     V* buf = (V*)smem;
     const SfPlan& S = p.sc;
-    const int tile = block_id(p), tiles = (p.N1 + p.V - 1) >> p.lw;
+    const int tile = block_id(p), tiles = (p.N1 + p.V - 1) / p.V;
     const int t = tile / tiles;
     if (t >= p.batch) return;                   // uniform across the CTA
-    const int r0 = (tile - t * tiles) << p.lw, rows = min(p.V, p.N1 - r0);
+    const int r0 = (tile - t * tiles) * p.V, rows = min(p.V, p.N1 - r0);
     const V* src = (const V*)p.in + (long long)t * p.in_dist + (long long)r0 * p.N2;
 #define SF_CALL(R) row_first<V, R>(p, buf, src, rows)
     SF_SWITCH(S.r[0], SF_CALL)
@@ -321,7 +361,7 @@ __device__ __forceinline__ void mid_center(const KParams& p, V* buf, int r0, int
     const int per = S.L / R, total = rows * per;
     const V* tw = (const V*)S.tw + S.boff[S.np - 1];
     for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
-        const int r = udiv_small(i, per), b = i - r * per;
+        const int r = sf_div(i, S.mper[S.np - 1]), b = i - r * per;
         V* e = buf + r * p.qw + b * p.qp;
         const double2* sp = p.spec + ((long long)(r0 + r) * S.L + b);
         V v[R];
@@ -341,11 +381,11 @@ __device__ __forceinline__ void mid_center(const KParams& p, V* buf, int r0, int
 template <typename V, int R>
 __device__ __forceinline__ void mid_last(const KParams& p, const V* buf, V* dst, int r0, int rows) {
     const SfPlan& S = p.sc;
-    const int nb = S.L / R, rl = S.r[S.np - 1], qp = p.qp, total = rows * nb;
-    const int ds = S.np > 2 ? udiv_small(nb, rl) * qp : qp;
+    const int nb = S.L / R, qp = p.qp, total = rows * nb;
+    const int ds = sf_div(nb, S.mr[S.np - 1]) * qp;
     for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
-        const int r = udiv_small(i, nb), b = i - r * nb;
-        const V* e = buf + r * p.qw + (S.np > 2 ? row_at(b, rl, qp) : b);
+        const int r = sf_div(i, S.mnb[0]), b = i - r * nb;
+        const V* e = buf + r * p.qw + row_at(S, b, qp);
         V v[R];
 #pragma unroll
         for (int m = 0; m < R; m++) v[m] = e[m * ds];

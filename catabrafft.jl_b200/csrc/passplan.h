@@ -7,6 +7,8 @@
 
 #include "engine_types.h"
 
+static const int SF_THREADS = 256;    // CTA size of the pass kernels
+
 // Radix sequence of L (7-smooth, L >= 2): the fewest stages first (a stage is
 // a shared-memory round trip and a barrier), then the least arithmetic, in
 // ascending order -- the last radix is the largest, so the runs that the row
@@ -38,6 +40,9 @@ inline void sf_search(int rem, int maxr, int depth, double cost, int* cur, int* 
         sf_search(rem / r, r, depth + 1, cost + sf_radix_cost(r) + 0.05 * r, cur, best, nbest, cbest);
     }
 }
+// x / d = (x m) >> 32 with m = ceil(2^32 / d), exact for x < 2^20 and d <= 2^12;
+// 0 stands for d = 1
+inline unsigned sf_magic(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
 // fills L, np, r and the table layout; false if L has no sequence
 inline bool sf_plan(int L, SfPlan& S) {
     S = SfPlan();
@@ -68,6 +73,13 @@ inline bool sf_plan(int L, SfPlan& S) {
         off += (S.r[s] - 1) * pre;
     }
     S.twall = off;
+    int sub = L;
+    for (int s = 0; s < S.np; s++) {
+        sub /= S.r[s];
+        S.mnb[s] = sf_magic(sub);
+        S.mper[s] = sf_magic(L / S.r[s]);
+        S.mr[s] = sf_magic(S.r[s]);
+    }
     return true;
 }
 // entry i of the twiddle table is w_N^e
@@ -95,52 +107,110 @@ inline __host__ __device__ void sf_tw_entry(const SfPlan& S, int i, long long* e
 // shared memory per CTA: three ComplexF32 or two ComplexF64 CTAs per SM (the
 // register budgets of the kernels)
 inline size_t sf_budget(size_t e) { return (e == 8 ? 74 : 112) * (size_t)1024; }
-inline int sf_lg(int v) {
-    int l = 0;
-    while ((2 << l) <= v) l++;
-    return l;
+// Pitches of a row tile, in elements: of a last-radix run, and of a row.
+// ROWPASS's later stages take V adjacent rows in adjacent lanes: B lanes (16
+// ComplexF32, 8 ComplexF64) share a wavefront, so from V = B rows an odd row
+// pitch alone is conflict-free; below, the rows step by B / V and the B / V
+// butterflies between them by an odd run pitch.  MIDPASS's lanes walk one row,
+// whose last stage reads runs at an odd pitch.
+inline int sf_qp(const SfPlan& S, int V, size_t e, bool mid) {
+    const int rl = S.r[S.np - 1], B = e == 8 ? 16 : 8;
+    return !mid && V >= B ? rl : rl | 1;
 }
-// rows: pitch of a last-radix run (odd) and of a row (odd, for ROWPASS)
-inline int sf_qp(const SfPlan& S) { return S.r[S.np - 1] | 1; }
-inline int sf_qw(const SfPlan& S) { return (S.L / S.r[S.np - 1] * sf_qp(S)) | 1; }
+inline int sf_qw(const SfPlan& S, int V, size_t e, bool mid) {
+    const int len = S.L / S.r[S.np - 1] * sf_qp(S, V, e, mid), B = e == 8 ? 16 : 8;
+    if (mid) return len;
+    const int step = V >= B || B % V ? 1 : B / V;
+    return len + ((step - len) % B + B) % B;
+}
 inline size_t sf_col_smem(const SfPlan& S, int V, size_t e) { return (size_t)S.L * V * e; }
-inline size_t sf_row_smem(const SfPlan& S, int V, size_t e) { return (size_t)sf_qw(S) * V * e; }
-// tile width (a power of two) of a pass over `count` columns / rows of `per`
-// shared elements: about 4096 (ComplexF32) or 2048 (ComplexF64) elements a
-// tile, wider until a segment of the strided side is 128 bytes as long as the
-// budget holds it, and no wider than the count needs
-inline int sf_tile(long long count, long long per, size_t e) {
-    const long long want = e == 8 ? 4096 : 2048;
-    long long V = 1;
-    while (2 * V <= 64 && 2 * V * per * (long long)e <= (long long)sf_budget(e) && V < count &&
-           (2 * V * per <= want || 2 * V * (long long)e <= 128))
-        V *= 2;
-    return (int)V;
-}
-// how a pass of sub-length L over `count` neighbours scores (lower is better):
-// stages, short segments on the strided side, idle columns of a partial tile
-inline double sf_pass_cost(const SfPlan& S, long long count, long long per, size_t e) {
-    const int V = sf_tile(count, per, e);
-    if ((size_t)V * per * e > sf_budget(e)) return 1e9;
-    double c = 2.0 + S.np;
-    for (int s = 0; s < S.np; s++) c += 0.06 * (S.r[s] > 1 ? sf_radix_cost(S.r[s]) : 0.0);
+inline size_t sf_row_smem(const SfPlan& S, int V, size_t e, bool mid) { return (size_t)sf_qw(S, V, e, mid) * V * e; }
+// Cost model of a tile, in SM cycles of one of its CTAs: a round of butterflies
+// of radix R (each active thread runs one) takes about 1340 + 171 R cycles at
+// three CTAs per SM -- fitted to B200 timings of COLPASS at radix 10 (268
+// instructions a butterfly, one every 12 cycles) -- whether or not every
+// thread has one, and a tile costs about one more such latency to start.  So
+// widths are picked to fill the rounds, not for a target size.
+inline double sf_round(int R, int dfts) { return 1340.0 + 171.0 * R * dfts; }
+inline double sf_start() { return 2500.0; }
+// cycles per useful element of a COLPASS / ROWPASS tile of width V
+inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bool row) {
+    const size_t smem = row ? sf_row_smem(S, V, e, false) : sf_col_smem(S, V, e);
+    if (smem > sf_budget(e)) return 1e9 + (double)smem;
+    const int ks = SF_THREADS / V;
+    double c = sf_start();
+    for (int s = 0; s < S.np; s++) {
+        const int nb = S.L / S.r[s];
+        c += sf_round(S.r[s], 1) * (row && s == 0 ? (V * nb + SF_THREADS - 1) / SF_THREADS : (nb + ks - 1) / ks);
+    }
+    // the strided side moves 32-byte sectors: whole ones if V and the row
+    // length allow, else one more per segment
     const long long seg = V * (long long)e;
-    if (seg < 32) c += 6.0;
-    else if (seg < 64) c += 2.5;
-    else if (seg < 128) c += 0.7;
+    const bool whole = seg % 32 == 0 && count * (long long)e % 32 == 0;
+    const double sectors = (double)((seg + 31) / 32 + (whole ? 0 : 1)) * 32.0 / (double)seg;
+    c *= 1.0 + 0.25 * (sectors - 1.0) + (seg < 64 ? 0.3 : seg < 128 ? 0.1 : 0.0);
     const long long tiles = (count + V - 1) / V;
-    return c * (double)(tiles * V) / (double)count;
+    return c / ((double)V * S.L) * (double)(tiles * V) / (double)count;
 }
-// MIDPASS: whole rows, contiguous on both sides; about 4096 (2048) elements
-inline int sf_mid_rows(const SfPlan& S, long long count, size_t e) {
-    const long long want = e == 8 ? 4096 : 2048;
-    return (int)std::max<long long>(1, std::min<long long>(count, want / sf_qw(S)));
+// the width with the least cost (at most 64)
+inline int sf_tile(const SfPlan& S, long long count, size_t e, bool row, double* cost = nullptr) {
+    int best = 1;
+    double bc = 1e300;
+    for (int V = 1; V <= 64 && V <= count; V++) {
+        const double c = sf_tile_cost(S, V, count, e, row);
+        if (c < bc) {
+            bc = c;
+            best = V;
+        }
+    }
+    if (cost) *cost = bc;
+    return best;
+}
+inline double sf_pass_cost(const SfPlan& S, long long count, size_t e, bool row) {
+    double c;
+    sf_tile(S, count, e, row, &c);
+    return c;
+}
+// MIDPASS: whole rows, contiguous on both sides, the second transform's first
+// stage fused with the first one's last
+inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e) {
+    const size_t smem = sf_row_smem(S, V, e, true);
+    if (smem > sf_budget(e)) return 1e9 + (double)smem;
+    double c = sf_start();
+    for (int s = 0; s < S.np; s++) {
+        const int rounds = (V * (S.L / S.r[s]) + SF_THREADS - 1) / SF_THREADS;
+        c += rounds * (s == S.np - 1 ? sf_round(S.r[s], 2) : 2.0 * sf_round(S.r[s], 1));
+    }
+    const long long tiles = (count + V - 1) / V;
+    return c / ((double)V * S.L) * (double)(tiles * V) / (double)count;
+}
+inline int sf_mid_rows(const SfPlan& S, long long count, size_t e, double* cost = nullptr) {
+    int best = 1;
+    double bc = 1e300;
+    for (int V = 1; V <= 32 && V <= count; V++) {
+        const double c = sf_mid_tile_cost(S, V, count, e);
+        if (c < bc) {
+            bc = c;
+            best = V;
+        }
+    }
+    if (cost) *cost = bc;
+    return best;
 }
 inline double sf_mid_cost(const SfPlan& S, long long count, size_t e) {
-    const int V = sf_mid_rows(S, count, e);
-    if (sf_row_smem(S, V, e) > sf_budget(e)) return 1e9;
-    double c = 2.0 + 1.6 * S.np;
-    for (int s = 0; s < S.np; s++) c += 0.12 * (S.r[s] > 1 ? sf_radix_cost(S.r[s]) : 0.0);
-    const long long tiles = (count + V - 1) / V;
-    return c * (double)(tiles * V) / (double)count;
+    double c;
+    sf_mid_rows(S, count, e, &c);
+    return c;
+}
+// tile, pitches and shared memory of a pass (mode, N1, N2, sa, sc set)
+inline void sf_stage(KParams& k, size_t e, size_t* smem) {
+    const bool mid = k.mode == MODE_MIDPASS;
+    if (k.mode == MODE_COLPASS) k.V = sf_tile(k.sa, k.N2, e, false);
+    else if (mid) k.V = sf_mid_rows(k.sc, k.N1, e);
+    else k.V = sf_tile(k.sc, k.N1, e, true);
+    k.mv = sf_magic(k.V);
+    k.ks = SF_THREADS / k.V;
+    k.qp = sf_qp(k.sc, k.V, e, mid);
+    k.qw = sf_qw(k.sc, k.V, e, mid);
+    *smem = k.mode == MODE_COLPASS ? sf_col_smem(k.sa, k.V, e) : sf_row_smem(k.sc, k.V, e, mid);
 }

@@ -495,7 +495,7 @@ static bool global_shape(int64_t M, int dtype, Shape& sh) {
         if (M % N1) continue;
         const SfPlan *a = sf_get(N1), *c = sf_get(M / N1);
         if (!a || !c) continue;
-        const double sc = sf_pass_cost(*a, M / N1, N1, e) + sf_pass_cost(*c, N1, sf_qw(*c), e);
+        const double sc = sf_pass_cost(*a, M / N1, e, false) + sf_pass_cost(*c, N1, e, true);
         if (sc < bests) { bests = sc; best = N1; }
     }
     if (best < 0) return false;
@@ -517,7 +517,7 @@ static bool conv_shape(int64_t M, int dtype, Shape& sh) {
             while (N2 <= kSfMax && !sf_get(N2)) N2++;
             if (N2 > kSfMax) break;
             const SfPlan* c = sf_get(N2);
-            const double sc = (double)(N1 * N2) * (2.0 * sf_pass_cost(*a, N2, N1, e) + sf_mid_cost(*c, N1, e));
+            const double sc = (double)(N1 * N2) * (2.0 * sf_pass_cost(*a, N2, e, false) + sf_mid_cost(*c, N1, e));
             if (sc < bests) { bests = sc; b1 = N1; b2 = N2; }
         }
     }
@@ -1489,8 +1489,6 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     if (rc) return rc;
     kp.N1 = (int)N1;
     kp.N2 = (int)N2;
-    kp.qp = sf_qp(kp.sc);
-    kp.qw = sf_qw(kp.sc);
     // chunk the batch so the scratch of one chunk stays within ~64 MB (L2 sized)
     int64_t chunk = std::max<int64_t>(1, scratch_budget() / (int64_t)(M * e));
     chunk = std::min<int64_t>(chunk, P->batch);
@@ -1506,17 +1504,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         s.kp.mode = mode;
         s.kp.pre = pre;
         s.kp.post = post;
-        if (mode == MODE_COLPASS) {
-            s.kp.V = sf_tile(N2, N1, e);
-            s.smem = sf_col_smem(kp.sa, s.kp.V, e);
-        } else if (mode == MODE_ROWPASS) {
-            s.kp.V = sf_tile(N1, kp.qw, e);
-            s.smem = sf_row_smem(kp.sc, s.kp.V, e);
-        } else {
-            s.kp.V = sf_mid_rows(kp.sc, N1, e);
-            s.smem = sf_row_smem(kp.sc, s.kp.V, e);
-        }
-        s.kp.lw = sf_lg(s.kp.V);
+        sf_stage(s.kp, e, &s.smem);
         s.threads = CFFT_THREADS;
         s.cluster = 1;
         s.in_sel = in_sel;

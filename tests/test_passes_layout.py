@@ -47,13 +47,14 @@ def dft(v):
 
 
 class Row:
-    """One row of a tile: position t at (t // rl) qp + t % rl."""
+    """One row of a tile: position t at (t // rl) qp + t % rl, with the odd run
+    pitch of MIDPASS and narrow ROWPASS tiles (wider ones use qp = rl)."""
 
     def __init__(self, L):
         self.L, self.r = L, radices(L)
         self.rl = self.r[-1]
         self.qp = self.rl | 1
-        self.qw = (L // self.rl * self.qp) | 1
+        self.qw = L // self.rl * self.qp
         self.buf = np.zeros(self.qw, complex)
 
     def at(self, t):
@@ -136,6 +137,40 @@ def test_mid_pass_is_the_cyclic_convolution(L):
     assert np.linalg.norm(out - ref) < 1e-12 * np.linalg.norm(ref)
 
 
+def row_pitches(L, V, e, mid):
+    """sf_qp and sf_qw (csrc/passplan.h)."""
+    rl, B = radices(L)[-1], 16 if e == 8 else 8
+    qp = rl if not mid and V >= B else rl | 1
+    n = L // rl * qp
+    if mid:
+        return qp, n
+    step = 1 if V >= B or B % V else B // V
+    return qp, n + (step - n) % B
+
+
+@pytest.mark.parametrize("e", [8, 16])
+@pytest.mark.parametrize("L", [81, 256, 324, 729, 1000])
+@pytest.mark.parametrize("V", [2, 4, 8, 16, 32])
+def test_row_pass_banks(L, V, e):
+    # the last stage's lanes (adjacent rows, then adjacent runs) fall in
+    # distinct slots of a wavefront for power-of-two widths
+    qp, qw = row_pitches(L, V, e, False)
+    B = 16 if e == 8 else 8
+    lanes = [(i % V) * qw + (i // V) * qp for i in range(B)]
+    assert len({x % B for x in lanes}) == B
+    assert qw >= L // radices(L)[-1] * qp
+
+
+def test_quotients_by_multiplier():
+    # sf_div: x / d = (x m) >> 32, m = ceil(2^32 / d), for x < 2^20, d <= 2^12
+    rng = np.random.default_rng(0)
+    for d in list(range(2, 300)) + [int(v) for v in rng.integers(300, 4097, 300)] + [4096]:
+        m = (2 ** 32 + d - 1) // d
+        q = rng.integers(0, 2 ** 20 // d, 200)
+        x = np.concatenate([q * d, q * d + d - 1, [0, 2 ** 20 - 1]]).astype(object)
+        assert all(int(v) * m >> 32 == int(v) // d for v in x), d
+
+
 @pytest.mark.parametrize("N1,N2", [(16, 21), (27, 100), (144, 140)])
 def test_three_pass_convolution(N1, N2):
     # COLPASS, MIDPASS, COLPASS over an N1 x N2 intermediate
@@ -149,4 +184,59 @@ def test_three_pass_convolution(N1, N2):
         z[k1] = y * w(M, k1 * np.arange(N2))
     out = np.conj(np.fft.fft(z, axis=0)).reshape(-1) / M
     ref = np.fft.ifft(np.fft.fft(x) * h)
+    assert np.linalg.norm(out - ref) < 1e-12 * np.linalg.norm(ref)
+
+
+class Line(Row):
+    """LINE's row: the first digit's blocks q0 further apart (line_at)."""
+
+    def __init__(self, L):
+        super().__init__(L)
+        self.nb0 = L // self.r[0]
+        self.q0 = 0 if len(self.r) < 3 or (self.nb0 // self.rl * self.qp) % 2 else 1
+        self.qw = L // self.rl * self.qp + self.r[0] * self.q0
+        self.buf = np.zeros(self.qw, complex)
+
+    def line_at(self, t):
+        return self.at(t) + t // self.nb0 * self.q0
+
+
+@pytest.mark.parametrize("L", LENGTHS + [8, 120, 2160, 3840, 8192, 8748, 6561, 7776])
+def test_line_stages_are_the_dft(L):
+    rng = np.random.default_rng(L + 2)
+    x = rng.standard_normal(L) + 1j * rng.standard_normal(L)
+    R = Line(L)
+    r, n = R.r, len(R.r)
+    out = np.zeros(L, complex)
+    for s in range(n):
+        Ls = L // int(np.prod(r[:s]))
+        nb, per = Ls // r[s], L // r[s]
+        seen = np.zeros(R.qw, bool)
+        for i in range(per):
+            K, tp = divmod(i, nb)
+            if s == 0:
+                base, st = R.at(i), nb // R.rl * R.qp + R.q0
+            elif s < n - 1:
+                base, st = R.line_at(K * Ls + tp), nb // R.rl * R.qp
+            if s == n - 1:
+                # i is the output index K; its digits in position order give the run
+                k = d0 = b = i
+                if n > 2:
+                    k, d0 = divmod(i, r[0])
+                    b = d0
+                    for q in range(1, n - 2):
+                        k, d = divmod(k, r[q])
+                        b = b * r[q] + d
+                    b = b * r[n - 2] + k
+                base, st = b * R.qp + d0 * R.q0 if n > 2 else b * R.qp, 1
+            idx = base + st * np.arange(r[s])
+            assert idx.min() >= 0 and idx.max() < R.qw and not seen[idx].any()
+            seen[idx] = True
+            v = dft(x[i + nb * np.arange(r[0])] if s == 0 else R.buf[idx])
+            if s < n - 1:
+                R.buf[idx] = v * w(Ls, tp * np.arange(r[s]))
+            else:
+                out[i + per * np.arange(r[s])] = v
+        assert seen.sum() == L
+    ref = np.fft.fft(x)
     assert np.linalg.norm(out - ref) < 1e-12 * np.linalg.norm(ref)
