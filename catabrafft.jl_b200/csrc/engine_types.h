@@ -56,13 +56,15 @@ struct TwoLevel {                 // w_N^e = lo[e & mask] * hi[e >> bits]  (FP64
 };
 
 enum { MODE_ROWS = 0, MODE_FOUR = 1, MODE_COLPASS = 2, MODE_ROWPASS = 3, MODE_P2COL = 4, MODE_P2ROW = 5,
-       MODE_CONVC = 6, MODE_MIXC = 7, MODE_P2CL = 8, MODE_MIDPASS = 9 };
+       MODE_CONVC = 6, MODE_MIXC = 7, MODE_P2CL = 8, MODE_MIDPASS = 9, MODE_LINE = 10 };
 // kernel selector only (KParams.mode stays MODE_FOUR): the generic four-step
 // kernel instantiated with warp-synchronous sub-transforms
 enum { MODE_FOUR_WARP = 16 };
 enum { CONV_NONE = 0, CONV_RADER = 1, CONV_BLUE = 2 };
 enum { PRE_NONE = 0, PRE_CHIRP = 1, PRE_RAW = 2 };       // COLPASS: the caller's input, times the chirp, an intermediate
-enum { POST_TWIDDLE = 0, POST_CHIRP = 1 };               // COLPASS: to the intermediate, to the caller's output
+// COLPASS: to the intermediate; times the chirp to the caller's output; to the
+// caller's output as it is (whole transforms in columns)
+enum { POST_TWIDDLE = 0, POST_CHIRP = 1, POST_STORE = 2 };
 
 struct KParams {
     int mode, conv;
@@ -77,7 +79,8 @@ struct KParams {
     SfPlan sa, sc;                // passes: column (N1) / row (N2) sub-transforms
     unsigned mv;                  // passes: multiplier of V (V = tile width of COLPASS / ROWPASS, rows of MIDPASS)
     int ks;                       // passes: floor(threads / V)
-    int qp, qw;                   // ROWPASS / MIDPASS: pitches of a last-radix run and of a row
+    int qp, qw;                   // ROWPASS / MIDPASS / LINE: pitches of a last-radix run and of a row
+    int q0;                       // LINE: extra pitch of the first digit
     TwoLevel t4;                  // four-step twiddles w_M^(i2 k1)
     const int* perm;              // Rader: g^j mod nx, j < nx-1
     const int* iperm;             // Rader: g^-j mod nx
@@ -129,7 +132,7 @@ struct BatchLaunch {
 // release of the scratch half its chunk reuses) and adds one to counter
 // `done` when finished.  Every wait is on items with smaller tickets, so the
 // queue drains whatever the residency.
-enum { QK_ROWS = 0, QK_FOUR = 1, QK_FOUR_WARP = 2, QK_COLPASS = 3, QK_ROWPASS = 4, QK_MIDPASS = 5 };
+enum { QK_ROWS = 0, QK_FOUR = 1, QK_FOUR_WARP = 2, QK_COLPASS = 3, QK_ROWPASS = 4, QK_MIDPASS = 5, QK_LINE = 6 };
 struct QItem {
     int desc;                     // parameter block
     int blk;                      // block within the parameter block

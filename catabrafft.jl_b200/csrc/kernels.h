@@ -13,8 +13,8 @@
 
 // generic kernel for a mode, or nullptr
 const void* cfft_kernel_for(int mode, int dtype);
-// the HBM-pass kernels (passes32.cu, passes64.cu): COLPASS, ROWPASS, MIDPASS,
-// for one plan or descriptor driven
+// the kernels of passes.cuh (passes32.cu, passes64.cu): COLPASS, ROWPASS,
+// MIDPASS, LINE, for one plan or descriptor driven
 const void* cfft_pass_kernel32(int mode, bool batched);
 const void* cfft_pass_kernel64(int mode, bool batched);
 // statically shaped FOUR kernel matching (N1, N2, C, radix multiplicities), or

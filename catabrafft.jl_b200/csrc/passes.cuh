@@ -10,6 +10,8 @@
 //            intermediate: N2-point DFT, product with the FP64 spectrum,
 //            conjugation, N2-point DFT that takes the digits in reverse
 //            order, four-step twiddle w_M^(k1 j2)
+//   LINE     V whole transforms that fit a CTA, one row each: one kernel from
+//            the caller's input to the caller's output
 //
 // A smooth length is COLPASS + ROWPASS; a Bluestein convolution is COLPASS
 // (chirp) + MIDPASS + COLPASS (chirp): three passes over its M points, the
@@ -124,6 +126,11 @@ __device__ __forceinline__ void col_first(const KParams& p, V* buf, int t, const
                 const V x = fromd<V>(cmul(tod(v[m]), __ldg(p.chirp + (j < p.nx ? j : j1))));
                 v[m] = j < p.nx ? x : zero<V>();
             }
+        } else if (p.post == POST_STORE) {
+            const V* src = (const V*)p.in + (long long)b * p.in_stride + c.col;
+            const long long rs = (long long)nb * p.in_stride;
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = load_in(p, ldg_stream(src + m * rs));
         } else if (p.pre == PRE_NONE && p.in_fmt != IO_PLAIN) {
 #pragma unroll
             for (int m = 0; m < R; m++) v[m] = load_in(p, user_ld<V>(p, t, (long long)j0 + (long long)m * step));
@@ -187,6 +194,11 @@ __device__ __forceinline__ void col_last(const KParams& p, const V* buf, int t, 
                 o[j * step] = cmul(v[j], fromd<V>(wk));
                 if (j < R - 1) wk = cmul(wk, st);
             }
+        } else if (p.post == POST_STORE) {
+            V* o = (V*)p.out + (long long)K * p.out_stride + col;
+            const long long step = (long long)total * p.out_stride;
+#pragma unroll
+            for (int j = 0; j < R; j++) stg_stream(o + j * step, store_out(p, v[j]));
         } else {
             // outputs past the transform's end are dropped
             const int j0 = K * N2 + col, step = total * N2, j1 = min(j0, p.nx - 1);
@@ -436,5 +448,115 @@ template <typename V> __device__ __forceinline__ void midpass_body(const KParams
     }
 #define SF_CALL(R) mid_last<V, R>(p, buf, dst, r0, rows)
     SF_SWITCH(S.r[0], SF_CALL)
+#undef SF_CALL
+}
+
+// ------------------------------------------------------------------- LINE
+// Row layout as above, plus the first digit's blocks q0 further apart, so that
+// the last stage's lanes, which take adjacent outputs (adjacent first digits),
+// step by an odd pitch too.
+__device__ __forceinline__ int line_at(const KParams& p, int t) {
+    return row_at(p.sc, t, p.qp) + sf_div(t, p.sc.mnb[0]) * p.q0;
+}
+template <typename V, int R>
+__device__ __forceinline__ void line_first(const KParams& p, V* buf, int t0, int rows) {
+    const SfPlan& S = p.sc;
+    const int nb = S.L / R, total = rows * nb;
+    const int ds = sf_div(nb, S.mr[S.np - 1]) * p.qp + p.q0;
+    const V* tw = (const V*)S.tw + S.off[0];
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = sf_div(i, S.mnb[0]), b = i - r * nb;
+        V v[R];
+        if (p.in_fmt == IO_PLAIN) {
+            const V* x = (const V*)p.in + (long long)(t0 + r) * p.in_dist + b;
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = ldg_stream(x + m * nb);
+        } else {
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = user_ld<V>(p, t0 + r, b + m * nb);
+        }
+        if (p.dir) {
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = conjv(v[m]);
+        }
+        sf_dft<R>(v);
+        sf_twiddle<R>(v, tw + b, nb);
+        V* e = buf + r * p.qw + row_at(S, b, p.qp);
+#pragma unroll
+        for (int m = 0; m < R; m++) e[m * ds] = v[m];
+    }
+}
+template <typename V, int R>
+__device__ __forceinline__ void line_mid(const KParams& p, V* buf, int s, int Ls, int rows) {
+    const SfPlan& S = p.sc;
+    const int nb = Ls / R, per = S.L / R, total = rows * per;
+    const int ds = sf_div(nb, S.mr[S.np - 1]) * p.qp;
+    const V* tw = (const V*)S.tw + S.off[s];
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = sf_div(i, S.mper[s]), b = i - r * per;
+        const int K = sf_div(b, S.mnb[s]), tp = b - K * nb;
+        V* e = buf + r * p.qw + line_at(p, K * Ls + tp);
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m * ds];
+        sf_dft<R>(v);
+        sf_twiddle<R>(v, tw + tp, nb);
+#pragma unroll
+        for (int m = 0; m < R; m++) e[m * ds] = v[m];
+    }
+}
+// lanes take adjacent outputs K (stores are whole segments); the butterfly's
+// position is K's digits in position order
+template <typename V, int R>
+__device__ __forceinline__ void line_last(const KParams& p, const V* buf, int t0, int rows) {
+    const SfPlan& S = p.sc;
+    const int per = S.L / R, total = rows * per;
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = sf_div(i, S.mper[S.np - 1]), K = i - r * per;
+        int k = K, d0 = K, b = K;
+        if (S.np > 2) {
+            k = sf_div(K, S.mr[0]);
+            d0 = b = K - k * S.r[0];
+            for (int s = 1; s < S.np - 2; s++) {
+                const int q = sf_div(k, S.mr[s]);
+                b = b * S.r[s] + (k - q * S.r[s]);
+                k = q;
+            }
+            b = b * S.r[S.np - 2] + k;
+        }
+        const V* e = buf + r * p.qw + b * p.qp + d0 * p.q0;
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m];
+        sf_dft<R>(v);
+        if (p.out_fmt == IO_PLAIN) {
+            V* o = (V*)p.out + (long long)(t0 + r) * p.out_dist + K;
+#pragma unroll
+            for (int j = 0; j < R; j++) stg_stream(o + j * per, store_out(p, v[j]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < R; j++) user_st(p, t0 + r, K + j * per, store_out(p, v[j]));
+        }
+    }
+}
+template <typename V> __device__ __forceinline__ void line_body(const KParams& p, unsigned char* smem) {
+    V* buf = (V*)smem;
+    const SfPlan& S = p.sc;
+    const int t0 = block_id(p) * p.V, rows = min(p.V, p.batch - t0);
+    if (rows <= 0) return;                      // uniform across the CTA
+#define SF_CALL(R) line_first<V, R>(p, buf, t0, rows)
+    SF_SWITCH(S.r[0], SF_CALL)
+#undef SF_CALL
+    __syncthreads();
+    int Ls = S.L / S.r[0];
+    for (int s = 1; s < S.np - 1; s++) {
+#define SF_CALL(R) line_mid<V, R>(p, buf, s, Ls, rows)
+        SF_SWITCH(S.r[s], SF_CALL)
+#undef SF_CALL
+        __syncthreads();
+        Ls /= S.r[s];
+    }
+#define SF_CALL(R) line_last<V, R>(p, buf, t0, rows)
+    SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
 }

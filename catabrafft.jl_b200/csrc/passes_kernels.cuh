@@ -11,7 +11,8 @@ template <> struct PassBlocks<double2> { static constexpr int value = 2; };
 template <typename V, int MODE> __device__ __forceinline__ void pass_body(const KParams& p, unsigned char* smem) {
     if constexpr (MODE == MODE_COLPASS) colpass_body<V>(p, smem);
     else if constexpr (MODE == MODE_ROWPASS) rowpass_body<V>(p, smem);
-    else midpass_body<V>(p, smem);
+    else if constexpr (MODE == MODE_MIDPASS) midpass_body<V>(p, smem);
+    else line_body<V>(p, smem);
 }
 template <typename V, int MODE>
 __global__ void __launch_bounds__(CFFT_THREADS, PassBlocks<V>::value) k_pass(const __grid_constant__ KParams p) {
@@ -29,6 +30,7 @@ template <typename V> const void* pass_kernel(int mode, bool batched) {
         case MODE_COLPASS: return batched ? (const void*)kb_pass<V, MODE_COLPASS> : (const void*)k_pass<V, MODE_COLPASS>;
         case MODE_ROWPASS: return batched ? (const void*)kb_pass<V, MODE_ROWPASS> : (const void*)k_pass<V, MODE_ROWPASS>;
         case MODE_MIDPASS: return batched ? (const void*)kb_pass<V, MODE_MIDPASS> : (const void*)k_pass<V, MODE_MIDPASS>;
+        case MODE_LINE: return batched ? (const void*)kb_pass<V, MODE_LINE> : (const void*)k_pass<V, MODE_LINE>;
     }
     return nullptr;
 }

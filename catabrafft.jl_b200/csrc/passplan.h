@@ -202,6 +202,39 @@ inline double sf_mid_cost(const SfPlan& S, long long count, size_t e) {
     sf_mid_rows(S, count, e, &c);
     return c;
 }
+// LINE: V whole rows; lanes of the first and middle stages walk a row, those
+// of the last one step by the first digit's pitch (odd)
+inline int sf_line_q0(const SfPlan& S) {
+    const int rl = S.r[S.np - 1];
+    if (S.np < 3) return 0;
+    return ((S.L / S.r[0] / rl) * (rl | 1)) % 2 ? 0 : 1;
+}
+inline int sf_line_qw(const SfPlan& S) {
+    const int rl = S.r[S.np - 1];
+    return S.L / rl * (rl | 1) + S.r[0] * sf_line_q0(S);
+}
+inline size_t sf_line_smem(const SfPlan& S, int V, size_t e) { return (size_t)sf_line_qw(S) * V * e; }
+// transforms per CTA: the model's cost of the whole batch, waves of CTAs on
+// 148 SMs x (three ComplexF32 or two ComplexF64)
+inline int sf_line_rows(const SfPlan& S, long long batch, size_t e) {
+    const long long slots = 148 * (e == 8 ? 3 : 2);
+    int best = 1;
+    double bc = 1e300;
+    for (int V = 1; V <= 1024 && V <= batch; V++) {
+        if (V > 1 && sf_line_smem(S, V, e) > sf_budget(e)) break;
+        double c = sf_start();
+        for (int s = 0; s < S.np; s++)
+            c += sf_round(S.r[s], 1) * (((long long)V * (S.L / S.r[s]) + SF_THREADS - 1) / SF_THREADS);
+        // whole waves while there are few; their tails matter less and less
+        const double waves = (double)((batch + V - 1) / V) / (double)slots;
+        c *= waves < 4.0 ? std::ceil(waves) : waves + 0.5;
+        if (c < bc) {
+            bc = c;
+            best = V;
+        }
+    }
+    return best;
+}
 // tile, pitches and shared memory of a pass (mode, N1, N2, sa, sc set)
 inline void sf_stage(KParams& k, size_t e, size_t* smem) {
     const bool mid = k.mode == MODE_MIDPASS;

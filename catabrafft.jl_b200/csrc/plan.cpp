@@ -272,6 +272,7 @@ struct Stage {
     int in_sel, out_sel;     // 0 user in, 1 user out, 2 scratch0, 3 scratch1
     int max_units = 0;       // persistent kernels: co-resident clusters (0 = one per unit)
     size_t smem_batched = 0; // shared memory of the descriptor-driven variant (0: smem)
+    bool cols = false;       // strided plans: the whole batch as the columns of one COLPASS
     unsigned persist = 0;    // kernels that loop over the batch: CTAs to launch at most
     int launch = 0;          // 1 / 3: pass A by tensor copies (ComplexF64 / ComplexF32 pairs); 2: dataflow
                              // launch; 4 / 5: mixed-radix / power-of-two cluster kernel with tensor copies
@@ -364,7 +365,31 @@ static std::string join_raw(const std::vector<int>& v) {
 }
 
 // ------------------------------------------------------------ shape choice
+// SfPlan of every sub-length the passes use, worked out once
+static const int kSfMax = 4096;      // factors of the passes
+static const int kLineMax = 9216;    // whole transforms in a CTA (74 KB of ComplexF32)
+static const SfPlan* sf_get(int64_t L) {
+    static const std::vector<SfPlan> tab = [] {
+        std::vector<SfPlan> t(kLineMax + 1);
+        for (int l = 2; l <= kLineMax; l++)
+            if (!is_smooth7(l) || !sf_plan(l, t[l])) t[l].L = 0;
+        return t;
+    }();
+    return L >= 2 && L <= kLineMax && tab[L].L ? &tab[L] : nullptr;
+}
+static std::vector<int> sf_radices(const SfPlan& S) { return std::vector<int>(S.r, S.r + S.np); }
 static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch, Shape& sh) {
+    const SfPlan* line = conv == CONV_NONE ? sf_get(M) : nullptr;
+    if (line && sf_line_smem(*line, 1, elem_bytes(dtype)) <= sf_budget(elem_bytes(dtype))) {
+        // LINE (passes.cuh)
+        sh.mode = MODE_ROWS;
+        sh.M = M;
+        // one row a CTA where the n = 4096 register kernel runs it
+        sh.V = M == 4096 ? 1 : sf_line_rows(*line, batch, elem_bytes(dtype));
+        sh.rc = sf_radices(*line);
+        sh.smem = sf_line_smem(*line, sh.V, elem_bytes(dtype));
+        return true;
+    }
     if (M > 4096) return false;
     auto rc = radix_split(M);
     if (M > 1 && rc.empty()) return false;
@@ -466,18 +491,30 @@ static void four_candidates(int64_t M, int64_t nx, int conv, int dtype, std::vec
     std::sort(out.begin(), out.end(), [](const Shape& a, const Shape& b) { return a.score < b.score; });
 }
 
-// SfPlan of every sub-length the passes use, worked out once
-static const int kSfMax = 4096;
-static const SfPlan* sf_get(int64_t L) {
-    static const std::vector<SfPlan> tab = [] {
-        std::vector<SfPlan> t(kSfMax + 1);
-        for (int l = 2; l <= kSfMax; l++)
-            if (!is_smooth7(l) || !sf_plan(l, t[l])) t[l].L = 0;
+// cost per element of COLPASS (kind 0), ROWPASS (1) or MIDPASS (2) with
+// sub-length L beside `count` neighbours: the model's best tile for many
+// aligned neighbours, worked out once per length, with the idle share of this
+// count's last tile
+static double sf_cost(int64_t L, int64_t count, size_t e, int kind) {
+    struct Entry { double c; int V; };
+    static const std::vector<Entry> tab = [] {
+        std::vector<Entry> t((size_t)6 * (kSfMax + 1), {1e9, 1});
+        for (int l = 2; l <= kSfMax; l++) {
+            const SfPlan* S = sf_get(l);
+            if (!S) continue;
+            for (int i = 0; i < 6; i++) {
+                Entry& x = t[(size_t)i * (kSfMax + 1) + l];
+                const size_t el = i < 3 ? 8 : 16;
+                x.V = i % 3 == 2 ? sf_mid_rows(*S, 1 << 16, el, &x.c) : sf_tile(*S, 1 << 16, el, i % 3 == 1, &x.c);
+            }
+        }
         return t;
     }();
-    return L >= 2 && L <= kSfMax && tab[L].L ? &tab[L] : nullptr;
+    const Entry& x = tab[(size_t)((e == 8 ? 0 : 3) + kind) * (kSfMax + 1) + L];
+    const int64_t V = std::min<int64_t>(x.V, count), tiles = (count + V - 1) / V;
+    const double odd = kind < 2 && count * (int64_t)e % 32 ? 1.08 : 1.0;     // segments off their sectors
+    return x.c * odd * (double)(tiles * V) / (double)count;
 }
-static std::vector<int> sf_radices(const SfPlan& S) { return std::vector<int>(S.r, S.r + S.np); }
 static void pass_shape(int64_t N1, int64_t N2, Shape& sh) {
     sh.mode = MODE_COLPASS;
     sh.M = N1 * N2;
@@ -493,9 +530,10 @@ static bool global_shape(int64_t M, int dtype, Shape& sh) {
     double bests = 1e8;
     for (int64_t N1 = 2; N1 <= kSfMax; N1++) {
         if (M % N1) continue;
+        if (M / N1 > kSfMax) continue;
         const SfPlan *a = sf_get(N1), *c = sf_get(M / N1);
         if (!a || !c) continue;
-        const double sc = sf_pass_cost(*a, M / N1, e, false) + sf_pass_cost(*c, N1, e, true);
+        const double sc = sf_cost(N1, M / N1, e, 0) + sf_cost(M / N1, N1, e, 1);
         if (sc < bests) { bests = sc; best = N1; }
     }
     if (best < 0) return false;
@@ -516,8 +554,7 @@ static bool conv_shape(int64_t M, int dtype, Shape& sh) {
         for (int tries = 0; tries < 2 && N2 <= kSfMax; tries++, N2++) {
             while (N2 <= kSfMax && !sf_get(N2)) N2++;
             if (N2 > kSfMax) break;
-            const SfPlan* c = sf_get(N2);
-            const double sc = (double)(N1 * N2) * (2.0 * sf_pass_cost(*a, N2, e, false) + sf_mid_cost(*c, N1, e));
+            const double sc = (double)(N1 * N2) * (2.0 * sf_cost(N1, N2, e, 0) + sf_cost(N2, N1, e, 2));
             if (sc < bests) { bests = sc; b1 = N1; b2 = N2; }
         }
     }
@@ -718,7 +755,7 @@ static std::string shape_desc(const Shape& s, int64_t n) {
     std::string c = s.conv == CONV_RADER ? "rader" : s.conv == CONV_BLUE ? "bluestein" : "";
     std::string pre = c.empty() ? "" : c + "(n=" + std::to_string(n) + ",M=" + std::to_string(s.M) + ")+";
     if (s.mode == MODE_ROWS)
-        return pre + "rows(V=" + std::to_string(s.V) + ")[" + join(s.rc) + "]";
+        return pre + "rows(V=" + std::to_string(s.V) + ")[" + (s.conv == CONV_NONE ? join_raw(s.rc) : join(s.rc)) + "]";
     if (s.mode == MODE_P2CL)
         return "pow2cluster(C=" + std::to_string(s.C) + ",4096 per CTA,ctas_per_sm=" + std::to_string(s.V) +
                (s.var == 1 ? ",tma" : "") + ")";
@@ -975,16 +1012,20 @@ static int conv_spectrum_rows(cfft_plan_s* P, const std::string& key, int64_t N1
     if (rc) return rc;
     const void* d = nullptr;
     rc = cached_dev_table(P, key, (size_t)M * sizeof(double2), [&](void* dp) -> int {
-        DevPtr tmp;
-        int r = dev_alloc((size_t)M * sizeof(double2), &tmp);
-        if (r) return r;
-        double2* v = (double2*)tmp->p;
-        CUDA_TRY(gen(v));
-        r = plan_execute(F, v, v, CFFT_FORWARD, 0);
-        if (r) return r;
-        CUDA_TRY(cfft_spec_center((double2*)dp, v, N1, S, 1.0 / (double)M, 0));
-        CUDA_TRY(cudaStreamSynchronize(0));      // before the buffer is released
-        return CFFT_OK;
+        // stream-ordered: a cudaMalloc / cudaFree pair per length was half of
+        // the time to plan a batch of many lengths
+        double2* v = nullptr;
+        if (alloc_injected_failure() || cudaMallocAsync((void**)&v, (size_t)M * sizeof(double2), 0) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(CFFT_ERR_NOMEM, "convolution spectrum: temporary buffer");
+        }
+        cudaError_t ce = gen(v);
+        int r = CFFT_OK;
+        if (ce == cudaSuccess) r = plan_execute(F, v, v, CFFT_FORWARD, 0);
+        if (ce == cudaSuccess && !r) ce = cfft_spec_center((double2*)dp, v, N1, S, 1.0 / (double)M, 0);
+        cudaFreeAsync(v, 0);
+        CUDA_TRY(ce);
+        return r;
     }, &d);
     *out = (const double2*)d;
     return rc;
@@ -1250,6 +1291,44 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     if (sh.mode == MODE_ROWS) {
         kp.mode = MODE_ROWS;
         kp.V = sh.V;
+        if (sh.conv == CONV_NONE && sh.M > 1) {
+            // V rows per CTA in register stages (passes.cuh), or the persistent
+            // register kernel of n = 4096
+            rc = make_sfplan(P, sh.M, kp.sc);
+            if (rc) return rc;
+            kp.mode = MODE_LINE;
+            kp.qp = sf_qp(kp.sc, 1, e, true);
+            kp.q0 = sf_line_q0(kp.sc);
+            kp.qw = sf_line_qw(kp.sc);
+            Stage s;
+            s.kp = kp;
+            s.threads = CFFT_THREADS;
+            s.smem = sh.smem;
+            s.cluster = 1;
+            s.grid = 0;
+            s.in_sel = 0;
+            s.out_sel = 1;
+            s.fn = cfft_kernel_for(MODE_LINE, P->dtype);
+            if (sh.M == 4096 && sh.V == 1) {
+                rc = make_twolevel(P, 4096, s.kp.t4);
+                if (rc) return rc;
+                s.fn = cfft_r4096_kernel(P->dtype);
+                s.smem_batched = sh.smem;
+                s.smem = cfft_r4096_smem(e);
+                P->desc += "+r4096";
+            }
+            CUDA_TRY(cfft_prepare_fn(s.fn, s.smem, 1));
+            if (s.fn == cfft_r4096_kernel(P->dtype)) {
+                // persistent: as many CTAs as are co-resident
+                int nsm = 0, occ = 0;
+                CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, P->device));
+                CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, s.fn, CFFT_THREADS, s.smem));
+                s.persist = (unsigned)(std::max(1, occ) * std::max(1, nsm));
+            }
+            P->stages.push_back(s);
+            P->chunk = P->batch;
+            return CFFT_OK;
+        }
         kp.PC = (int)(sh.M + ((sh.M % 2 == 0) ? 1 : 0));
         kp.XP = (sh.conv == CONV_RADER) ? (int)P->n : 0;
         kp.mX = magic(P->n);
@@ -1266,24 +1345,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         s.in_sel = 0;
         s.out_sel = 1;
         s.fn = cfft_kernel_for(MODE_ROWS, P->dtype);
-        if (sh.conv == CONV_NONE && sh.M == 4096 && sh.V == 1) {
-            // the register kernel; descriptor-driven launches keep the
-            // generic rows kernel and its shared memory
-            rc = make_twolevel(P, 4096, s.kp.t4);
-            if (rc) return rc;
-            s.fn = cfft_r4096_kernel(P->dtype);
-            s.smem_batched = sh.smem;
-            s.smem = cfft_r4096_smem(elem_bytes(P->dtype));
-            P->desc += "+r4096";
-        }
         CUDA_TRY(cfft_prepare_fn(s.fn, s.smem, 1));
-        if (s.fn == cfft_r4096_kernel(P->dtype)) {
-            // persistent: as many CTAs as are co-resident
-            int nsm = 0, occ = 0;
-            CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, P->device));
-            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, s.fn, CFFT_THREADS, s.smem));
-            s.persist = (unsigned)(std::max(1, occ) * std::max(1, nsm));
-        }
         P->stages.push_back(s);
         P->chunk = P->batch;
         return CFFT_OK;
@@ -1598,10 +1660,13 @@ static int plan_execute(cfft_plan_s* P, const void* in, void* out, int dir, cuda
             }
             unsigned grid;
             if (p2) grid = (unsigned)kp.batch;
-            else if (kp.mode == MODE_ROWS) grid = (unsigned)((nb + kp.V - 1) / kp.V);
+            else if (kp.mode == MODE_ROWS || kp.mode == MODE_LINE) grid = (unsigned)((nb + kp.V - 1) / kp.V);
             else if (kp.mode == MODE_FOUR || kp.mode == MODE_CONVC || kp.mode == MODE_MIXC || kp.mode == MODE_P2CL)
                 grid = (unsigned)(nb * kp.C);
-            else grid = (unsigned)(nb * blocks_for(kp));
+            else if (s.cols) {
+                kp.batch = 1;
+                grid = (unsigned)blocks_for(kp);
+            } else grid = (unsigned)(nb * blocks_for(kp));
             if (s.persist && grid > s.persist) grid = s.persist;
             cudaError_t ce;
             if (s.launch == 2) {
@@ -1702,7 +1767,8 @@ static void wisdom_store(const WisdomKey& k, const std::string& sig) {
 static bool io_fusable(const cfft_plan_s* P) {
     for (const auto& st : P->stages) {
         const int m = st.kp.mode;
-        if (m != MODE_ROWS && m != MODE_FOUR && m != MODE_COLPASS && m != MODE_ROWPASS && m != MODE_MIDPASS)
+        if (m != MODE_ROWS && m != MODE_FOUR && m != MODE_COLPASS && m != MODE_ROWPASS && m != MODE_MIDPASS &&
+            m != MODE_LINE)
             return false;
         if (st.launch != 0 || st.fn == cfft_r4096_kernel(P->dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64))
             return false;
@@ -1982,7 +2048,8 @@ static int build_queue_plan(int64_t n, int dtype, int flags, int device, size_t 
 static size_t batched_smem(const Stage& st) { return st.smem_batched ? st.smem_batched : st.smem; }
 static bool single_kernel(const cfft_plan_s* P) {
     return P->stages.size() == 1 &&
-           (P->stages[0].kp.mode == MODE_ROWS || P->stages[0].kp.mode == MODE_FOUR);
+           (P->stages[0].kp.mode == MODE_ROWS || P->stages[0].kp.mode == MODE_FOUR ||
+            P->stages[0].kp.mode == MODE_LINE);
 }
 // CTAs one parameter block occupies in a batched launch
 static int blocks_for(const KParams& kp) {
@@ -2189,7 +2256,8 @@ static int batch_create_queue(cfft_batch_s* B) {
         cfft_plan_s* P = B->plans[B->len[i]];
         KParams kp = P->stages[0].kp;
         const void* vf = batched_variant(kp, dtype);
-        const int kind = kp.mode == MODE_ROWS ? QK_ROWS
+        const int kind = kp.mode == MODE_ROWS   ? QK_ROWS
+                         : kp.mode == MODE_LINE ? QK_LINE
                          : vf == cfft_batch_kernel_for(MODE_FOUR_WARP, dt) ? QK_FOUR_WARP : QK_FOUR;
         kp.batch = 1;
         kp.in_off = kp.out_off = B->off[i];
@@ -2876,6 +2944,26 @@ int cfft_plan_create_many(cfft_plan* plan, int64_t n, int64_t batch, int dtype, 
     P->idist = idist;
     P->ostride = ostride;
     P->odist = odist;
+    // transforms side by side (distance 1, rows at the stride): they are the
+    // columns of one COLPASS tile row, so every access is a segment of V
+    // elements (LINE would gather its rows one element per sector)
+    if (idist == 1 && odist == 1 && istride >= batch && ostride >= batch && P->stages.size() == 1 &&
+        P->stages[0].kp.mode == MODE_LINE && P->stages[0].smem_batched == 0 && batch <= 0x7fffffffLL) {
+        Stage s = P->stages[0];
+        const size_t e = elem_bytes(dtype);
+        s.kp.mode = MODE_COLPASS;
+        s.kp.sa = s.kp.sc;
+        s.kp.N1 = (int)n;
+        s.kp.N2 = (int)batch;
+        s.kp.pre = PRE_NONE;
+        s.kp.post = POST_STORE;
+        sf_stage(s.kp, e, &s.smem);
+        s.cols = true;
+        s.fn = cfft_kernel_for(MODE_COLPASS, dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64);
+        if ((s.kp.V * e >= 32 || s.kp.V == batch) && s.smem <= sf_budget(e) &&
+            cfft_prepare_fn(s.fn, s.smem, 1) == cudaSuccess)
+            P->stages[0] = s;
+    }
     if (io_fusable(P)) {
         // the first kernel gathers as it loads, the last scatters as it stores
         P->io_fused = true;
