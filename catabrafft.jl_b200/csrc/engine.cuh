@@ -891,16 +891,7 @@ __device__ __forceinline__ void four_transform(const KParams& p, V* buf, V* bufC
     // ---- prologue fix-ups on the arrived input (column layout)
     double2 xsum = make_double2(0, 0);
     V x0 = zero<V>();
-    if (p.conv == CONV_NONE) {
-        if (p.dir) {
-#pragma unroll 4
-            for (int idx = tid; idx < N1 * W; idx += T) {
-                const int i1 = K::dW(p, idx), j = idx - i1 * W;
-                V* e = buf + i1 * PA + j;
-                *e = conjv(*e);
-            }
-        }
-    } else if (p.conv == CONV_BLUE) {
+    if (p.conv == CONV_BLUE) {
 #pragma unroll 4
         for (int idx = tid; idx < N1 * W; idx += T) {
             const int i1 = K::dW(p, idx), j = idx - i1 * W;
@@ -957,24 +948,6 @@ __device__ __forceinline__ void four_transform(const KParams& p, V* buf, V* bufC
     else if (C > 1) four_push_fwd<V, K>(p, buf, bufC, cl, c, t4);
     else four_twiddle_local<V, K>(p, buf, t4);
     K::template rowC<V, EMAX>(bufC, p, twC);
-
-    if (p.conv == CONV_NONE) {
-        // X[k1 + N1 k2] from row layout (r, k2), k1 = c*R1 + r
-        if (p.out_fmt == IO_PLAIN) {
-            V* out = (V*)p.out + (long long)t * p.out_dist;
-#pragma unroll 4
-            for (int idx = tid; idx < R1 * N2; idx += T) {
-                const int k2 = K::dR1(p, idx), r = idx - k2 * R1;
-                stg_stream(out + (long long)(c * R1 + r) + (long long)N1 * k2, store_out(p, bufC[r * PC + k2]));
-            }
-        } else {
-            for (int idx = tid; idx < R1 * N2; idx += T) {
-                const int k2 = K::dR1(p, idx), r = idx - k2 * R1;
-                user_st(p, t, (long long)(c * R1 + r) + (long long)N1 * k2, store_out(p, bufC[r * PC + k2]));
-            }
-        }
-        return;
-    }
 
     // ---- pointwise multiply by spectrum/M and conjugate (inverse via conj)
 #pragma unroll 4

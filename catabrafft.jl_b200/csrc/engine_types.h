@@ -56,7 +56,8 @@ struct TwoLevel {                 // w_N^e = lo[e & mask] * hi[e >> bits]  (FP64
 };
 
 enum { MODE_ROWS = 0, MODE_FOUR = 1, MODE_COLPASS = 2, MODE_ROWPASS = 3, MODE_P2COL = 4, MODE_P2ROW = 5,
-       MODE_CONVC = 6, MODE_MIXC = 7, MODE_P2CL = 8, MODE_MIDPASS = 9, MODE_LINE = 10 };
+       MODE_CONVC = 6, MODE_MIXC = 7, MODE_P2CL = 8, MODE_MIDPASS = 9, MODE_LINE = 10,
+       MODE_CLUS = 11 };
 // kernel selector only (KParams.mode stays MODE_FOUR): the generic four-step
 // kernel instantiated with warp-synchronous sub-transforms
 enum { MODE_FOUR_WARP = 16 };
@@ -81,6 +82,8 @@ struct KParams {
     int ks;                       // passes: floor(threads / V)
     int qp, qw;                   // ROWPASS / MIDPASS / LINE: pitches of a last-radix run and of a row
     int q0;                       // LINE: extra pitch of the first digit
+    unsigned mr1;                 // CLUS: multiplier of R1 = N1 / C (rows per CTA)
+    int ks2;                      // CLUS: floor(threads / R1)
     TwoLevel t4;                  // four-step twiddles w_M^(i2 k1)
     const int* perm;              // Rader: g^j mod nx, j < nx-1
     const int* iperm;             // Rader: g^-j mod nx

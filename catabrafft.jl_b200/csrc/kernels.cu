@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) kb_four(Bat
 }
 
 const void* cfft_batch_kernel_for(int mode, int dtype) {
-    if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE)
+    if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE ||
+        mode == MODE_CLUS)
         return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, true) : cfft_pass_kernel32(mode, true);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {
@@ -63,12 +64,12 @@ const void* cfft_batch_kernel_for(int mode, int dtype) {
     return nullptr;
 }
 
-cudaError_t cfft_launch_batch(const void* f, const BatchLaunch& L, unsigned grid, size_t smem,
+cudaError_t cfft_launch_batch(const void* f, const BatchLaunch& L, unsigned grid, int threads, size_t smem,
                               int cluster, cudaStream_t stream) {
     if (!f) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid, 1, 1);
-    cfg.blockDim = dim3(CFFT_THREADS, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -456,7 +457,8 @@ int cfft_mixc_lookup(long long n, int dtype, int variant, const void** fn, int* 
 }
 
 const void* cfft_kernel_for(int mode, int dtype) {
-    if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE)
+    if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE ||
+        mode == MODE_CLUS)
         return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, false) : cfft_pass_kernel32(mode, false);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {
@@ -483,34 +485,17 @@ struct StaticFour {
     const void* fn;
     int single;                   // one shared buffer for both layouts
 };
-// 30240 = 168 x 180 on a 12-CTA cluster (ComplexF64 mixed-radix batch)
-using K_168x180_c12 = StatK<168, 180, 12, Seq<7, 3, 8>, true, 1, Seq<9, 5, 4>, true, 1>;
 // Rader M = 20160 = 168 x 120 on an 8-CTA cluster (primes 10007 .. 10081)
 using K_168x120_c8 = StatK<168, 120, 8, Seq<7, 3, 8>, true, 1, Seq<5, 3, 8>, true, 3>;
-// 30240 on a 6-CTA cluster with one shared buffer per CTA (two CTAs/SM at
-// twice the elements per CTA; 8 % faster than the 12-CTA kernel on B200),
-// each warp transforming two columns at a time (another 10 %)
-using K_168x180_c6s = StatK<168, 180, 6, Seq<7, 3, 8>, true, 2, Seq<9, 5, 4>, true, 1, true>;
-// single-buffer 12- and 8-CTA shapes at three CTAs/SM (EMAX 10 / 9)
-using K_168x180_c12s = StatK<168, 180, 12, Seq<7, 3, 8>, true, 1, Seq<9, 5, 4>, true, 1, true>;
+// with a single buffer, at three CTAs/SM (EMAX 9)
 using K_168x120_c8s = StatK<168, 120, 8, Seq<7, 3, 8>, true, 1, Seq<5, 3, 8>, true, 1, true>;
-// 65536 = 256 x 256 on a 16-CTA cluster (ComplexF32 precision form)
-using K_256x256_c16 = StatK<256, 256, 16, Seq<16, 16>, true, 2, Seq<16, 16>, true, 2>;
 
 static const StaticFour kStatic[] = {
     //                        9  7  5  3 16  8  4  2
-    {CFFT_DT_C128, 168, 180, 12, {0, 1, 0, 1, 0, 1, 0, 0}, {1, 0, 1, 0, 0, 0, 1, 0},
-     (const void*)k_four_mb<double2, 10, K_168x180_c12s, 3>, 1},
-    {CFFT_DT_C64, 168, 180, 12, {0, 1, 0, 1, 0, 1, 0, 0}, {1, 0, 1, 0, 0, 0, 1, 0},
-     (const void*)k_four<float2, CFFT_EMAX, K_168x180_c12>, 0},
     {CFFT_DT_C128, 168, 120, 8, {0, 1, 0, 1, 0, 1, 0, 0}, {0, 0, 1, 1, 0, 1, 0, 0},
      (const void*)k_four_mb<double2, 9, K_168x120_c8s, 3>, 1},
     {CFFT_DT_C64, 168, 120, 8, {0, 1, 0, 1, 0, 1, 0, 0}, {0, 0, 1, 1, 0, 1, 0, 0},
      (const void*)k_four<float2, CFFT_EMAX, K_168x120_c8>, 0},
-    {CFFT_DT_C128, 168, 180, 6, {0, 1, 0, 1, 0, 1, 0, 0}, {1, 0, 1, 0, 0, 0, 1, 0},
-     (const void*)k_four<double2, CFFT_EMAX, K_168x180_c6s>, 1},
-    {CFFT_DT_C64, 256, 256, 16, {0, 0, 0, 0, 2, 0, 0, 0}, {0, 0, 0, 0, 2, 0, 0, 0},
-     (const void*)k_four<float2, CFFT_EMAX, K_256x256_c16>, 0},
 };
 
 const void* cfft_static_four(int dtype, int N1, int N2, int C, const unsigned char* ca,

@@ -8,6 +8,9 @@
 #define CFFT_DT_C64 1
 #define CFFT_EMAX 16
 #define CFFT_THREADS 256
+// threads per CTA of the cluster four-step kernels (MODE_CLUS)
+#define CFFT_CLUS32 384
+#define CFFT_CLUS64 256
 
 #include "engine_types.h"
 
@@ -88,7 +91,7 @@ cudaError_t cfft_launch_fn(const void* fn, const KParams& p, unsigned grid, int 
 cudaError_t cfft_max_active_clusters_fn(const void* fn, int threads, size_t smem, int cluster, int* out);
 // batched (descriptor-driven) kernels
 const void* cfft_batch_kernel_for(int mode, int dtype);
-cudaError_t cfft_launch_batch(const void* fn, const BatchLaunch& L, unsigned grid, size_t smem,
+cudaError_t cfft_launch_batch(const void* fn, const BatchLaunch& L, unsigned grid, int threads, size_t smem,
                               int cluster, cudaStream_t stream);
 // the batched form's persistent queue kernel (QueueLaunch, queue.cu), built
 // for mb = 2 or 3 CTAs per SM, its launcher (ctl must be zero) and its

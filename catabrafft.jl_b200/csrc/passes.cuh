@@ -10,6 +10,10 @@
 //            intermediate: N2-point DFT, product with the FP64 spectrum,
 //            conjugation, N2-point DFT that takes the digits in reverse
 //            order, four-step twiddle w_M^(k1 j2)
+//   CLUS     one transform on a cluster of C CTAs: COLPASS's stages over N2 / C
+//            columns in each CTA, whose last stage writes the twiddled values
+//            through distributed shared memory into the rows of the CTA that
+//            owns them, then ROWPASS's stages over N1 / C rows
 //   LINE     V whole transforms that fit a CTA, one row each: one kernel from
 //            the caller's input to the caller's output
 //
@@ -283,7 +287,7 @@ __device__ __forceinline__ void row_first(const KParams& p, V* buf, const V* src
 // a middle stage; LANES_W: adjacent lanes take adjacent rows (as COLPASS's
 // adjacent columns), else adjacent butterflies of a row.  BACK: the second
 // transform's stage on the same digit
-template <typename V, int R, bool LANES_W, bool BACK>
+template <typename V, int R, bool LANES_W, bool BACK, int T = CFFT_THREADS>
 __device__ __forceinline__ void row_mid(const KParams& p, V* buf, int s, int Ls, int rows) {
     const SfPlan& S = p.sc;
     const int nb = Ls / R, per = S.L / R, qp = p.qp;
@@ -291,7 +295,7 @@ __device__ __forceinline__ void row_mid(const KParams& p, V* buf, int s, int Ls,
     const V* tw = (const V*)S.tw + (BACK ? S.boff[s] : S.off[s]);
     const int tid = opaque_tid(), k0 = LANES_W ? sf_div(tid, p.mv) : 0;
     const int total = LANES_W ? (k0 < p.ks ? per : 0) : rows * per;
-    for (int i = LANES_W ? k0 : tid; i < total; i += LANES_W ? p.ks : CFFT_THREADS) {
+    for (int i = LANES_W ? k0 : tid; i < total; i += LANES_W ? p.ks : T) {
         int r, b;
         if (LANES_W) {
             r = tid - k0 * p.V;
@@ -314,12 +318,13 @@ __device__ __forceinline__ void row_mid(const KParams& p, V* buf, int s, int Ls,
 }
 
 // ---------------------------------------------------------------- ROWPASS
+// thread -> row r of the tile and butterflies k0, k0 + ks, ... (adjacent lanes
+// take adjacent rows: adjacent outputs)
 template <typename V, int R>
-__device__ __forceinline__ void row_last(const KParams& p, const V* buf, int t, int r0, int rows) {
+__device__ __forceinline__ void row_last(const KParams& p, const V* buf, int t, int r0, int r, int k0, int ks) {
     const SfPlan& S = p.sc;
-    const int per = S.L / R, N1 = p.N1, tid = opaque_tid(), k0 = sf_div(tid, p.mv), r = tid - k0 * p.V;
-    if (k0 >= p.ks || r >= rows) return;
-    for (int b = k0; b < per; b += p.ks) {
+    const int per = S.L / R, N1 = p.N1;
+    for (int b = k0; b < per; b += ks) {
         const V* e = buf + r * p.qw + b * p.qp;
         V v[R];
 #pragma unroll
@@ -357,7 +362,9 @@ template <typename V> __device__ __forceinline__ void rowpass_body(const KParams
         __syncthreads();
         Ls /= S.r[s];
     }
-#define SF_CALL(R) row_last<V, R>(p, buf, t, r0, rows)
+    const int tid = opaque_tid(), k0 = sf_div(tid, p.mv), r = tid - k0 * p.V;
+    if (k0 >= p.ks || r >= rows) return;
+#define SF_CALL(R) row_last<V, R>(p, buf, t, r0, r, k0, p.ks)
     SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
 }
@@ -557,6 +564,82 @@ template <typename V> __device__ __forceinline__ void line_body(const KParams& p
         Ls /= S.r[s];
     }
 #define SF_CALL(R) line_last<V, R>(p, buf, t0, rows)
+    SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
+#undef SF_CALL
+}
+
+// ------------------------------------------------------------------- CLUS
+// the last column stage: output k1 = K + total j of column i2 goes, twiddled,
+// to row k1 % R1 of CTA k1 / R1, whose row buffer nobody reads before the
+// cluster barrier that follows
+template <typename V, int R>
+__device__ __forceinline__ void clus_exchange(const KParams& p, const V* buf, V* rowbuf, const ColThread& c) {
+    cg::cluster_group cl = cg::this_cluster();
+    const SfPlan& S = p.sa;
+    const int total = S.L / R, W = p.V, R1 = p.N1 / p.C, at = row_at(p.sc, c.col, p.qp);
+    const double2 st = tw_two(p.t4, (unsigned)(c.col * total));
+    for (int b = c.k0; b < total; b += p.ks) {
+        const V* e = buf + b * R * W + c.w;
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m * W];
+        sf_dft<R>(v);
+        const int K = sf_index(S, S.np - 1, b);
+        double2 wk = tw_two(p.t4, (unsigned)(c.col * K));
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const int k1 = K + total * j, d = sf_div(k1, p.mr1);
+            V* dst = cl.map_shared_rank(rowbuf, d);
+            dst[(k1 - d * R1) * p.qw + at] = cmul(v[j], fromd<V>(wk));
+            if (j < R - 1) wk = cmul(wk, st);
+        }
+    }
+}
+template <typename V, int T> __device__ __forceinline__ void clus_body(const KParams& p, unsigned char* smem) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), t = block_id(p) / p.C;
+    if (t >= p.batch) return;                   // uniform across the cluster
+    V* buf = (V*)smem;                          // N1 x W columns
+    V* rowbuf = buf + p.N1 * p.V;               // R1 rows
+    {
+        const SfPlan& S = p.sa;
+        ColThread c;
+        const int tid = opaque_tid();
+        c.k0 = sf_div(tid, p.mv);
+        c.w = tid - c.k0 * p.V;
+        c.col = rank * p.V + c.w;
+        c.ok = c.k0 < p.ks;
+#define SF_CALL(R) col_first<V, R>(p, buf, t, c)
+        if (c.ok) { SF_SWITCH(S.r[0], SF_CALL) }
+#undef SF_CALL
+        __syncthreads();
+        int Ls = S.L / S.r[0];
+        for (int s = 1; s < S.np - 1; s++) {
+#define SF_CALL(R) col_mid<V, R>(p, buf, s, Ls, c)
+            if (c.ok) { SF_SWITCH(S.r[s], SF_CALL) }
+#undef SF_CALL
+            __syncthreads();
+            Ls /= S.r[s];
+        }
+        cl.sync();                              // every CTA of the cluster has started
+#define SF_CALL(R) clus_exchange<V, R>(p, buf, rowbuf, c)
+        if (c.ok) { SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL) }
+#undef SF_CALL
+    }
+    cl.sync();                                  // rows complete; no remote access after this
+    const SfPlan& S = p.sc;
+    const int R1 = p.N1 / p.C;
+    int Ls = S.L;
+    for (int s = 0; s < S.np - 1; s++) {
+#define SF_CALL(R) row_mid<V, R, false, false, T>(p, rowbuf, s, Ls, R1)
+        SF_SWITCH(S.r[s], SF_CALL)
+#undef SF_CALL
+        __syncthreads();
+        Ls /= S.r[s];
+    }
+    const int tid = opaque_tid(), k0 = sf_div(tid, p.mr1), r = tid - k0 * R1;
+    if (k0 >= p.ks2) return;
+#define SF_CALL(R) row_last<V, R>(p, rowbuf, t, rank * R1, r, k0, p.ks2)
     SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
 }

@@ -25,12 +25,27 @@ __global__ void __launch_bounds__(CFFT_THREADS, PassBlocks<V>::value) kb_pass(Ba
     __shared__ KParams sp;
     pass_body<V, MODE>(stage_params<V>(L, &sp), smem);
 }
+// cluster kernels: 384 ComplexF32 threads (two CTAs per SM at 80 registers, as
+// many warps as three of 256) or 256 ComplexF64 ones
+template <typename V> struct ClusThreads { static constexpr int value = CFFT_CLUS32; };
+template <> struct ClusThreads<double2> { static constexpr int value = CFFT_CLUS64; };
+template <typename V>
+__global__ void __launch_bounds__(ClusThreads<V>::value, 2) k_clus(const __grid_constant__ KParams p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    clus_body<V, ClusThreads<V>::value>(p, smem);
+}
+template <typename V> __global__ void __launch_bounds__(ClusThreads<V>::value, 2) kb_clus(BatchLaunch L) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ KParams sp;
+    clus_body<V, ClusThreads<V>::value>(stage_params<V>(L, &sp), smem);
+}
 template <typename V> const void* pass_kernel(int mode, bool batched) {
     switch (mode) {
         case MODE_COLPASS: return batched ? (const void*)kb_pass<V, MODE_COLPASS> : (const void*)k_pass<V, MODE_COLPASS>;
         case MODE_ROWPASS: return batched ? (const void*)kb_pass<V, MODE_ROWPASS> : (const void*)k_pass<V, MODE_ROWPASS>;
         case MODE_MIDPASS: return batched ? (const void*)kb_pass<V, MODE_MIDPASS> : (const void*)k_pass<V, MODE_MIDPASS>;
         case MODE_LINE: return batched ? (const void*)kb_pass<V, MODE_LINE> : (const void*)k_pass<V, MODE_LINE>;
+        case MODE_CLUS: return batched ? (const void*)kb_clus<V> : (const void*)k_clus<V>;
     }
     return nullptr;
 }

@@ -247,3 +247,23 @@ inline void sf_stage(KParams& k, size_t e, size_t* smem) {
     k.qw = sf_qw(k.sc, k.V, e, mid);
     *smem = k.mode == MODE_COLPASS ? sf_col_smem(k.sa, k.V, e) : sf_row_smem(k.sc, k.V, e, mid);
 }
+// CLUS: shared memory and cost per element of an N1 x N2 split on C CTAs
+inline size_t sf_clus_smem(const SfPlan& a, const SfPlan& c, int C, size_t e) {
+    return ((size_t)a.L * (c.L / C) + (size_t)(a.L / C) * sf_qw(c, a.L / C, e, false)) * e;
+}
+inline double sf_clus_cost(const SfPlan& a, const SfPlan& c, int C, size_t e, int threads) {
+    const int W = c.L / C, R1 = a.L / C;
+    if (W > threads || R1 > threads) return 1e9;
+    const int kc = threads / W, kr = threads / R1;
+    double t = sf_start() + 2000.0;
+    for (int s = 0; s < a.np; s++) t += sf_round(a.r[s], 1) * ((a.L / a.r[s] + kc - 1) / kc);
+    for (int s = 0; s < c.np; s++) {
+        const int nb = c.L / c.r[s];
+        t += sf_round(c.r[s], 1) * (s == c.np - 1 ? (nb + kr - 1) / kr : (R1 * nb + threads - 1) / threads);
+    }
+    if (sf_clus_smem(a, c, C, e) > 112 * 1024) t *= 1.6;
+    for (long long seg : {W * (long long)e, R1 * (long long)e})
+        t *= seg < 32 ? 1.6 : seg < 64 ? 1.2 : seg < 128 ? 1.05 : 1.0;
+    if (W < 32) t *= 1.2;          // the exchange writes runs of W elements
+    return t * (1.0 + 0.02 * C + (C > 8 ? 0.3 : 0.0)) / ((double)a.L * W);
+}

@@ -430,8 +430,41 @@ static size_t four_smem_bytes(int64_t M, int64_t twA, int64_t twC, int64_t bufsz
     return b;
 }
 
+// CLUS shapes of a smooth length, best first
+static int clus_threads(int dtype) { return dtype == CFFT_C128 ? CFFT_CLUS64 : CFFT_CLUS32; }
+static void clus_candidates(int64_t M, int dtype, std::vector<Shape>& out) {
+    const size_t e = elem_bytes(dtype);
+    std::vector<Shape> v;
+    for (int64_t N1 = 4; N1 <= kSfMax; N1++) {
+        if (M % N1) continue;
+        const int64_t N2 = M / N1;
+        if (N2 < 4 || N2 > kSfMax) continue;
+        const SfPlan *a = sf_get(N1), *c = sf_get(N2);
+        if (!a || !c) continue;
+        for (int C = 2; C <= 16; C++) {
+            if (N1 % C || N2 % C || sf_clus_smem(*a, *c, C, e) > kSmemMax) continue;
+            Shape sh;
+            sh.score = sf_clus_cost(*a, *c, C, e, clus_threads(dtype));
+            if (sh.score >= 1e9) continue;
+            sh.mode = MODE_FOUR;
+            sh.M = M;
+            sh.N1 = (int)N1;
+            sh.N2 = (int)N2;
+            sh.C = C;
+            sh.ra = sf_radices(*a);
+            sh.rc = sf_radices(*c);
+            sh.smem = sh.smem_dyn = sf_clus_smem(*a, *c, C, e);
+            v.push_back(sh);
+        }
+    }
+    std::sort(v.begin(), v.end(), [](const Shape& a, const Shape& b) { return a.score < b.score; });
+    if (v.size() > 8) v.resize(8);
+    out.insert(out.end(), v.begin(), v.end());
+}
+
 static void four_candidates(int64_t M, int64_t nx, int conv, int dtype, std::vector<Shape>& out) {
     size_t e = elem_bytes(dtype);
+    if (conv == CONV_NONE) return clus_candidates(M, dtype, out);
     for (int64_t N1 = 2; N1 <= 4096; N1++) {
         if (M % N1) continue;
         int64_t N2 = M / N1;
@@ -732,14 +765,17 @@ static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch) 
     if (M > 64) four_candidates(M, n, conv, dtype, v);
     Shape g;
     if ((v.empty() || M >= 16384) && twopass_shape(n, conv, M, dtype, g)) {
-        // beyond a cluster (or as the timed planners' alternative to one).
-        // Measured on B200: from 2^15 points the two passes beat a cluster
-        // for ComplexF32 transforms (1.3-1.5x at 2^16-2^17) and for
-        // power-of-two ComplexF64 ones (1.3x at 2^15, 1.7x at 2^16);
-        // otherwise second in line, so the heuristic keeps a single-kernel
-        // shape and MEASURE/ENCHANT time both
+        // beyond a cluster, or in place of one.  Measured on B200: a batch of
+        // 32 MB or more of smooth transforms runs faster as two passes than
+        // on clusters (ComplexF64 60480 x 256 317 against 530 us, 24000 x 512
+        // 200 / 253; ComplexF32 48000 x 256 134 / 153, 24000 x 1024 211 / 222),
+        // a few of them faster on clusters, one launch and no intermediate
+        // (60480 x 1 17 / 26, 24000 x 32 ComplexF32 15 / 20; 64 x 19683 21 /
+        // 24); from 2^15 points ComplexF32 clusters no longer win either way.
+        // Otherwise second in line, so that MEASURE / ENCHANT time both
         const bool pow2 = (M & (M - 1)) == 0;
-        const bool first = (dtype == CFFT_C64 || pow2) && conv == CONV_NONE && M >= 32768;
+        const bool first = conv == CONV_NONE && (((dtype == CFFT_C64 || pow2) && M >= 32768) ||
+                                                 (double)batch * (double)M * (double)elem_bytes(dtype) >= 32.0 * (1 << 20));
         v.insert(v.begin() + (first ? 0 : std::min<size_t>(v.size(), 1)), g);
     }
     // the register kernels lead for the lengths they cover
@@ -770,7 +806,8 @@ static std::string shape_desc(const Shape& s, int64_t n) {
                (s.var == 1 ? ",tma" : s.var == 2 ? ",dataflow" : "") + ")";
     if (s.mode == MODE_FOUR)
         return pre + "four(C=" + std::to_string(s.C) + ",N1=" + std::to_string(s.N1) +
-               ",N2=" + std::to_string(s.N2) + ")[" + join(s.ra) + "|" + join(s.rc) + "]";
+               ",N2=" + std::to_string(s.N2) + ")[" +
+               (s.conv == CONV_NONE ? join_raw(s.ra) + "|" + join_raw(s.rc) : join(s.ra) + "|" + join(s.rc)) + "]";
     return pre + "twopass(N1=" + std::to_string(s.N1) + ",N2=" + std::to_string(s.N2) + ")[" +
            join_raw(s.ra) + "|" + join_raw(s.rc) + "]";
 }
@@ -1350,6 +1387,48 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         P->chunk = P->batch;
         return CFFT_OK;
     }
+    if (sh.mode == MODE_FOUR && sh.conv == CONV_NONE) {
+        const int T = clus_threads(P->dtype), R1 = sh.N1 / sh.C;
+        rc = make_sfplan(P, sh.N1, kp.sa);
+        if (rc) return rc;
+        rc = make_sfplan(P, sh.N2, kp.sc);
+        if (rc) return rc;
+        rc = make_twolevel(P, sh.M, kp.t4);
+        if (rc) return rc;
+        kp.mode = MODE_CLUS;
+        kp.N1 = sh.N1;
+        kp.N2 = sh.N2;
+        kp.C = sh.C;
+        kp.V = sh.N2 / sh.C;
+        kp.mv = sf_magic(kp.V);
+        kp.ks = T / kp.V;
+        kp.mr1 = sf_magic(R1);
+        kp.ks2 = T / R1;
+        kp.qp = sf_qp(kp.sc, R1, e, false);
+        kp.qw = sf_qw(kp.sc, R1, e, false);
+        kp.pre = PRE_NONE;
+        kp.post = POST_TWIDDLE;
+        Stage s;
+        s.kp = kp;
+        s.threads = T;
+        s.smem = sh.smem;
+        s.cluster = sh.C;
+        s.grid = 0;
+        s.in_sel = 0;
+        s.out_sel = 1;
+        s.fn = cfft_kernel_for(MODE_CLUS, P->dtype);
+        CUDA_TRY(cfft_prepare_fn(s.fn, s.smem, sh.C));
+        int nclusters = 0;
+        cudaError_t ce = cfft_max_active_clusters_fn(s.fn, T, s.smem, sh.C, &nclusters);
+        if (ce != cudaSuccess || nclusters < 1) {
+            cudaGetLastError();
+            return fail(CFFT_ERR_UNSUPPORTED, "cluster configuration not schedulable: C=" + std::to_string(sh.C));
+        }
+        s.max_units = nclusters;
+        P->stages.push_back(s);
+        P->chunk = P->batch;
+        return CFFT_OK;
+    }
     if (sh.mode == MODE_FOUR) {
         kp.mode = MODE_FOUR;
         kp.N1 = sh.N1;
@@ -1661,7 +1740,7 @@ static int plan_execute(cfft_plan_s* P, const void* in, void* out, int dir, cuda
             unsigned grid;
             if (p2) grid = (unsigned)kp.batch;
             else if (kp.mode == MODE_ROWS || kp.mode == MODE_LINE) grid = (unsigned)((nb + kp.V - 1) / kp.V);
-            else if (kp.mode == MODE_FOUR || kp.mode == MODE_CONVC || kp.mode == MODE_MIXC || kp.mode == MODE_P2CL)
+            else if (kp.mode == MODE_FOUR || kp.mode == MODE_CLUS || kp.mode == MODE_CONVC || kp.mode == MODE_MIXC || kp.mode == MODE_P2CL)
                 grid = (unsigned)(nb * kp.C);
             else if (s.cols) {
                 kp.batch = 1;
@@ -1768,7 +1847,7 @@ static bool io_fusable(const cfft_plan_s* P) {
     for (const auto& st : P->stages) {
         const int m = st.kp.mode;
         if (m != MODE_ROWS && m != MODE_FOUR && m != MODE_COLPASS && m != MODE_ROWPASS && m != MODE_MIDPASS &&
-            m != MODE_LINE)
+            m != MODE_LINE && m != MODE_CLUS)
             return false;
         if (st.launch != 0 || st.fn == cfft_r4096_kernel(P->dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64))
             return false;
@@ -2049,11 +2128,11 @@ static size_t batched_smem(const Stage& st) { return st.smem_batched ? st.smem_b
 static bool single_kernel(const cfft_plan_s* P) {
     return P->stages.size() == 1 &&
            (P->stages[0].kp.mode == MODE_ROWS || P->stages[0].kp.mode == MODE_FOUR ||
-            P->stages[0].kp.mode == MODE_LINE);
+            P->stages[0].kp.mode == MODE_LINE || P->stages[0].kp.mode == MODE_CLUS);
 }
 // CTAs one parameter block occupies in a batched launch
 static int blocks_for(const KParams& kp) {
-    if (kp.mode == MODE_FOUR) return kp.C;
+    if (kp.mode == MODE_FOUR || kp.mode == MODE_CLUS) return kp.C;
     if (kp.mode == MODE_COLPASS) return (kp.N2 + kp.V - 1) / kp.V;
     if (kp.mode == MODE_ROWPASS || kp.mode == MODE_MIDPASS) return (kp.N1 + kp.V - 1) / kp.V;
     return 1;
@@ -2071,6 +2150,10 @@ static const void* batched_variant(KParams& kp, int dtype) {
 
 // launches are grouped by how many CTAs fit an SM (two below ~113 KB of
 // shared memory, one above); a group runs with its largest member's size
+static int batched_threads(const void* fn, int dtype) {
+    return fn == cfft_batch_kernel_for(MODE_CLUS, dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64) ? clus_threads(dtype)
+                                                                                             : CFFT_THREADS;
+}
 static int smem_class(size_t smem) { return smem <= (size_t)112 * 1024 ? 0 : 1; }
 // one launch: parameter blocks (largest first) and the block -> block map
 template <class ItemT>
@@ -2464,7 +2547,7 @@ static int batch_enqueue(cfft_batch_s* B, const void* in, void* out, int dir, cu
             L.out_base = out;
             L.dir = dir;
             L.pad_ = 0;
-            cudaError_t ce = cfft_launch_batch(g.fn, L, g.grid, g.smem, g.cluster, st);
+            cudaError_t ce = cfft_launch_batch(g.fn, L, g.grid, batched_threads(g.fn, B->dtype), g.smem, g.cluster, st);
             if (ce != cudaSuccess)
                 return fail(CFFT_ERR_CUDA, std::string("batched launch: ") + cudaGetErrorString(ce));
             launches++;
@@ -2681,7 +2764,7 @@ static int serve_launch(cfft_server_s* S, ServeSlot& sl) {
         L.out_base = nullptr;
         L.dir = -1;
         L.pad_ = 0;
-        cudaError_t ce = cfft_launch_batch(g.fn, L, g.grid, g.smem, g.cluster, sl.st);
+        cudaError_t ce = cfft_launch_batch(g.fn, L, g.grid, batched_threads(g.fn, S->dtype), g.smem, g.cluster, sl.st);
         if (ce != cudaSuccess) return fail(CFFT_ERR_CUDA, std::string("serve launch: ") + cudaGetErrorString(ce));
     }
     CUDA_TRY(cudaEventRecord(sl.ev, sl.st));
