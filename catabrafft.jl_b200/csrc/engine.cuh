@@ -506,124 +506,6 @@ __device__ __forceinline__ void r4096_body(const KParams& p, unsigned char* smem
     }
 }
 
-// ---------------------------------------------------------------- ROWS mode
-// smem: buf[V][PC] (+ for Rader: xs[V][XP]) + reduction scratch
-template <typename V, int EMAX>
-__device__ __forceinline__ void rows_body(const KParams& p, unsigned char* smem) {
-    const int T = blockDim.x, tid = opaque_tid();
-    V* buf = (V*)smem;
-    V* xs = buf + (size_t)p.V * p.PC;
-    const int t0 = block_id(p) * p.V;
-    const int nrows = min(p.V, p.batch - t0);
-    if (nrows <= 0) return;
-    const int nx = p.nx, M = p.M;
-
-    if (p.conv == CONV_NONE) {
-        if (p.in_fmt == IO_PLAIN) {
-            const V* in = (const V*)p.in + (long long)t0 * p.in_dist;
-            for (int idx = tid; idx < nrows * nx; idx += T) {
-                const int r = fdiv(idx, p.mX), i = idx - r * nx;
-                buf[r * p.PC + i] = load_in(p, ldg_stream(in + (long long)r * p.in_dist + i));
-            }
-        } else {
-            for (int idx = tid; idx < nrows * nx; idx += T) {
-                const int r = fdiv(idx, p.mX), i = idx - r * nx;
-                buf[r * p.PC + i] = load_in(p, user_ld<V>(p, t0 + r, i));
-            }
-        }
-        __syncthreads();
-        run_subffts<V, EMAX>(buf, p.pc, nrows, 1, p.PC);
-        if (p.out_fmt == IO_PLAIN) {
-            V* out = (V*)p.out + (long long)t0 * p.out_dist;
-            for (int idx = tid; idx < nrows * nx; idx += T) {
-                const int r = fdiv(idx, p.mX), i = idx - r * nx;
-                stg_stream(out + (long long)r * p.out_dist + i, store_out(p, buf[r * p.PC + i]));
-            }
-        } else {
-            for (int idx = tid; idx < nrows * nx; idx += T) {
-                const int r = fdiv(idx, p.mX), i = idx - r * nx;
-                user_st(p, t0 + r, i, store_out(p, buf[r * p.PC + i]));
-            }
-        }
-        return;
-    }
-
-    if (p.conv == CONV_RADER) {
-        for (int idx = tid; idx < nrows * nx; idx += T) {
-            const int r = fdiv(idx, p.mX), i = idx - r * nx;
-            xs[r * p.XP + i] = load_in(p, user_ld<V>(p, t0 + r, i));
-        }
-        __syncthreads();
-        const int L = nx - 1;
-        for (int idx = tid; idx < nrows * M; idx += T) {
-            const int r = fdiv(idx, p.mM), j = idx - r * M;
-            buf[r * p.PC + j] = (j < L) ? xs[r * p.XP + __ldg(p.perm + j)] : zero<V>();
-        }
-    } else {
-        for (int idx = tid; idx < nrows * M; idx += T) {
-            const int r = fdiv(idx, p.mM), j = idx - r * M;
-            V v = zero<V>();
-            if (j < nx) {
-                V x = load_in(p, user_ld<V>(p, t0 + r, j));
-                v = fromd<V>(cmul(tod(x), __ldg(p.chirp + j)));
-            }
-            buf[r * p.PC + j] = v;
-        }
-    }
-    __syncthreads();
-    run_subffts<V, EMAX>(buf, p.pc, nrows, 1, p.PC);
-    for (int idx = tid; idx < nrows * M; idx += T) {
-        const int r = fdiv(idx, p.mM), k = idx - r * M;
-        V* e = buf + r * p.PC + k;
-        *e = conjv(fromd<V>(cmul(tod(*e), __ldg(p.spec + k))));
-    }
-    __syncthreads();
-    run_subffts<V, EMAX>(buf, p.pc, nrows, 1, p.PC);
-
-    if (p.conv == CONV_RADER) {
-        const int L = nx - 1;
-        // y[g^-j] = x0 + c[j]  (prime.jl:76-78), written into the staging rows
-        for (int idx = tid; idx < nrows * L; idx += T) {
-            const int r = fdiv(idx, p.mL), j = idx - r * L;
-            const V x0 = xs[r * p.XP];
-            const V c = conjv(buf[r * p.PC + j]);
-            buf[r * p.PC + j] = mk<V>(x0.x + c.x, x0.y + c.y);  // park result in place
-        }
-        __syncthreads();
-        // y0 = x0 + sum(x[1:]) per row, reduced in FP64
-        double2* red = after16(xs + (size_t)p.V * p.XP);
-        for (int r = 0; r < nrows; r++) {
-            double2 acc = make_double2(0, 0);
-            for (int i = 1 + tid; i < nx; i += T) {
-                double2 d = tod(xs[r * p.XP + i]);
-                acc.x += d.x; acc.y += d.y;
-            }
-            double2 s = block_sum(acc, red);
-            if (tid == 0) {
-                double2 x0 = tod(xs[r * p.XP]);
-                xs[r * p.XP] = fromd<V>(make_double2(x0.x + s.x, x0.y + s.y));
-            }
-        }
-        __syncthreads();
-        for (int idx = tid; idx < nrows * L; idx += T) {
-            const int r = fdiv(idx, p.mL), j = idx - r * L;
-            xs[r * p.XP + __ldg(p.iperm + j)] = buf[r * p.PC + j];
-        }
-        __syncthreads();
-        for (int idx = tid; idx < nrows * nx; idx += T) {
-            const int r = fdiv(idx, p.mX), i = idx - r * nx;
-            user_st(p, t0 + r, i, store_out(p, xs[r * p.XP + i]));
-        }
-    } else {
-        for (int idx = tid; idx < nrows * nx; idx += T) {
-            const int r = fdiv(idx, p.mX), k = idx - r * nx;
-            const V c = conjv(buf[r * p.PC + k]);
-            const V y = fromd<V>(cmul(tod(c), __ldg(p.chirp + k)));
-            user_st(p, t0 + r, k, store_out(p, y));
-        }
-    }
-}
-
 // ---------------------------------------------------------------- FOUR mode
 // Column layout (step A): (i1, j) at i1*PA + j, j < W = N2/C
 // Row layout    (step C): (r, i2) at r*PC + i2, r < N1/C

@@ -57,7 +57,7 @@ struct TwoLevel {                 // w_N^e = lo[e & mask] * hi[e >> bits]  (FP64
 
 enum { MODE_ROWS = 0, MODE_FOUR = 1, MODE_COLPASS = 2, MODE_ROWPASS = 3, MODE_P2COL = 4, MODE_P2ROW = 5,
        MODE_CONVC = 6, MODE_MIXC = 7, MODE_P2CL = 8, MODE_MIDPASS = 9, MODE_LINE = 10,
-       MODE_CLUS = 11 };
+       MODE_CLUS = 11, MODE_LCONV = 12 };
 // kernel selector only (KParams.mode stays MODE_FOUR): the generic four-step
 // kernel instantiated with warp-synchronous sub-transforms
 enum { MODE_FOUR_WARP = 16 };
@@ -135,7 +135,7 @@ struct BatchLaunch {
 // release of the scratch half its chunk reuses) and adds one to counter
 // `done` when finished.  Every wait is on items with smaller tickets, so the
 // queue drains whatever the residency.
-enum { QK_ROWS = 0, QK_FOUR = 1, QK_FOUR_WARP = 2, QK_COLPASS = 3, QK_ROWPASS = 4, QK_MIDPASS = 5, QK_LINE = 6 };
+enum { QK_COLPASS = 0, QK_ROWPASS = 1, QK_MIDPASS = 2, QK_LINE = 3, QK_LCONV = 4 };
 struct QItem {
     int desc;                     // parameter block
     int blk;                      // block within the parameter block

@@ -13,11 +13,6 @@
 template <typename V> struct MinBlocks { static constexpr int value = 2; };
 template <> struct MinBlocks<double2> { static constexpr int value = 2; };
 
-template <typename V, int EMAX>
-__global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) k_rows(KParams p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    rows_body<V, EMAX>(p, smem);
-}
 template <typename V, int EMAX, class K>
 __global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) k_four(KParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -31,12 +26,6 @@ __global__ void __launch_bounds__(CFFT_THREADS, MB) k_four_mb(KParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     four_body<V, EMAX, K>(p, smem);
 }
-template <typename V, int EMAX>
-__global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) kb_rows(BatchLaunch L) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ KParams sp;
-    rows_body<V, EMAX>(stage_params<V>(L, &sp), smem);
-}
 template <typename V, int EMAX, class K>
 __global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) kb_four(BatchLaunch L) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -46,17 +35,15 @@ __global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) kb_four(Bat
 
 const void* cfft_batch_kernel_for(int mode, int dtype) {
     if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE ||
-        mode == MODE_CLUS)
+        mode == MODE_LCONV || mode == MODE_CLUS)
         return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, true) : cfft_pass_kernel32(mode, true);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {
-            case MODE_ROWS: return (const void*)kb_rows<double2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)kb_four<double2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)kb_four<double2, CFFT_EMAX, DynK<1>>;
         }
     } else {
         switch (mode) {
-            case MODE_ROWS: return (const void*)kb_rows<float2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)kb_four<float2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)kb_four<float2, CFFT_EMAX, DynK<1>>;
         }
@@ -458,17 +445,15 @@ int cfft_mixc_lookup(long long n, int dtype, int variant, const void** fn, int* 
 
 const void* cfft_kernel_for(int mode, int dtype) {
     if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE ||
-        mode == MODE_CLUS)
+        mode == MODE_LCONV || mode == MODE_CLUS)
         return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, false) : cfft_pass_kernel32(mode, false);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {
-            case MODE_ROWS: return (const void*)k_rows<double2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)k_four<double2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)k_four<double2, CFFT_EMAX, DynK<1>>;
         }
     } else {
         switch (mode) {
-            case MODE_ROWS: return (const void*)k_rows<float2, CFFT_EMAX>;
             case MODE_FOUR: return (const void*)k_four<float2, CFFT_EMAX, DynK<0>>;
             case MODE_FOUR_WARP: return (const void*)k_four<float2, CFFT_EMAX, DynK<1>>;
         }

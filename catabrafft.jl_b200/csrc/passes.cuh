@@ -10,6 +10,10 @@
 //            intermediate: N2-point DFT, product with the FP64 spectrum,
 //            conjugation, N2-point DFT that takes the digits in reverse
 //            order, four-step twiddle w_M^(k1 j2)
+//   LCONV    V whole convolutions (Rader or Bluestein) that fit a CTA, one row
+//            of M points each: MIDPASS's stages between a prologue that reads
+//            the caller's input (through the generator permutation, or times
+//            the chirp) and an epilogue that writes the caller's output
 //   CLUS     one transform on a cluster of C CTAs: COLPASS's stages over N2 / C
 //            columns in each CTA, whose last stage writes the twiddled values
 //            through distributed shared memory into the rows of the CTA that
@@ -372,9 +376,9 @@ template <typename V> __device__ __forceinline__ void rowpass_body(const KParams
 // ---------------------------------------------------------------- MIDPASS
 // The last stage of the first transform leaves X[row][K + per j] of position
 // b = the butterfly's in its registers: times the spectrum (stored in this
-// order: entry row L + j per + b), conjugated, it is the input of the second
+// order: entry row L + j per + b; ONE: one spectrum for every row), conjugated, it is the input of the second
 // transform's first stage over the same digit.
-template <typename V, int R>
+template <typename V, int R, bool ONE>
 __device__ __forceinline__ void mid_center(const KParams& p, V* buf, int r0, int rows) {
     const SfPlan& S = p.sc;
     const int per = S.L / R, total = rows * per;
@@ -382,7 +386,7 @@ __device__ __forceinline__ void mid_center(const KParams& p, V* buf, int r0, int
     for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
         const int r = sf_div(i, S.mper[S.np - 1]), b = i - r * per;
         V* e = buf + r * p.qw + b * p.qp;
-        const double2* sp = p.spec + ((long long)(r0 + r) * S.L + b);
+        const double2* sp = p.spec + (ONE ? (long long)b : (long long)(r0 + r) * S.L + b);
         V v[R];
 #pragma unroll
         for (int m = 0; m < R; m++) v[m] = e[m];
@@ -442,7 +446,7 @@ template <typename V> __device__ __forceinline__ void midpass_body(const KParams
         __syncthreads();
         Ls /= S.r[s];
     }
-#define SF_CALL(R) mid_center<V, R>(p, buf, r0, rows)
+#define SF_CALL(R) mid_center<V, R, false>(p, buf, r0, rows)
     SF_SWITCH(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
     __syncthreads();
@@ -552,7 +556,7 @@ template <typename V> __device__ __forceinline__ void line_body(const KParams& p
     const int t0 = block_id(p) * p.V, rows = min(p.V, p.batch - t0);
     if (rows <= 0) return;                      // uniform across the CTA
 #define SF_CALL(R) line_first<V, R>(p, buf, t0, rows)
-    SF_SWITCH(S.r[0], SF_CALL)
+    SF_SWITCH_LAST(S.r[0], SF_CALL)
 #undef SF_CALL
     __syncthreads();
     int Ls = S.L / S.r[0];
@@ -566,6 +570,161 @@ template <typename V> __device__ __forceinline__ void line_body(const KParams& p
 #define SF_CALL(R) line_last<V, R>(p, buf, t0, rows)
     SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
+}
+
+// ------------------------------------------------------------------ LCONV
+// prologue + first stage: row r holds the zero-padded convolution input
+//   Rader      x[g^j], j < n - 1 (src/prime.jl:66-74)
+//   Bluestein  x[j] chirp[j], j < n
+// reads past the end go to the butterfly's first entry (or the last one), so
+// that no branch keeps the loads apart
+template <typename V, int R>
+__device__ __forceinline__ void lconv_first(const KParams& p, V* buf, int t0, int rows) {
+    const SfPlan& S = p.sc;
+    const int nb = S.L / R, total = rows * nb, len = p.conv == CONV_RADER ? p.nx - 1 : p.nx;
+    const int ds = sf_div(nb, S.mr[S.np - 1]) * p.qp;
+    const V* tw = (const V*)S.tw + S.off[0];
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = sf_div(i, S.mnb[0]), b = i - r * nb, b1 = min(b, len - 1);
+        V v[R];
+        if (p.conv == CONV_RADER) {
+            int g[R];
+#pragma unroll
+            for (int m = 0; m < R; m++) g[m] = __ldg(p.perm + (b + nb * m < len ? b + nb * m : b1));
+            if (p.in_fmt == IO_PLAIN) {
+                const V* x = (const V*)p.in + (long long)(t0 + r) * p.in_dist;
+#pragma unroll
+                for (int m = 0; m < R; m++) v[m] = x[g[m]];
+            } else {
+#pragma unroll
+                for (int m = 0; m < R; m++) v[m] = user_ld<V>(p, t0 + r, g[m]);
+            }
+        } else if (p.in_fmt == IO_PLAIN) {
+            const V* x = (const V*)p.in + (long long)(t0 + r) * p.in_dist;
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = ldg_stream(x + (b + nb * m < len ? b + nb * m : b1));
+        } else {
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = user_ld<V>(p, t0 + r, b + nb * m < len ? b + nb * m : b1);
+        }
+        if (p.dir) {
+#pragma unroll
+            for (int m = 0; m < R; m++) v[m] = conjv(v[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < R; m++) {
+            const int j = b + nb * m;
+            if (p.conv == CONV_BLUE) v[m] = fromd<V>(cmul(tod(v[m]), __ldg(p.chirp + (j < len ? j : b1))));
+            if (j >= len) v[m] = zero<V>();
+        }
+        sf_dft<R>(v);
+        sf_twiddle<R>(v, tw + b, nb);
+        V* e = buf + r * p.qw + row_at(S, b, p.qp);
+#pragma unroll
+        for (int m = 0; m < R; m++) e[m * ds] = v[m];
+    }
+}
+// last stage + epilogue: c[j] = the conjugated outputs j = b + nb m
+//   Rader      y[g^-j] = x[0] + c[j]  (x0: this row's, already conjugated)
+//   Bluestein  y[j] = c[j] chirp[j]
+template <typename V, int R>
+__device__ __forceinline__ void lconv_last(const KParams& p, const V* buf, const double2* x0, int t0, int rows) {
+    const SfPlan& S = p.sc;
+    const int nb = S.L / R, total = rows * nb, len = p.conv == CONV_RADER ? p.nx - 1 : p.nx;
+    const int ds = sf_div(nb, S.mr[S.np - 1]) * p.qp;
+    for (int i = opaque_tid(); i < total; i += CFFT_THREADS) {
+        const int r = sf_div(i, S.mnb[0]), b = i - r * nb, b1 = min(b, len - 1);
+        const V* e = buf + r * p.qw + row_at(S, b, p.qp);
+        V v[R];
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = e[m * ds];
+        sf_dft<R>(v);
+        int k[R];
+        if (p.conv == CONV_RADER) {
+            const V z = fromd<V>(x0[2 * r]);
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                k[m] = __ldg(p.iperm + (b + nb * m < len ? b + nb * m : b1));
+                const V c = conjv(v[m]);
+                v[m] = store_out(p, mk<V>(z.x + c.x, z.y + c.y));
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                k[m] = b + nb * m;
+                v[m] = store_out(p, fromd<V>(cmul(tod(conjv(v[m])), __ldg(p.chirp + (k[m] < len ? k[m] : b1)))));
+            }
+        }
+        if (p.out_fmt == IO_PLAIN) {
+            V* o = (V*)p.out + (long long)(t0 + r) * p.out_dist;
+#pragma unroll
+            for (int m = 0; m < R; m++)
+                if (b + nb * m < len) o[k[m]] = v[m];
+        } else {
+#pragma unroll
+            for (int m = 0; m < R; m++)
+                if (b + nb * m < len) user_st(p, t0 + r, k[m], v[m]);
+        }
+    }
+}
+template <typename V> __device__ __forceinline__ void lconv_body(const KParams& p, unsigned char* smem) {
+    V* buf = (V*)smem;
+    const SfPlan& S = p.sc;
+    const int t0 = block_id(p) * p.V, rows = min(p.V, p.batch - t0);
+    if (rows <= 0) return;                      // uniform across the CTA
+    double2* x0 = after16(buf + p.V * p.qw);    // per row: x[0], x[0] + the sum of the others
+    if (p.conv == CONV_RADER) {
+        // y[0] = x[0] + sum(x[1:]), summed in FP64 by one warp per row
+        // (src/prime.jl:63-65); the input may be overwritten later (in place)
+        const int lane = opaque_tid() & 31;
+        for (int r = opaque_tid() >> 5; r < rows; r += CFFT_THREADS / 32) {
+            double2 s = make_double2(0, 0);
+            for (int j = 1 + lane; j < p.nx; j += 32) {
+                const double2 d = tod(load_in(p, user_ld<V>(p, t0 + r, j)));
+                s.x += d.x;
+                s.y += d.y;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+                s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+            }
+            if (lane == 0) {
+                const double2 z = tod(load_in(p, user_ld<V>(p, t0 + r, 0)));
+                x0[2 * r] = z;
+                x0[2 * r + 1] = make_double2(z.x + s.x, z.y + s.y);
+            }
+        }
+    }
+#define SF_CALL(R) lconv_first<V, R>(p, buf, t0, rows)
+    SF_SWITCH(S.r[0], SF_CALL)
+#undef SF_CALL
+    __syncthreads();
+    int Ls = S.L / S.r[0];
+    for (int s = 1; s < S.np - 1; s++) {
+#define SF_CALL(R) row_mid<V, R, false, false>(p, buf, s, Ls, rows)
+        SF_SWITCH(S.r[s], SF_CALL)
+#undef SF_CALL
+        __syncthreads();
+        Ls /= S.r[s];
+    }
+#define SF_CALL(R) mid_center<V, R, true>(p, buf, 0, rows)
+    SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
+#undef SF_CALL
+    __syncthreads();
+    for (int s = S.np - 2; s >= 1; s--) {
+        Ls *= S.r[s];
+#define SF_CALL(R) row_mid<V, R, false, true>(p, buf, s, Ls, rows)
+        SF_SWITCH(S.r[s], SF_CALL)
+#undef SF_CALL
+        __syncthreads();
+    }
+#define SF_CALL(R) lconv_last<V, R>(p, buf, x0, t0, rows)
+    SF_SWITCH(S.r[0], SF_CALL)
+#undef SF_CALL
+    if (p.conv == CONV_RADER)
+        for (int r = opaque_tid(); r < rows; r += CFFT_THREADS)
+            user_st(p, t0 + r, 0, store_out(p, fromd<V>(x0[2 * r + 1])));
 }
 
 // ------------------------------------------------------------------- CLUS

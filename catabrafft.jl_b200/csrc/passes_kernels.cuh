@@ -12,7 +12,8 @@ template <typename V, int MODE> __device__ __forceinline__ void pass_body(const 
     if constexpr (MODE == MODE_COLPASS) colpass_body<V>(p, smem);
     else if constexpr (MODE == MODE_ROWPASS) rowpass_body<V>(p, smem);
     else if constexpr (MODE == MODE_MIDPASS) midpass_body<V>(p, smem);
-    else line_body<V>(p, smem);
+    else if constexpr (MODE == MODE_LINE) line_body<V>(p, smem);
+    else lconv_body<V>(p, smem);
 }
 template <typename V, int MODE>
 __global__ void __launch_bounds__(CFFT_THREADS, PassBlocks<V>::value) k_pass(const __grid_constant__ KParams p) {
@@ -45,6 +46,7 @@ template <typename V> const void* pass_kernel(int mode, bool batched) {
         case MODE_ROWPASS: return batched ? (const void*)kb_pass<V, MODE_ROWPASS> : (const void*)k_pass<V, MODE_ROWPASS>;
         case MODE_MIDPASS: return batched ? (const void*)kb_pass<V, MODE_MIDPASS> : (const void*)k_pass<V, MODE_MIDPASS>;
         case MODE_LINE: return batched ? (const void*)kb_pass<V, MODE_LINE> : (const void*)k_pass<V, MODE_LINE>;
+        case MODE_LCONV: return batched ? (const void*)kb_pass<V, MODE_LCONV> : (const void*)k_pass<V, MODE_LCONV>;
         case MODE_CLUS: return batched ? (const void*)kb_clus<V> : (const void*)k_clus<V>;
     }
     return nullptr;

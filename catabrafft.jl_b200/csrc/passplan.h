@@ -47,7 +47,12 @@ inline unsigned sf_magic(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) 
 inline bool sf_plan(int L, SfPlan& S) {
     S = SfPlan();
     S.L = L;
-    if (L < 2) return false;
+    if (L < 1) return false;
+    if (L == 1) {                      // the identity (LINE)
+        S.np = 2;
+        S.r[0] = S.r[1] = 1;
+        return true;
+    }
     int cur[SF_MAXS], best[SF_MAXS], n = SF_MAXS + 1;
     double c = 1e30;
     sf_search(L, 16, 0, 0.0, cur, best, &n, &c);
@@ -233,6 +238,31 @@ inline int sf_line_rows(const SfPlan& S, long long batch, size_t e) {
             best = V;
         }
     }
+    return best;
+}
+// LCONV: V rows of M points, and two FP64 values a row (Rader)
+inline size_t sf_lconv_smem(const SfPlan& S, int V, size_t e) {
+    return ((size_t)sf_qw(S, V, e, true) * V * e + 15) / 16 * 16 + (size_t)V * 32;
+}
+inline int sf_lconv_rows(const SfPlan& S, long long batch, size_t e, double* cost = nullptr) {
+    const long long slots = 148 * (e == 8 ? 3 : 2);
+    int best = 1;
+    double bc = 1e300;
+    for (int V = 1; V <= 256 && V <= batch; V++) {
+        if (V > 1 && sf_lconv_smem(S, V, e) > sf_budget(e)) break;
+        double c = sf_start();
+        for (int s = 0; s < S.np; s++) {
+            const long long rounds = ((long long)V * (S.L / S.r[s]) + SF_THREADS - 1) / SF_THREADS;
+            c += rounds * (s == S.np - 1 ? sf_round(S.r[s], 2) : 2.0 * sf_round(S.r[s], 1));
+        }
+        const double waves = (double)((batch + V - 1) / V) / (double)slots;
+        c *= waves < 4.0 ? std::ceil(waves) : waves + 0.5;
+        if (c < bc) {
+            bc = c;
+            best = V;
+        }
+    }
+    if (cost) *cost = bc;
     return best;
 }
 // tile, pitches and shared memory of a pass (mode, N1, N2, sa, sc set)

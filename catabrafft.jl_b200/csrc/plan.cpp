@@ -371,43 +371,44 @@ static const int kLineMax = 9216;    // whole transforms in a CTA (74 KB of Comp
 static const SfPlan* sf_get(int64_t L) {
     static const std::vector<SfPlan> tab = [] {
         std::vector<SfPlan> t(kLineMax + 1);
-        for (int l = 2; l <= kLineMax; l++)
+        for (int l = 1; l <= kLineMax; l++)
             if (!is_smooth7(l) || !sf_plan(l, t[l])) t[l].L = 0;
         return t;
     }();
-    return L >= 2 && L <= kLineMax && tab[L].L ? &tab[L] : nullptr;
+    return L >= 1 && L <= kLineMax && tab[L].L ? &tab[L] : nullptr;
 }
 static std::vector<int> sf_radices(const SfPlan& S) { return std::vector<int>(S.r, S.r + S.np); }
+// one CTA: LINE, or LCONV with the cheapest convolution length within 2 % of
+// the shortest
 static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch, Shape& sh) {
-    const SfPlan* line = conv == CONV_NONE ? sf_get(M) : nullptr;
-    if (line && sf_line_smem(*line, 1, elem_bytes(dtype)) <= sf_budget(elem_bytes(dtype))) {
-        // LINE (passes.cuh)
-        sh.mode = MODE_ROWS;
+    const size_t e = elem_bytes(dtype);
+    if (M > kLineMax) return false;
+    sh.mode = MODE_ROWS;
+    if (conv == CONV_NONE) {
+        const SfPlan* S = sf_get(M);
+        if (!S || sf_line_smem(*S, 1, e) > sf_budget(e)) return false;
         sh.M = M;
         // one row a CTA where the n = 4096 register kernel runs it
-        sh.V = M == 4096 ? 1 : sf_line_rows(*line, batch, elem_bytes(dtype));
-        sh.rc = sf_radices(*line);
-        sh.smem = sf_line_smem(*line, sh.V, elem_bytes(dtype));
+        sh.V = M == 4096 ? 1 : sf_line_rows(*S, batch, e);
+        sh.rc = sf_radices(*S);
+        sh.smem = sf_line_smem(*S, sh.V, e);
         return true;
     }
-    if (M > 4096) return false;
-    auto rc = radix_split(M);
-    if (M > 1 && rc.empty()) return false;
-    if (wave_G(rc, M, CFFT_THREADS) < 1) return false;
-    size_t e = elem_bytes(dtype);
-    int64_t PC = M + ((M % 2 == 0) ? 1 : 0);
-    int64_t XP = (conv == CONV_RADER) ? nx : 0;
-    size_t per_row = (size_t)(PC + XP) * e;
-    // rows per CTA: ~48 KB of smem, but keep >= ~2 CTAs per SM busy
-    int64_t V = std::max<int64_t>(1, (int64_t)(48 * 1024) / (int64_t)per_row);
-    int64_t need = (batch + 295) / 296;
-    V = std::max<int64_t>(1, std::min<int64_t>(V, need));
-    sh.mode = MODE_ROWS;
-    sh.M = M;
-    sh.V = (int)V;
-    sh.rc = rc;
-    sh.smem = (size_t)V * per_row + 64 * sizeof(double2) + 16;
-    return sh.smem <= kSmemMax;
+    double best = 1e300;
+    for (int64_t m = M; m <= M + M / 50 && m <= kLineMax; m++) {
+        const SfPlan* S = sf_get(m);
+        if (!S || S->r[S->np - 1] < 2 || sf_lconv_smem(*S, 1, e) > sf_budget(e)) continue;
+        double c;
+        const int V = sf_lconv_rows(*S, batch, e, &c);
+        if (c >= best) continue;
+        best = c;
+        sh.M = m;
+        sh.V = V;
+        sh.rc = sf_radices(*S);
+        sh.smem = sf_lconv_smem(*S, V, e);
+    }
+    (void)nx;
+    return best < 1e300;
 }
 
 // shared memory of a FOUR CTA: sub-transform twiddles, the two-level four-step
@@ -764,7 +765,7 @@ static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch) 
     }
     if (M > 64) four_candidates(M, n, conv, dtype, v);
     Shape g;
-    if ((v.empty() || M >= 16384) && twopass_shape(n, conv, M, dtype, g)) {
+    if ((v.empty() || M >= 16384 || (conv != CONV_NONE && M >= 8192)) && twopass_shape(n, conv, M, dtype, g)) {
         // beyond a cluster, or in place of one.  Measured on B200: a batch of
         // 32 MB or more of smooth transforms runs faster as two passes than
         // on clusters (ComplexF64 60480 x 256 317 against 530 us, 24000 x 512
@@ -774,8 +775,15 @@ static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch) 
         // 24); from 2^15 points ComplexF32 clusters no longer win either way.
         // Otherwise second in line, so that MEASURE / ENCHANT time both
         const bool pow2 = (M & (M - 1)) == 0;
-        const bool first = conv == CONV_NONE && (((dtype == CFFT_C64 || pow2) && M >= 32768) ||
-                                                 (double)batch * (double)M * (double)elem_bytes(dtype) >= 32.0 * (1 << 20));
+        const bool big = (double)batch * (double)M * (double)elem_bytes(dtype) >= 2.0 * (1 << 20);
+        // convolutions (C64 20011 x 64 60 against 128 us on a cluster, C128
+        // 20002 x 64 86 / 109, 10006 x 1 36 / 30); a ComplexF64 prime keeps
+        // Rader's algorithm, whose twiddles follow the reference, while a
+        // cluster holds it
+        const bool cfirst = (conv == CONV_BLUE || (conv == CONV_RADER && dtype == CFFT_C64)) && (M >= 32768 || big);
+        const bool first = cfirst ||
+                           (conv == CONV_NONE && (((dtype == CFFT_C64 || pow2) && M >= 32768) ||
+                                                 (double)batch * (double)M * (double)elem_bytes(dtype) >= 32.0 * (1 << 20)));
         v.insert(v.begin() + (first ? 0 : std::min<size_t>(v.size(), 1)), g);
     }
     // the register kernels lead for the lengths they cover
@@ -791,7 +799,7 @@ static std::string shape_desc(const Shape& s, int64_t n) {
     std::string c = s.conv == CONV_RADER ? "rader" : s.conv == CONV_BLUE ? "bluestein" : "";
     std::string pre = c.empty() ? "" : c + "(n=" + std::to_string(n) + ",M=" + std::to_string(s.M) + ")+";
     if (s.mode == MODE_ROWS)
-        return pre + "rows(V=" + std::to_string(s.V) + ")[" + (s.conv == CONV_NONE ? join_raw(s.rc) : join(s.rc)) + "]";
+        return pre + "rows(V=" + std::to_string(s.V) + ")[" + join_raw(s.rc) + "]";
     if (s.mode == MODE_P2CL)
         return "pow2cluster(C=" + std::to_string(s.C) + ",4096 per CTA,ctas_per_sm=" + std::to_string(s.V) +
                (s.var == 1 ? ",tma" : "") + ")";
@@ -1101,6 +1109,10 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
         }
         const int* iperm = kp.iperm;
         *spec_key = "sr/" + tag + "/" + std::to_string(exact);
+        if (sh.mode == MODE_ROWS)
+            return conv_spectrum_rows(P, *spec_key + "/c", 1, *sf_get(M), [&](double2* v) {
+                return cfft_gen_rader_b(v, iperm, n, M, exact, winv, 0);
+            }, &kp.spec);
         return conv_spectrum(P, *spec_key, M, [&](double2* v) {
             return cfft_gen_rader_b(v, iperm, n, M, exact, winv, 0);
         }, &kp.spec);
@@ -1114,8 +1126,9 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
     if (rc) return rc;
     kp.chirp = (const double2*)dch;
     const double2* ch = kp.chirp;
-    if (sh.mode == MODE_COLPASS)
-        return conv_spectrum_rows(P, "sc/" + tag + "/" + std::to_string(sh.N1), sh.N1, *sf_get(sh.N2),
+    if (sh.mode == MODE_COLPASS || sh.mode == MODE_ROWS)
+        return conv_spectrum_rows(P, "sc/" + tag + "/" + std::to_string(sh.mode == MODE_ROWS ? 1 : sh.N1),
+                                  sh.mode == MODE_ROWS ? 1 : sh.N1, *sf_get(sh.mode == MODE_ROWS ? sh.M : sh.N2),
                                   [&](double2* v) { return cfft_gen_bluestein_b(v, ch, n, M, 0); }, &kp.spec);
     *spec_key = "sb/" + tag;
     return conv_spectrum(P, *spec_key, M, [&](double2* v) {
@@ -1328,11 +1341,11 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     if (sh.mode == MODE_ROWS) {
         kp.mode = MODE_ROWS;
         kp.V = sh.V;
-        if (sh.conv == CONV_NONE && sh.M > 1) {
+        rc = make_sfplan(P, sh.M, kp.sc);
+        if (rc) return rc;
+        if (sh.conv == CONV_NONE) {
             // V rows per CTA in register stages (passes.cuh), or the persistent
             // register kernel of n = 4096
-            rc = make_sfplan(P, sh.M, kp.sc);
-            if (rc) return rc;
             kp.mode = MODE_LINE;
             kp.qp = sf_qp(kp.sc, 1, e, true);
             kp.q0 = sf_line_q0(kp.sc);
@@ -1366,13 +1379,9 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
             P->chunk = P->batch;
             return CFFT_OK;
         }
-        kp.PC = (int)(sh.M + ((sh.M % 2 == 0) ? 1 : 0));
-        kp.XP = (sh.conv == CONV_RADER) ? (int)P->n : 0;
-        kp.mX = magic(P->n);
-        kp.mM = magic(sh.M);
-        kp.mL = magic(std::max<int64_t>(1, P->n - 1));
-        rc = make_subplan(P, sh.M, sh.rc, sh.V, kp.pc);
-        if (rc) return rc;
+        kp.mode = MODE_LCONV;
+        kp.qp = sf_qp(kp.sc, sh.V, e, true);
+        kp.qw = sf_qw(kp.sc, sh.V, e, true);
         Stage s;
         s.kp = kp;
         s.threads = CFFT_THREADS;
@@ -1381,7 +1390,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         s.grid = 0;  // set per execution from batch
         s.in_sel = 0;
         s.out_sel = 1;
-        s.fn = cfft_kernel_for(MODE_ROWS, P->dtype);
+        s.fn = cfft_kernel_for(MODE_LCONV, P->dtype);
         CUDA_TRY(cfft_prepare_fn(s.fn, s.smem, 1));
         P->stages.push_back(s);
         P->chunk = P->batch;
@@ -1739,7 +1748,7 @@ static int plan_execute(cfft_plan_s* P, const void* in, void* out, int dir, cuda
             }
             unsigned grid;
             if (p2) grid = (unsigned)kp.batch;
-            else if (kp.mode == MODE_ROWS || kp.mode == MODE_LINE) grid = (unsigned)((nb + kp.V - 1) / kp.V);
+            else if (kp.mode == MODE_LCONV || kp.mode == MODE_LINE) grid = (unsigned)((nb + kp.V - 1) / kp.V);
             else if (kp.mode == MODE_FOUR || kp.mode == MODE_CLUS || kp.mode == MODE_CONVC || kp.mode == MODE_MIXC || kp.mode == MODE_P2CL)
                 grid = (unsigned)(nb * kp.C);
             else if (s.cols) {
@@ -1846,7 +1855,7 @@ static void wisdom_store(const WisdomKey& k, const std::string& sig) {
 static bool io_fusable(const cfft_plan_s* P) {
     for (const auto& st : P->stages) {
         const int m = st.kp.mode;
-        if (m != MODE_ROWS && m != MODE_FOUR && m != MODE_COLPASS && m != MODE_ROWPASS && m != MODE_MIDPASS &&
+        if (m != MODE_LCONV && m != MODE_FOUR && m != MODE_COLPASS && m != MODE_ROWPASS && m != MODE_MIDPASS &&
             m != MODE_LINE && m != MODE_CLUS)
             return false;
         if (st.launch != 0 || st.fn == cfft_r4096_kernel(P->dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64))
@@ -2077,16 +2086,15 @@ static int build_shared_plan(int64_t n, int dtype, int flags, int device, cfft_p
     *out = P;
     return CFFT_OK;
 }
-// batch-1 plan for the work queue: a single-CTA shape (rows or a
-// one-CTA four-step) whose descriptor-driven variant fits `cap` bytes of
-// shared memory, else two HBM passes
+// batch-1 plan for the work queue: a single-CTA shape (LINE or LCONV) that
+// fits `cap` bytes of shared memory, else the HBM passes
 static size_t batched_smem(const Stage& st);
 static bool single_kernel(const cfft_plan_s* P);
 static int build_queue_plan(int64_t n, int dtype, int flags, int device, size_t cap, cfft_plan_s** out) {
     if (n > (1LL << 26)) return fail(CFFT_ERR_UNSUPPORTED, "length above 2^26");
     std::vector<Shape> v;
     for (auto& c : candidate_shapes(n, dtype, 1))
-        if ((c.mode == MODE_ROWS || c.mode == MODE_FOUR) && c.C == 1) v.push_back(c);
+        if (c.mode == MODE_ROWS) v.push_back(c);
     int conv;
     int64_t M;
     conv_kind(n, conv, M);
@@ -2127,7 +2135,7 @@ static int build_queue_plan(int64_t n, int dtype, int flags, int device, size_t 
 static size_t batched_smem(const Stage& st) { return st.smem_batched ? st.smem_batched : st.smem; }
 static bool single_kernel(const cfft_plan_s* P) {
     return P->stages.size() == 1 &&
-           (P->stages[0].kp.mode == MODE_ROWS || P->stages[0].kp.mode == MODE_FOUR ||
+           (P->stages[0].kp.mode == MODE_LCONV || P->stages[0].kp.mode == MODE_FOUR ||
             P->stages[0].kp.mode == MODE_LINE || P->stages[0].kp.mode == MODE_CLUS);
 }
 // CTAs one parameter block occupies in a batched launch
@@ -2338,10 +2346,7 @@ static int batch_create_queue(cfft_batch_s* B) {
     auto emit_single = [&](int64_t i) {
         cfft_plan_s* P = B->plans[B->len[i]];
         KParams kp = P->stages[0].kp;
-        const void* vf = batched_variant(kp, dtype);
-        const int kind = kp.mode == MODE_ROWS   ? QK_ROWS
-                         : kp.mode == MODE_LINE ? QK_LINE
-                         : vf == cfft_batch_kernel_for(MODE_FOUR_WARP, dt) ? QK_FOUR_WARP : QK_FOUR;
+        const int kind = kp.mode == MODE_LINE ? QK_LINE : QK_LCONV;
         kp.batch = 1;
         kp.in_off = kp.out_off = B->off[i];
         kp.in_user = kp.out_user = 1;

@@ -46,13 +46,11 @@ __global__ void __launch_bounds__(CFFT_THREADS, MB) kq_batch(QueueLaunch L) {
     }
     __syncthreads();
     switch (it.kind) {
-        case QK_ROWS: rows_body<V, CFFT_EMAX>(sp, smem); break;
-        case QK_FOUR: four_body<V, CFFT_EMAX, DynK<0>>(sp, smem); break;
-        case QK_FOUR_WARP: four_body<V, CFFT_EMAX, DynK<1>>(sp, smem); break;
         case QK_COLPASS: colpass_body<V>(sp, smem); break;
         case QK_ROWPASS: rowpass_body<V>(sp, smem); break;
         case QK_MIDPASS: midpass_body<V>(sp, smem); break;
-        default: line_body<V>(sp, smem); break;
+        case QK_LINE: line_body<V>(sp, smem); break;
+        default: lconv_body<V>(sp, smem); break;
     }
     if (it.done >= 0) flow_publish(ctr + it.done);
 }
