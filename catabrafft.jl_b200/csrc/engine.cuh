@@ -938,18 +938,28 @@ __device__ __forceinline__ void four_body(const KParams& p, unsigned char* smem)
 // ---- batched entry points: each block finds its parameter block, stages it
 // in shared memory with the launch's base pointers and direction applied, and
 // runs the same body as the single-plan kernels.
+// a parameter block into shared memory, a word per thread (one thread copying
+// it serially held every CTA up for about a microsecond); caller synchronises
+__device__ __forceinline__ void copy_params(KParams* sp, const KParams* src) {
+    static_assert(sizeof(KParams) % 4 == 0, "copied in 32-bit words");
+    const uint32_t* s = (const uint32_t*)src;
+    for (int i = threadIdx.x; i < (int)(sizeof(KParams) / 4); i += blockDim.x) ((uint32_t*)sp)[i] = __ldg(s + i);
+}
+// the launch's base pointers and direction
+template <typename V>
+__device__ __forceinline__ void patch_params(KParams* sp, const void* in_base, void* out_base, int dir) {
+    if (sp->in_user) sp->in = (const V*)in_base + sp->in_off;
+    if (sp->out_user) sp->out = (V*)out_base + sp->out_off;
+    if (dir >= 0) {                       // one direction for the launch
+        sp->dir = dir;
+        if (dir != 1) sp->scale = 1.0;
+    }                                     // else: per-block direction and scale
+}
 template <typename V>
 __device__ __forceinline__ const KParams& stage_params(const BatchLaunch& L, KParams* sp) {
-    if (threadIdx.x == 0) {
-        KParams p = L.desc[L.block_desc[blockIdx.x]];
-        if (p.in_user) p.in = (const V*)L.in_base + p.in_off;
-        if (p.out_user) p.out = (V*)L.out_base + p.out_off;
-        if (L.dir >= 0) {                 // one direction for the launch
-            p.dir = L.dir;
-            if (L.dir != 1) p.scale = 1.0;
-        }                                 // else: per-block direction and scale
-        *sp = p;
-    }
+    copy_params(sp, L.desc + L.block_desc[blockIdx.x]);
+    __syncthreads();
+    if (threadIdx.x == 0) patch_params<V>(sp, L.in_base, L.out_base, L.dir);
     __syncthreads();
     return *sp;
 }

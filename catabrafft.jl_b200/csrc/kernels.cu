@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(CFFT_THREADS, MinBlocks<V>::value) kb_four(Bat
 
 const void* cfft_batch_kernel_for(int mode, int dtype) {
     if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE ||
-        mode == MODE_LCONV || mode == MODE_CLUS)
+        mode == MODE_LCONV || mode == MODE_CLUS || mode == MODE_COLS)
         return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, true) : cfft_pass_kernel32(mode, true);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {
@@ -445,7 +445,7 @@ int cfft_mixc_lookup(long long n, int dtype, int variant, const void** fn, int* 
 
 const void* cfft_kernel_for(int mode, int dtype) {
     if (mode == MODE_COLPASS || mode == MODE_ROWPASS || mode == MODE_MIDPASS || mode == MODE_LINE ||
-        mode == MODE_LCONV || mode == MODE_CLUS)
+        mode == MODE_LCONV || mode == MODE_CLUS || mode == MODE_COLS)
         return dtype == CFFT_DT_C128 ? cfft_pass_kernel64(mode, false) : cfft_pass_kernel32(mode, false);
     if (dtype == CFFT_DT_C128) {
         switch (mode) {

@@ -55,22 +55,34 @@
 #pragma once
 #include "engine.cuh"
 
-// R as a compile-time constant for each radix the planner uses (sf_radix)
+// R as a compile-time constant for each radix the planner uses (sf_search in
+// passplan.h); SF_SWITCH_LINE adds 18 and 20 for ComplexF32 (V of the enclosing
+// template) in LINE and LCONV
+#define SF_CASES(CALL)              \
+    case 2: CALL(2); break;         \
+    case 3: CALL(3); break;         \
+    case 4: CALL(4); break;         \
+    case 5: CALL(5); break;         \
+    case 6: CALL(6); break;         \
+    case 7: CALL(7); break;         \
+    case 8: CALL(8); break;         \
+    case 9: CALL(9); break;         \
+    case 10: CALL(10); break;       \
+    case 12: CALL(12); break;       \
+    case 14: CALL(14); break;       \
+    case 15: CALL(15); break;
 #define SF_SWITCH(r, CALL)          \
     switch (r) {                    \
-        case 2: CALL(2); break;     \
-        case 3: CALL(3); break;     \
-        case 4: CALL(4); break;     \
-        case 5: CALL(5); break;     \
-        case 6: CALL(6); break;     \
-        case 7: CALL(7); break;     \
-        case 8: CALL(8); break;     \
-        case 9: CALL(9); break;     \
-        case 10: CALL(10); break;   \
-        case 12: CALL(12); break;   \
-        case 14: CALL(14); break;   \
-        case 15: CALL(15); break;   \
+        SF_CASES(CALL)              \
         default: CALL(16); break;   \
+    }
+#define SF_SWITCH_LINE(r, CALL)                                   \
+    switch (r) {                                                  \
+        SF_CASES(CALL)                                            \
+        case 1: CALL(1); break;                                   \
+        case 18: if constexpr (sizeof(V) == 8) { CALL(18); } break; \
+        case 20: if constexpr (sizeof(V) == 8) { CALL(20); } break; \
+        default: CALL(16); break;                                 \
     }
 #define SF_SWITCH_LAST(r, CALL)     \
     if ((r) == 1) { CALL(1); }      \
@@ -228,7 +240,8 @@ __device__ __forceinline__ void col_last(const KParams& p, const V* buf, int t, 
         }
     }
 }
-template <typename V> __device__ __forceinline__ void colpass_body(const KParams& p, unsigned char* smem) {
+// LINE: whole transforms in columns, with LINE's radices (the same arithmetic)
+template <typename V, bool LINE = false> __device__ __forceinline__ void colpass_body(const KParams& p, unsigned char* smem) {
     V* buf = (V*)smem;
     const SfPlan& S = p.sa;
     const int tile = block_id(p), tiles = (p.N2 + p.V - 1) / p.V;
@@ -243,19 +256,28 @@ template <typename V> __device__ __forceinline__ void colpass_body(const KParams
         c.ok = c.k0 < p.ks && c.col < p.N2;     // the last tile may be partial
     }
 #define SF_CALL(R) col_first<V, R>(p, buf, t, c)
-    if (c.ok) { SF_SWITCH(S.r[0], SF_CALL) }
+    if (c.ok) {
+        if constexpr (LINE) { SF_SWITCH_LINE(S.r[0], SF_CALL) }
+        else { SF_SWITCH(S.r[0], SF_CALL) }
+    }
 #undef SF_CALL
     __syncthreads();
     int Ls = S.L / S.r[0];
     for (int s = 1; s < S.np - 1; s++) {
 #define SF_CALL(R) col_mid<V, R>(p, buf, s, Ls, c)
-        if (c.ok) { SF_SWITCH(S.r[s], SF_CALL) }
+        if (c.ok) {
+            if constexpr (LINE) { SF_SWITCH_LINE(S.r[s], SF_CALL) }
+            else { SF_SWITCH(S.r[s], SF_CALL) }
+        }
 #undef SF_CALL
         __syncthreads();
         Ls /= S.r[s];
     }
 #define SF_CALL(R) col_last<V, R>(p, buf, t, c)
-    if (c.ok) { SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL) }
+    if (c.ok) {
+        if constexpr (LINE) { SF_SWITCH_LINE(S.r[S.np - 1], SF_CALL) }
+        else { SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL) }
+    }
 #undef SF_CALL
 }
 
@@ -556,19 +578,19 @@ template <typename V> __device__ __forceinline__ void line_body(const KParams& p
     const int t0 = block_id(p) * p.V, rows = min(p.V, p.batch - t0);
     if (rows <= 0) return;                      // uniform across the CTA
 #define SF_CALL(R) line_first<V, R>(p, buf, t0, rows)
-    SF_SWITCH_LAST(S.r[0], SF_CALL)
+    SF_SWITCH_LINE(S.r[0], SF_CALL)
 #undef SF_CALL
     __syncthreads();
     int Ls = S.L / S.r[0];
     for (int s = 1; s < S.np - 1; s++) {
 #define SF_CALL(R) line_mid<V, R>(p, buf, s, Ls, rows)
-        SF_SWITCH(S.r[s], SF_CALL)
+        SF_SWITCH_LINE(S.r[s], SF_CALL)
 #undef SF_CALL
         __syncthreads();
         Ls /= S.r[s];
     }
 #define SF_CALL(R) line_last<V, R>(p, buf, t0, rows)
-    SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
+    SF_SWITCH_LINE(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
 }
 
@@ -697,30 +719,30 @@ template <typename V> __device__ __forceinline__ void lconv_body(const KParams& 
         }
     }
 #define SF_CALL(R) lconv_first<V, R>(p, buf, t0, rows)
-    SF_SWITCH(S.r[0], SF_CALL)
+    SF_SWITCH_LINE(S.r[0], SF_CALL)
 #undef SF_CALL
     __syncthreads();
     int Ls = S.L / S.r[0];
     for (int s = 1; s < S.np - 1; s++) {
 #define SF_CALL(R) row_mid<V, R, false, false>(p, buf, s, Ls, rows)
-        SF_SWITCH(S.r[s], SF_CALL)
+        SF_SWITCH_LINE(S.r[s], SF_CALL)
 #undef SF_CALL
         __syncthreads();
         Ls /= S.r[s];
     }
 #define SF_CALL(R) mid_center<V, R, true>(p, buf, 0, rows)
-    SF_SWITCH_LAST(S.r[S.np - 1], SF_CALL)
+    SF_SWITCH_LINE(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
     __syncthreads();
     for (int s = S.np - 2; s >= 1; s--) {
         Ls *= S.r[s];
 #define SF_CALL(R) row_mid<V, R, false, true>(p, buf, s, Ls, rows)
-        SF_SWITCH(S.r[s], SF_CALL)
+        SF_SWITCH_LINE(S.r[s], SF_CALL)
 #undef SF_CALL
         __syncthreads();
     }
 #define SF_CALL(R) lconv_last<V, R>(p, buf, x0, t0, rows)
-    SF_SWITCH(S.r[0], SF_CALL)
+    SF_SWITCH_LINE(S.r[0], SF_CALL)
 #undef SF_CALL
     if (p.conv == CONV_RADER)
         for (int r = opaque_tid(); r < rows; r += CFFT_THREADS)

@@ -10,6 +10,7 @@ template <> struct PassBlocks<double2> { static constexpr int value = 2; };
 
 template <typename V, int MODE> __device__ __forceinline__ void pass_body(const KParams& p, unsigned char* smem) {
     if constexpr (MODE == MODE_COLPASS) colpass_body<V>(p, smem);
+    else if constexpr (MODE == MODE_COLS) colpass_body<V, true>(p, smem);
     else if constexpr (MODE == MODE_ROWPASS) rowpass_body<V>(p, smem);
     else if constexpr (MODE == MODE_MIDPASS) midpass_body<V>(p, smem);
     else if constexpr (MODE == MODE_LINE) line_body<V>(p, smem);
@@ -47,6 +48,7 @@ template <typename V> const void* pass_kernel(int mode, bool batched) {
         case MODE_MIDPASS: return batched ? (const void*)kb_pass<V, MODE_MIDPASS> : (const void*)k_pass<V, MODE_MIDPASS>;
         case MODE_LINE: return batched ? (const void*)kb_pass<V, MODE_LINE> : (const void*)k_pass<V, MODE_LINE>;
         case MODE_LCONV: return batched ? (const void*)kb_pass<V, MODE_LCONV> : (const void*)k_pass<V, MODE_LCONV>;
+        case MODE_COLS: return batched ? nullptr : (const void*)k_pass<V, MODE_COLS>;
         case MODE_CLUS: return batched ? (const void*)kb_clus<V> : (const void*)k_clus<V>;
     }
     return nullptr;

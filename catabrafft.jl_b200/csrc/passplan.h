@@ -12,19 +12,23 @@ static const int SF_THREADS = 256;    // CTA size of the pass kernels
 // Radix sequence of L (7-smooth, L >= 2): the fewest stages first (a stage is
 // a shared-memory round trip and a barrier), then the least arithmetic, in
 // ascending order -- the last radix is the largest, so the runs that the row
-// layout keeps contiguous span a half-warp.  One stage becomes two (L, 1), as
-// the kernels always run a first and a last one.
+// layout keeps contiguous span a half-warp (the other way round a 24000-point
+// two-pass plan took 225 us against 212).  One stage becomes two (L, 1), as
+// the kernels always run a first and a last one.  Radices go up to maxr: 20 for
+// ComplexF32 in LINE and LCONV (50000 x 360 as 18 x 20 63 us, as 6 x 6 x 10
+// 86), 16 elsewhere (in the HBM passes 18 and 20 measured from 5 % faster to
+// 10 % slower, and 21 to 27 spill at 80 registers and lose 15 - 25 %).
 inline double sf_radix_cost(int r) {
     // real additions and multiplications per point of the codelets
     switch (r) {
         case 2: return 2.0; case 3: return 5.3; case 4: return 4.0; case 5: return 8.0; case 6: return 7.3;
         case 7: return 12.9; case 8: return 6.5; case 9: return 11.1; case 10: return 10.0; case 12: return 9.3;
-        case 14: return 14.9; case 15: return 13.6; case 16: return 9.8;
+        case 14: return 14.9; case 15: return 13.6; case 16: return 9.8; case 18: return 14.5; case 20: return 13.0;
     }
     return 1e9;
 }
 inline void sf_search(int rem, int maxr, int depth, double cost, int* cur, int* best, int* nbest, double* cbest) {
-    static const int rad[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+    static const int rad[] = {20, 18, 16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
     if (rem == 1) {
         if (depth < *nbest || (depth == *nbest && cost < *cbest)) {
             *nbest = depth;
@@ -44,7 +48,7 @@ inline void sf_search(int rem, int maxr, int depth, double cost, int* cur, int* 
 // 0 stands for d = 1
 inline unsigned sf_magic(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
 // fills L, np, r and the table layout; false if L has no sequence
-inline bool sf_plan(int L, SfPlan& S) {
+inline bool sf_plan(int L, SfPlan& S, int maxr = 16) {
     S = SfPlan();
     S.L = L;
     if (L < 1) return false;
@@ -55,7 +59,7 @@ inline bool sf_plan(int L, SfPlan& S) {
     }
     int cur[SF_MAXS], best[SF_MAXS], n = SF_MAXS + 1;
     double c = 1e30;
-    sf_search(L, 16, 0, 0.0, cur, best, &n, &c);
+    sf_search(L, maxr, 0, 0.0, cur, best, &n, &c);
     if (n > SF_MAXS) return false;
     S.np = n < 2 ? 2 : n;
     if (n == 1) {
@@ -130,14 +134,28 @@ inline int sf_qw(const SfPlan& S, int V, size_t e, bool mid) {
 }
 inline size_t sf_col_smem(const SfPlan& S, int V, size_t e) { return (size_t)S.L * V * e; }
 inline size_t sf_row_smem(const SfPlan& S, int V, size_t e, bool mid) { return (size_t)sf_qw(S, V, e, mid) * V * e; }
-// Cost model of a tile, in SM cycles of one of its CTAs: a round of butterflies
-// of radix R (each active thread runs one) takes about 1340 + 171 R cycles at
-// three CTAs per SM -- fitted to B200 timings of COLPASS at radix 10 (268
-// instructions a butterfly, one every 12 cycles) -- whether or not every
-// thread has one, and a tile costs about one more such latency to start.  So
-// widths are picked to fill the rounds, not for a target size.
+// Cost model of a tile, in SM cycles of one of its CTAs.  In the HBM passes a
+// round of butterflies of radix R (each thread runs at most one) takes about
+// 1340 + 171 R cycles at three CTAs per SM -- fitted to B200 timings of COLPASS
+// at radix 10 (268 instructions a butterfly, one every 12 cycles) -- whether or
+// not every thread has one, and a tile costs about one more such latency to
+// start.  So widths are picked to fill the rounds, not for a target size.
 inline double sf_round(int R, int dfts) { return 1340.0 + 171.0 * R * dfts; }
 inline double sf_start() { return 2500.0; }
+// LINE and LCONV, whole launches of equal CTAs: a round with idle threads costs
+// its share less, a CTA a third of a round to start.  400000 x 120 ComplexF32
+// (radices 10, 12) by rows per CTA: 10 224 us, 21 (one full round a stage) 160,
+// 32 168, 42 (two) 148, 64 (three) 168: beyond about 130 KB of shared memory
+// per SM the L1 left for the loads in flight shrinks.
+inline double sf_rounds(long long items, int threads, int R, int dfts) {
+    const double full = (double)(items / threads), rest = (double)(items % threads) / threads;
+    return sf_round(R, dfts) * (full + (rest > 0 ? 0.4 + 0.6 * rest : 0.0));
+}
+inline double sf_line_start() { return 1100.0; }
+inline double sf_crowd(size_t smem, size_t e) {
+    const double total = (double)smem * (e == 8 ? 3 : 2) / 1024.0;
+    return total > 130.0 ? 1.0 + 0.12 * (total - 130.0) / 68.0 : 1.0;
+}
 // cycles per useful element of a COLPASS / ROWPASS tile of width V
 inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bool row) {
     const size_t smem = row ? sf_row_smem(S, V, e, false) : sf_col_smem(S, V, e);
@@ -146,6 +164,7 @@ inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bo
     double c = sf_start();
     for (int s = 0; s < S.np; s++) {
         const int nb = S.L / S.r[s];
+        // the column mapping keeps ks V threads
         c += sf_round(S.r[s], 1) * (row && s == 0 ? (V * nb + SF_THREADS - 1) / SF_THREADS : (nb + ks - 1) / ks);
     }
     // the strided side moves 32-byte sectors: whole ones if V and the row
@@ -227,9 +246,9 @@ inline int sf_line_rows(const SfPlan& S, long long batch, size_t e) {
     double bc = 1e300;
     for (int V = 1; V <= 1024 && V <= batch; V++) {
         if (V > 1 && sf_line_smem(S, V, e) > sf_budget(e)) break;
-        double c = sf_start();
-        for (int s = 0; s < S.np; s++)
-            c += sf_round(S.r[s], 1) * (((long long)V * (S.L / S.r[s]) + SF_THREADS - 1) / SF_THREADS);
+        double c = sf_line_start();
+        for (int s = 0; s < S.np; s++) c += sf_rounds((long long)V * (S.L / S.r[s]), SF_THREADS, S.r[s], 1);
+        c *= sf_crowd(sf_line_smem(S, V, e), e);
         // whole waves while there are few; their tails matter less and less
         const double waves = (double)((batch + V - 1) / V) / (double)slots;
         c *= waves < 4.0 ? std::ceil(waves) : waves + 0.5;
@@ -250,11 +269,12 @@ inline int sf_lconv_rows(const SfPlan& S, long long batch, size_t e, double* cos
     double bc = 1e300;
     for (int V = 1; V <= 256 && V <= batch; V++) {
         if (V > 1 && sf_lconv_smem(S, V, e) > sf_budget(e)) break;
-        double c = sf_start();
+        double c = sf_line_start();
         for (int s = 0; s < S.np; s++) {
-            const long long rounds = ((long long)V * (S.L / S.r[s]) + SF_THREADS - 1) / SF_THREADS;
-            c += rounds * (s == S.np - 1 ? sf_round(S.r[s], 2) : 2.0 * sf_round(S.r[s], 1));
+            const long long items = (long long)V * (S.L / S.r[s]);
+            c += s == S.np - 1 ? sf_rounds(items, SF_THREADS, S.r[s], 2) : 2.0 * sf_rounds(items, SF_THREADS, S.r[s], 1);
         }
+        c *= sf_crowd(sf_lconv_smem(S, V, e), e);
         const double waves = (double)((batch + V - 1) / V) / (double)slots;
         c *= waves < 4.0 ? std::ceil(waves) : waves + 0.5;
         if (c < bc) {

@@ -370,12 +370,27 @@ static const int kSfMax = 4096;      // factors of the passes
 static const int kLineMax = 9216;    // whole transforms in a CTA (74 KB of ComplexF32)
 static const SfPlan* sf_get(int64_t L) {
     static const std::vector<SfPlan> tab = [] {
-        std::vector<SfPlan> t(kLineMax + 1);
-        for (int l = 1; l <= kLineMax; l++)
+        std::vector<SfPlan> t(kSfMax + 1);
+        for (int l = 1; l <= kSfMax; l++)
             if (!is_smooth7(l) || !sf_plan(l, t[l])) t[l].L = 0;
         return t;
     }();
-    return L >= 1 && L <= kLineMax && tab[L].L ? &tab[L] : nullptr;
+    return L >= 1 && L <= kSfMax && tab[L].L ? &tab[L] : nullptr;
+}
+// ... and of every length LINE and LCONV use
+static const SfPlan* sf_line(int64_t L, int dtype) {
+    static const std::vector<SfPlan> tab = [] {
+        std::vector<SfPlan> t(2 * (kLineMax + 1));
+        for (int l = 1; l <= kLineMax; l++)
+            for (int d = 0; d < 2; d++) {
+                SfPlan& S = t[d * (kLineMax + 1) + l];
+                if (!is_smooth7(l) || !sf_plan(l, S, d ? 20 : 16)) S.L = 0;
+            }
+        return t;
+    }();
+    if (L < 1 || L > kLineMax) return nullptr;
+    const SfPlan* S = &tab[(dtype == CFFT_C128 ? 0 : kLineMax + 1) + L];
+    return S->L ? S : nullptr;
 }
 static std::vector<int> sf_radices(const SfPlan& S) { return std::vector<int>(S.r, S.r + S.np); }
 // one CTA: LINE, or LCONV with the cheapest convolution length within 2 % of
@@ -385,7 +400,7 @@ static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch
     if (M > kLineMax) return false;
     sh.mode = MODE_ROWS;
     if (conv == CONV_NONE) {
-        const SfPlan* S = sf_get(M);
+        const SfPlan* S = sf_line(M, dtype);
         if (!S || sf_line_smem(*S, 1, e) > sf_budget(e)) return false;
         sh.M = M;
         // one row a CTA where the n = 4096 register kernel runs it
@@ -396,7 +411,7 @@ static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch
     }
     double best = 1e300;
     for (int64_t m = M; m <= M + M / 50 && m <= kLineMax; m++) {
-        const SfPlan* S = sf_get(m);
+        const SfPlan* S = sf_line(m, dtype);
         if (!S || S->r[S->np - 1] < 2 || sf_lconv_smem(*S, 1, e) > sf_budget(e)) continue;
         double c;
         const int V = sf_lconv_rows(*S, batch, e, &c);
@@ -534,11 +549,11 @@ static double sf_cost(int64_t L, int64_t count, size_t e, int kind) {
     static const std::vector<Entry> tab = [] {
         std::vector<Entry> t((size_t)6 * (kSfMax + 1), {1e9, 1});
         for (int l = 2; l <= kSfMax; l++) {
-            const SfPlan* S = sf_get(l);
-            if (!S) continue;
             for (int i = 0; i < 6; i++) {
                 Entry& x = t[(size_t)i * (kSfMax + 1) + l];
                 const size_t el = i < 3 ? 8 : 16;
+                const SfPlan* S = sf_get(l);
+                if (!S) continue;
                 x.V = i % 3 == 2 ? sf_mid_rows(*S, 1 << 16, el, &x.c) : sf_tile(*S, 1 << 16, el, i % 3 == 1, &x.c);
             }
         }
@@ -933,12 +948,12 @@ static int make_subplan(cfft_plan_s* P, int64_t L, const std::vector<int>& rad, 
     }, &sp.tw);
 }
 // sub-transform of the passes with its twiddle blocks (SfPlan.off / .boff)
-static int make_sfplan(cfft_plan_s* P, int64_t L, SfPlan& S) {
-    const SfPlan* q = sf_get(L);
+static int make_sfplan(cfft_plan_s* P, int64_t L, SfPlan& S, bool line = false) {
+    const SfPlan* q = line ? sf_line(L, P->dtype) : sf_get(L);
     if (!q) return fail(CFFT_ERR_UNSUPPORTED, "no radix sequence for " + std::to_string(L));
     S = *q;
     const int dtype = P->dtype;
-    return cached_table(P, "sf/" + std::to_string(dtype) + "/" + std::to_string(L), [&](std::vector<unsigned char>& img) {
+    return cached_table(P, "sf/" + std::to_string(dtype) + (line ? "l/" : "/") + std::to_string(L), [&](std::vector<unsigned char>& img) {
         std::vector<double2> w(std::max(1, q->twall));
         for (int i = 0; i < q->twall; i++) {
             long long e;
@@ -1110,7 +1125,7 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
         const int* iperm = kp.iperm;
         *spec_key = "sr/" + tag + "/" + std::to_string(exact);
         if (sh.mode == MODE_ROWS)
-            return conv_spectrum_rows(P, *spec_key + "/c", 1, *sf_get(M), [&](double2* v) {
+            return conv_spectrum_rows(P, *spec_key + "/c" + std::to_string(P->dtype), 1, *sf_line(M, P->dtype), [&](double2* v) {
                 return cfft_gen_rader_b(v, iperm, n, M, exact, winv, 0);
             }, &kp.spec);
         return conv_spectrum(P, *spec_key, M, [&](double2* v) {
@@ -1127,8 +1142,8 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
     kp.chirp = (const double2*)dch;
     const double2* ch = kp.chirp;
     if (sh.mode == MODE_COLPASS || sh.mode == MODE_ROWS)
-        return conv_spectrum_rows(P, "sc/" + tag + "/" + std::to_string(sh.mode == MODE_ROWS ? 1 : sh.N1),
-                                  sh.mode == MODE_ROWS ? 1 : sh.N1, *sf_get(sh.mode == MODE_ROWS ? sh.M : sh.N2),
+        return conv_spectrum_rows(P, "sc/" + tag + "/" + std::to_string(P->dtype) + "/" + std::to_string(sh.mode == MODE_ROWS ? 1 : sh.N1),
+                                  sh.mode == MODE_ROWS ? 1 : sh.N1, sh.mode == MODE_ROWS ? *sf_line(sh.M, P->dtype) : *sf_get(sh.N2),
                                   [&](double2* v) { return cfft_gen_bluestein_b(v, ch, n, M, 0); }, &kp.spec);
     *spec_key = "sb/" + tag;
     return conv_spectrum(P, *spec_key, M, [&](double2* v) {
@@ -1341,7 +1356,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     if (sh.mode == MODE_ROWS) {
         kp.mode = MODE_ROWS;
         kp.V = sh.V;
-        rc = make_sfplan(P, sh.M, kp.sc);
+        rc = make_sfplan(P, sh.M, kp.sc, true);
         if (rc) return rc;
         if (sh.conv == CONV_NONE) {
             // V rows per CTA in register stages (passes.cuh), or the persistent
@@ -3047,7 +3062,7 @@ int cfft_plan_create_many(cfft_plan* plan, int64_t n, int64_t batch, int dtype, 
         s.kp.post = POST_STORE;
         sf_stage(s.kp, e, &s.smem);
         s.cols = true;
-        s.fn = cfft_kernel_for(MODE_COLPASS, dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64);
+        s.fn = cfft_kernel_for(MODE_COLS, dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64);
         if ((s.kp.V * e >= 32 || s.kp.V == batch) && s.smem <= sf_budget(e) &&
             cfft_prepare_fn(s.fn, s.smem, 1) == cudaSuccess)
             P->stages[0] = s;

@@ -32,17 +32,15 @@ __global__ void __launch_bounds__(CFFT_THREADS, MB) kq_batch(QueueLaunch L) {
     const int i = s_item[0];
     if (i >= L.nitems) return;
     const QItem it = L.items[i];
-    if (it.wait >= 0 && !flow_wait(ctr + it.wait, it.need, s_item + 1, abort)) return;
+    copy_params(&sp, L.desc + it.desc);         // in flight while the dependency is awaited
+    if (it.wait >= 0) {
+        if (!flow_wait(ctr + it.wait, it.need, s_item + 1, abort)) return;
+    } else {
+        __syncthreads();
+    }
     if (threadIdx.x == 0) {
-        KParams p = L.desc[it.desc];
-        if (p.in_user) p.in = (const V*)L.in_base + p.in_off;
-        if (p.out_user) p.out = (V*)L.out_base + p.out_off;
-        if (L.dir >= 0) {
-            p.dir = L.dir;
-            if (L.dir != 1) p.scale = 1.0;
-        }
-        p.blk0 = (int)blockIdx.x - it.blk;
-        sp = p;
+        patch_params<V>(&sp, L.in_base, L.out_base, L.dir);
+        sp.blk0 = (int)blockIdx.x - it.blk;
     }
     __syncthreads();
     switch (it.kind) {
