@@ -3613,6 +3613,7 @@ struct cfft_rplan_s {
     int64_t n = 0, batch = 0;
     int dtype = 0;
     cfft_plan_s* P = nullptr;
+    TwoLevel w = {};             // even n: table of w_n
     void* scratch = nullptr;     // odd n: batch * n complex
     void* d_real = nullptr;      // host entry: device copies of the two sides
     void* d_cplx = nullptr;
@@ -3632,6 +3633,7 @@ int cfft_rfft_plan_create(cfft_rplan* plan, int64_t n, int64_t batch, int dtype,
     R->dtype = dtype;
     const bool even = (n % 2 == 0);
     int rc = plan_create_impl(&R->P, even ? n / 2 : n, batch, dtype, flags);
+    if (rc == CFFT_OK && even) rc = make_twolevel(R->P, n, R->w);
     if (rc == CFFT_OK && !even) {
         if (lib_malloc(&R->scratch, (size_t)n * batch * elem_bytes(dtype)) != cudaSuccess) {
             cudaGetLastError();
@@ -3662,9 +3664,16 @@ int cfft_rfft_execute(cfft_rplan plan, const void* d_real, void* d_complex, void
     if (n % 2 == 0) {
         if (((uintptr_t)d_real % e) != 0 || ((uintptr_t)d_complex % e) != 0)
             return fail(CFFT_ERR_INVALID, "buffers must be aligned to the complex element size");
-        int rc = plan_execute(R->P, d_real, d_complex, CFFT_FORWARD, st, -1, n / 2, h);
-        if (rc) return rc;
-        CUDA_TRY(cfft_r2c_post(d_complex, n / 2, n, R->batch, h, R->dtype, st));
+        // chunk by chunk where the complex plan is: the sweep then finds the
+        // chunk's outputs in L2
+        for (int64_t b0 = 0; b0 < R->batch; b0 += R->P->chunk) {
+            const int64_t nb = std::min(R->P->chunk, R->batch - b0);
+            char* out = (char*)d_complex + (size_t)b0 * h * e;
+            int rc = plan_execute(R->P, (const char*)d_real + (size_t)b0 * (n / 2) * e, out, CFFT_FORWARD, st, nb,
+                                  n / 2, h);
+            if (rc) return rc;
+            CUDA_TRY(cfft_r2c_post(out, n / 2, R->w, nb, h, R->dtype, st));
+        }
         return CFFT_OK;
     }
     CUDA_TRY(cfft_r2c_widen(d_real, R->scratch, n, R->batch, R->dtype, st));
@@ -3687,8 +3696,15 @@ int cfft_rfft_execute_inverse(cfft_rplan plan, const void* d_complex, void* d_re
     if (n % 2 == 0) {
         if (((uintptr_t)d_real % e) != 0 || ((uintptr_t)d_complex % e) != 0)
             return fail(CFFT_ERR_INVALID, "buffers must be aligned to the complex element size");
-        CUDA_TRY(cfft_c2r_pre(d_complex, d_real, n / 2, n, R->batch, h, scale, R->dtype, st));
-        return plan_execute(R->P, d_real, d_real, CFFT_BACKWARD, st, -1);
+        for (int64_t b0 = 0; b0 < R->batch; b0 += R->P->chunk) {
+            const int64_t nb = std::min(R->P->chunk, R->batch - b0);
+            char* z = (char*)d_real + (size_t)b0 * (n / 2) * e;
+            CUDA_TRY(cfft_c2r_pre((const char*)d_complex + (size_t)b0 * h * e, z, n / 2, R->w, nb, h, scale, R->dtype,
+                                  st));
+            int rc = plan_execute(R->P, z, z, CFFT_BACKWARD, st, nb);
+            if (rc) return rc;
+        }
+        return CFFT_OK;
     }
     CUDA_TRY(cfft_c2r_expand(d_complex, R->scratch, n, R->batch, scale, R->dtype, st));
     int rc = plan_execute(R->P, R->scratch, R->scratch, CFFT_BACKWARD, st, -1);

@@ -13,63 +13,80 @@
 // Hermitian spectrum has none).
 // Odd n: the reals are widened to complex in a scratch buffer, transformed
 // by the complex path, and the first n/2 + 1 outputs kept; the inverse
-// rebuilds the full Hermitian spectrum there.  Twiddles are evaluated in
-// FP64 (sincospi) and rounded once to the data type.
+// rebuilds the full Hermitian spectrum there.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include "engine.cuh"
 #include "kernels.h"
 
-// w^k with w = exp(sign * 2 pi i / n), in FP64
-__device__ __forceinline__ double2 wpow(long long k, long long n, int sign) {
-    double s, c;
-    sincospi(2.0 * (double)k / (double)n, &s, &c);
-    return make_double2(c, sign * s);
+// One thread per pair (k, N - k), k = 0 .. N/2: both of its elements are read
+// and written once.  w^k comes from the two-level FP64 table of w (lanes read
+// adjacent low entries and one high entry), and w^(N-k) = -conj(w^k), since
+// w^N = -1.  These sweeps are bandwidth bound: evaluating both twiddles of a
+// pair by sincospi, with 64-bit quotients per element, took 150 us for
+// 1024 x 24000 ComplexF32 (2.6 TB/s).
+// pair i of a launch -> transform t, pair k (half = N/2 + 1 pairs each)
+__device__ __forceinline__ bool pair_index(long long half, long long total, long long* t, int* k) {
+    const long long base = (long long)blockIdx.x * blockDim.x;
+    *t = base / half;
+    long long r = base - *t * half + threadIdx.x;
+    if (half >= (long long)blockDim.x) {
+        if (r >= half) {
+            r -= half;
+            (*t)++;
+        }
+    } else {
+        const int q = udiv_small((int)r, (int)half);
+        *t += q;
+        r -= q * half;
+    }
+    *k = (int)r;
+    return base + threadIdx.x < total;
+}
+template <typename V>
+__global__ void __launch_bounds__(256) k_r2c_post(V* out, int N, TwoLevel w, long long half, long long total,
+                                                  long long dist) {
+    long long t;
+    int k;
+    if (!pair_index(half, total, &t, &k)) return;
+    V* X = out + t * dist;
+    if (k == 0) {
+        const V z0 = X[0];
+        X[0] = mk<V>(z0.x + z0.y, 0);
+        X[N] = mk<V>(z0.x - z0.y, 0);
+        return;
+    }
+    const int j = N - k;
+    const double2 A = tod(X[k]), B = conjv(tod(X[j]));
+    const double2 fe = make_double2(0.5 * (A.x + B.x), 0.5 * (A.y + B.y));
+    // (A - B) / 2i = (Im(A - B) / 2, -Re(A - B) / 2)
+    const double2 fo = make_double2(0.5 * (A.y - B.y), -0.5 * (A.x - B.x));
+    const double2 a = cmul(tw_two(w, (unsigned)k), fo);
+    X[k] = fromd<V>(make_double2(fe.x + a.x, fe.y + a.y));
+    if (j != k) X[j] = fromd<V>(make_double2(fe.x - a.x, a.y - fe.y));
 }
 
 template <typename V>
-__global__ void k_r2c_post(V* out, long long N, long long n, long long batch, long long dist) {
-    const long long half = N / 2 + 1;             // pairs (k, N - k), k = 0..N/2
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < half * batch;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long t = i / half, k = i - t * half;
-        V* X = out + t * dist;
-        if (k == 0) {
-            const V z0 = X[0];
-            X[0] = mk<V>(z0.x + z0.y, 0);
-            X[N] = mk<V>(z0.x - z0.y, 0);
-            continue;
-        }
-        const long long j = N - k;
-        const double2 A = tod(X[k]), B = conjv(tod(X[j]));
-        const double2 fe = make_double2(0.5 * (A.x + B.x), 0.5 * (A.y + B.y));
-        // (A - B) / 2i = (Im(A - B) / 2, -Re(A - B) / 2)
-        const double2 fo = make_double2(0.5 * (A.y - B.y), -0.5 * (A.x - B.x));
-        const double2 wk = wpow(k, n, -1), wj = wpow(j, n, -1);
-        const double2 a = cmul(wk, fo), b = cmul(wj, conjv(fo));
-        X[k] = fromd<V>(make_double2(fe.x + a.x, fe.y + a.y));
-        if (j != k) X[j] = fromd<V>(make_double2(fe.x + b.x, -fe.y + b.y));
+__global__ void __launch_bounds__(256) k_c2r_pre(const V* in, V* z, int N, TwoLevel w, long long half,
+                                                 long long total, long long in_dist, double scale) {
+    long long t;
+    int k;
+    if (!pair_index(half, total, &t, &k)) return;
+    const V* X = in + t * in_dist;
+    V* Z = z + t * N;
+    if (k == 0) {
+        const double a = (double)X[0].x, b = (double)X[N].x;
+        Z[0] = fromd<V>(make_double2(scale * (a + b), scale * (a - b)));
+        return;
     }
-}
-
-template <typename V>
-__global__ void k_c2r_pre(const V* in, V* z, long long N, long long n, long long batch, long long in_dist,
-                          double scale) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N * batch;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long t = i / N, k = i - t * N;
-        const V* X = in + t * in_dist;
-        double2 A = tod(X[k]), B = conjv(tod(X[N - k]));
-        if (k == 0) {
-            A.y = 0;
-            B.y = 0;
-        }
-        const double2 fe = make_double2(A.x + B.x, A.y + B.y);
-        const double2 fo = cmul(make_double2(A.x - B.x, A.y - B.y), wpow(k, n, +1));
-        // fe + i fo
-        z[t * N + k] = fromd<V>(make_double2(scale * (fe.x - fo.y), scale * (fe.y + fo.x)));
-    }
+    const int j = N - k;
+    const double2 A = tod(X[k]), B = conjv(tod(X[j]));
+    const double2 fe = make_double2(A.x + B.x, A.y + B.y);
+    const double2 fo = cmul(make_double2(A.x - B.x, A.y - B.y), conjv(tw_two(w, (unsigned)k)));
+    // fe + i fo, and of N - k: conj(fe) + i conj(fo)
+    Z[k] = fromd<V>(make_double2(scale * (fe.x - fo.y), scale * (fe.y + fo.x)));
+    if (j != k) Z[j] = fromd<V>(make_double2(scale * (fe.x + fo.y), scale * (fo.x - fe.y)));
 }
 
 // odd n: widen reals to complex; keep the first n/2 + 1 outputs
@@ -112,20 +129,26 @@ static unsigned grid_for(long long work) {
     return (unsigned)(g < 1 ? 1 : (g > 8192 ? 8192 : g));
 }
 
-cudaError_t cfft_r2c_post(void* out, long long N, long long n, long long batch, long long dist, int dtype,
+cudaError_t cfft_r2c_post(void* out, long long N, const TwoLevel& w, long long batch, long long dist, int dtype,
                           cudaStream_t st) {
-    const long long work = (N / 2 + 1) * batch;
-    if (dtype == CFFT_DT_C128) k_r2c_post<double2><<<grid_for(work), 256, 0, st>>>((double2*)out, N, n, batch, dist);
-    else k_r2c_post<float2><<<grid_for(work), 256, 0, st>>>((float2*)out, N, n, batch, dist);
+    const long long half = N / 2 + 1, total = half * batch, grid = (total + 255) / 256;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+    if (dtype == CFFT_DT_C128)
+        k_r2c_post<double2><<<(unsigned)grid, 256, 0, st>>>((double2*)out, (int)N, w, half, total, dist);
+    else
+        k_r2c_post<float2><<<(unsigned)grid, 256, 0, st>>>((float2*)out, (int)N, w, half, total, dist);
     return cudaGetLastError();
 }
-cudaError_t cfft_c2r_pre(const void* in, void* z, long long N, long long n, long long batch, long long in_dist,
-                         double scale, int dtype, cudaStream_t st) {
-    const long long work = N * batch;
+cudaError_t cfft_c2r_pre(const void* in, void* z, long long N, const TwoLevel& w, long long batch,
+                         long long in_dist, double scale, int dtype, cudaStream_t st) {
+    const long long half = N / 2 + 1, total = half * batch, grid = (total + 255) / 256;
+    if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
     if (dtype == CFFT_DT_C128)
-        k_c2r_pre<double2><<<grid_for(work), 256, 0, st>>>((const double2*)in, (double2*)z, N, n, batch, in_dist, scale);
+        k_c2r_pre<double2><<<(unsigned)grid, 256, 0, st>>>((const double2*)in, (double2*)z, (int)N, w, half, total,
+                                                            in_dist, scale);
     else
-        k_c2r_pre<float2><<<grid_for(work), 256, 0, st>>>((const float2*)in, (float2*)z, N, n, batch, in_dist, scale);
+        k_c2r_pre<float2><<<(unsigned)grid, 256, 0, st>>>((const float2*)in, (float2*)z, (int)N, w, half, total,
+                                                           in_dist, scale);
     return cudaGetLastError();
 }
 cudaError_t cfft_r2c_widen(const void* x, void* s, long long n, long long batch, int dtype, cudaStream_t st) {
