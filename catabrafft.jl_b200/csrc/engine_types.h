@@ -33,14 +33,14 @@ struct SubPlan {
 #define SF_MAXS 6
 struct SfPlan {
     int L, np;
-    int r[SF_MAXS];
+    unsigned char r[SF_MAXS + 2];
     // forward twiddles of stage s < np - 1 (Ls = r[s] r[s+1] ..., nb = Ls / r[s]):
     //   tw[off[s] + (k - 1) nb + t] = w_Ls^(t k), 1 <= k < r[s], t < nb
-    int off[SF_MAXS];
+    unsigned short off[SF_MAXS];
     // twiddles of stage s >= 1 of a second transform that takes the digits
     // last to first (pre = r[0] .. r[s - 1], K = the index of digits 0 .. s - 1):
     //   tw[boff[s] + (n - 1) pre + b] = w_(pre r[s])^(K(b) n), 1 <= n < r[s], b < pre
-    int boff[SF_MAXS];
+    unsigned short boff[SF_MAXS];
     int twlen;                    // entries of the forward blocks
     int twall;                    // entries of all blocks
     // ceil(2^32 / d) for quotients by d = nb of stage s, L / r[s] and r[s] (sf_div)
@@ -79,8 +79,10 @@ struct KParams {
     int PA, PC;                   // smem pitches (column layout / row layout)
     int XP;                       // Rader x staging: row pitch (ROWS) or chunk (FOUR)
     int pre, post;                // pass prologue / epilogue
-    SubPlan pa, pc;               // ROWS / FOUR: column (N1) / row (N2, or M in ROWS) plans
-    SfPlan sa, sc;                // passes: column (N1) / row (N2) sub-transforms
+    union {                       // FOUR: column (N1) / row (N2) plans; passes.cuh: sub-transforms
+        struct { SubPlan pa, pc; };
+        struct { SfPlan sa, sc; };
+    };
     unsigned mv;                  // passes: multiplier of V (V = tile width of COLPASS / ROWPASS, rows of MIDPASS)
     int ks;                       // passes: floor(threads / V)
     int qp, qw;                   // ROWPASS / MIDPASS / LINE: pitches of a last-radix run and of a row

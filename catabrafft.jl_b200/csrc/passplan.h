@@ -63,14 +63,14 @@ inline bool sf_plan(int L, SfPlan& S, int maxr = 16) {
     if (n > SF_MAXS) return false;
     S.np = n < 2 ? 2 : n;
     if (n == 1) {
-        S.r[0] = best[0];
+        S.r[0] = (unsigned char)best[0];
         S.r[1] = 1;
     } else {
-        for (int i = 0; i < n; i++) S.r[i] = best[n - 1 - i];
+        for (int i = 0; i < n; i++) S.r[i] = (unsigned char)best[n - 1 - i];
     }
     int off = 0, Ls = L;
     for (int s = 0; s < S.np - 1; s++) {
-        S.off[s] = off;
+        S.off[s] = (unsigned short)off;      // at most 2 x 9216 entries
         off += (S.r[s] - 1) * (Ls / S.r[s]);
         Ls /= S.r[s];
     }
@@ -78,7 +78,7 @@ inline bool sf_plan(int L, SfPlan& S, int maxr = 16) {
     int pre = 1;
     for (int s = 1; s < S.np; s++) {
         pre *= S.r[s - 1];
-        S.boff[s] = off;
+        S.boff[s] = (unsigned short)off;
         off += (S.r[s] - 1) * pre;
     }
     S.twall = off;
