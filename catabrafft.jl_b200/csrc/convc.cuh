@@ -66,17 +66,19 @@ __device__ __forceinline__ void convc_rader_body(const KParams& p, unsigned char
         const V* x = (const V*)p.in + (long long)tr * p.in_dist;
         const int* pc = p.perm + c * 4096 + t;
         double2 acc = make_double2(0, 0);
+        // padding (-1) reads x[0]: no branch keeps the sixteen gathers apart
+        // (with one, each waited for the one before)
+        int src[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) src[k] = __ldg(pc + 256 * k);
+#pragma unroll
+        for (int k = 0; k < 16; k++) v[k] = __ldg(x + max(src[k], 0));
 #pragma unroll
         for (int k = 0; k < 16; k++) {
-            const int src = __ldg(pc + 256 * k);
-            V a = zero<V>();
-            if (src >= 0) {
-                a = load_in(p, __ldg(x + src));
-                const double2 d = tod(a);
-                acc.x += d.x;
-                acc.y += d.y;
-            }
-            v[k] = a;
+            v[k] = src[k] >= 0 ? load_in(p, v[k]) : zero<V>();
+            const double2 d = tod(v[k]);
+            acc.x += d.x;
+            acc.y += d.y;
         }
         const double2 s = block_sum(acc, red);  // barriers inside: tables staged too
         if (t == 0) *part = s;
@@ -113,12 +115,15 @@ __device__ __forceinline__ void convc_rader_body(const KParams& p, unsigned char
             w[0] = make_double2(1, 0);
             w[1] = convc_w(p.t4n, (unsigned)k);
 #pragma unroll
-            for (int q = 2; q < C; q++) w[q] = cmul(w[q - 1], w[1]);
+            for (int q = 2; q < C; q++) w[q] = cmul(w[q / 2], w[q - q / 2]);
 #pragma unroll
             for (int q = 1; q < C; q++) f[q] = cmul(f[q], fromd<V>(w[q]));
+            double2 sp[C];                      // in flight during the DFT
+#pragma unroll
+            for (int q = 0; q < C; q++) sp[q] = __ldg(p.spec + k + 4096 * q);
             dft<C>(f);                          // f[q] = A[k + 4096 q]
 #pragma unroll
-            for (int q = 0; q < C; q++) f[q] = conjv(fromd<V>(cmul(tod(f[q]), __ldg(p.spec + k + 4096 * q))));
+            for (int q = 0; q < C; q++) f[q] = conjv(fromd<V>(cmul(tod(f[q]), sp[q])));
             dft<C>(f);                          // f[q] = sum_r u[k + 4096 r] w_C^(rq)
 #pragma unroll
             for (int q = 1; q < C; q++) f[q] = cmul(f[q], fromd<V>(w[q]));

@@ -331,6 +331,27 @@ __device__ __forceinline__ double2 r4096_w(const double2* lo, const double2* hi,
     const unsigned l = e & 63;
     return cmul(lo[l ^ (l >> 3)], hi[e >> 6]);
 }
+// f(k, b^k) for k = 1 .. R - 1 in order: FP64 products in two chains (even and
+// odd k, both stepping by b^2), so that half as many wait for one another, for
+// one more product and eight registers.  Against one chain, B200: 4096 x 16384
+// ComplexF64 385 -> 370 us, 8192 x 4096 294 -> 282, 16384 x 2048 363 -> 358; in
+// the row pass and the column DFTs of pow2.cuh and in mixc.cuh one chain stayed
+// 1 - 3 % faster.
+template <int R, class F> __device__ __forceinline__ void fp64_powers(double2 b, F f) {
+    double2 odd = b;
+    f(1, odd);
+    if constexpr (R > 2) {
+        const double2 sq = cmul(b, b);
+        double2 even = sq;
+        f(2, even);
+#pragma unroll
+        for (int k = 3; k < R; k++) {
+            double2& w = (k & 1) ? odd : even;
+            w = cmul(w, sq);
+            f(k, w);
+        }
+    }
+}
 // dst[k stride] = v[k] w_4096^(e0 k), k < 16 (e0 k < 4096): the FP64 powers
 // w^(e0 k) = w^(e0 (k-1)) w^e0 of one two-level table value, each rounded
 // once to V.  The FP64 power's relative error stays below ~4e-15.  Against
@@ -339,25 +360,29 @@ __device__ __forceinline__ double2 r4096_w(const double2* lo, const double2* hi,
 // go: measured on B200, 4096-point ComplexF64 0.446 -> 0.376 ms per GiB,
 // 1024 x 10007 (Rader) 0.516 -> 0.453 ms, 4096 x 2^16 ComplexF32 2.97 ->
 // 2.52 ms (the table reads were most of the shared-memory wavefronts).
-template <typename V>
+template <typename V, bool TWO>
 __device__ __forceinline__ void r4096_tw_store(V (&v)[16], V* dst, int stride, const double2* lo,
                                                const double2* hi, unsigned e0) {
-    const double2 b = r4096_w(lo, hi, e0);
-    double2 w = b;
     dst[0] = v[0];
+    const double2 b = r4096_w(lo, hi, e0);
+    if constexpr (TWO) {
+        fp64_powers<16>(b, [&](int k, double2 w) { dst[k * stride] = cmul(v[k], fromd<V>(w)); });
+    } else {
+        double2 w = b;
 #pragma unroll
-    for (int k = 1; k < 16; k++) {
-        dst[k * stride] = cmul(v[k], fromd<V>(w));
-        if (k < 15) w = cmul(w, b);
+        for (int k = 1; k < 16; k++) {
+            dst[k * stride] = cmul(v[k], fromd<V>(w));
+            if (k < 15) w = cmul(w, b);
+        }
     }
 }
 // 4096-point DFT of the registers: thread t holds x[t + 256 k] in v[k] and
 // gets X[t + 256 k3] in v[k3].  buf (16 planes of R4096_PL elements) must be
 // free on entry; on return every thread has finished reading it.
-template <typename V>
+template <typename V, bool TWO = true>
 __device__ __forceinline__ void fft4096_regs(V (&v)[16], V* buf, const double2* tlo, const double2* thi, int t) {
     dft<16>(v);
-    r4096_tw_store(v, buf + t, 256, tlo, thi, (unsigned)t);
+    r4096_tw_store<V, TWO>(v, buf + t, 256, tlo, thi, (unsigned)t);
     __syncthreads();
     {
         const int t1 = t & 15, k1 = t >> 4;
@@ -365,7 +390,7 @@ __device__ __forceinline__ void fft4096_regs(V (&v)[16], V* buf, const double2* 
         for (int t2 = 0; t2 < 16; t2++) v[t2] = buf[k1 * 256 + t1 + 16 * t2];
         dft<16>(v);
         __syncthreads();                        // every Y read before Z overwrites it
-        r4096_tw_store(v, buf + k1 * R4096_PL + t1, R4096_PB, tlo, thi, (unsigned)(16 * t1));
+        r4096_tw_store<V, TWO>(v, buf + k1 * R4096_PL + t1, R4096_PB, tlo, thi, (unsigned)(16 * t1));
     }
     __syncthreads();
     {
@@ -459,7 +484,7 @@ __device__ __forceinline__ void r4096_body(const KParams& p, unsigned char* smem
 #pragma unroll
         for (int k = 0; k < 16; k++) v[k] = load_in(p, buf[t + 256 * k]);
         dft<16>(v);
-        r4096_tw_store(v, buf + t, 256, tlo, thi, (unsigned)t);
+        r4096_tw_store<V, !P2A>(v, buf + t, 256, tlo, thi, (unsigned)t);
         if (TMA) {
             // every thread leaves together when a copy timed out
             if (__syncthreads_or(!ok)) {
@@ -475,7 +500,7 @@ __device__ __forceinline__ void r4096_body(const KParams& p, unsigned char* smem
             for (int t2 = 0; t2 < 16; t2++) v[t2] = buf[k1 * 256 + t1 + 16 * t2];
             dft<16>(v);
             __syncthreads();                    // every Y read before Z overwrites it
-            r4096_tw_store(v, buf + k1 * R4096_PL + t1, R4096_PB, tlo, thi, (unsigned)(16 * t1));
+            r4096_tw_store<V, !P2A>(v, buf + k1 * R4096_PL + t1, R4096_PB, tlo, thi, (unsigned)(16 * t1));
         }
         __syncthreads();
         {

@@ -247,7 +247,7 @@ __device__ __forceinline__ void p2row_pair_body(const KParams& p, unsigned char*
                     p2row_pair_issue(p, pair, tm, bar, bn);
                 }
             }
-            fft4096_regs(v, buf, tlo, thi, t);
+            fft4096_regs<float2, false>(v, buf, tlo, thi, t);
             float2* out = (float2*)p.out + (long long)(2 * b + h) * p.out_dist;
 #pragma unroll
             for (int k3 = 0; k3 < 16; k3++) out[t + 256 * k3] = v[k3];
@@ -407,12 +407,7 @@ __device__ __forceinline__ void p2cl_body(const KParams& p, unsigned char* smem,
             for (int q = 0; q < C; q++) f[q] = cl.map_shared_rank(buf, q)[k];
             // w_n^(q k) as FP64 powers of one table value, rounded once
             const double2 wk = cmul(__ldg(p.t4n.lo + (k & mask)), __ldg(p.t4n.hi + (k >> p.t4n.bits)));
-            double2 w = wk;
-#pragma unroll
-            for (int q = 1; q < C; q++) {
-                f[q] = cmul(f[q], fromd<V>(w));
-                if (q + 1 < C) w = cmul(w, wk);
-            }
+            fp64_powers<C>(wk, [&](int q, double2 w) { f[q] = cmul(f[q], fromd<V>(w)); });
             dft<C>(f);
 #pragma unroll
             for (int q = 0; q < C; q++) stg_stream(out + k + 4096 * q, store_out(p, f[q]));
@@ -530,7 +525,7 @@ __device__ __forceinline__ void p2flow_body(const KParams& pa, const KParams& pb
 #pragma unroll
                 for (int k = 0; k < 16; k++) v[k] = load_in(pa, buf[t + 256 * k]);
             }
-            fft4096_regs(v, buf, tlo, thi, opaque_tid());
+            fft4096_regs<V, false>(v, buf, tlo, thi, opaque_tid());
             {
                 const int t = opaque_tid();
                 V* row = (V*)fc.ring + (long long)(tr % fc.depth) * n + ((long long)i << 12);
