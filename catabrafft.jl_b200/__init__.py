@@ -71,6 +71,13 @@ def _is_torch(x) -> bool:
     return type(x).__module__.startswith("torch")
 
 
+def _stream_handle(index: int) -> int:
+    """torch's current stream on a device, as a cudaStream_t."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)     # without a Stream object, where torch has it
+    return raw(index) if raw is not None else torch.cuda.current_stream(index).cuda_stream
+
+
 class _Plan:
     """Owns one cfft_plan handle (device tables, scratch)."""
 
@@ -291,6 +298,9 @@ class Spell:
         self.device = device
         self.direction = int(direction)
         self.inverse = None
+        # what the direct path of p * x compares with (None: never taken)
+        self._torch_type = datatype if _is_torch(datatype) else None
+        self._shapes = ((self.batch, self.n), (self.n,) if self.batch == 1 else None)
         self._plan = _get_plan(self.n, self.batch, _dtype_code(datatype), self.flag, device)
 
     def describe(self) -> str:
@@ -305,6 +315,19 @@ class Spell:
             raise ValueError(f"plan is for n={self.n}, batch={self.batch}; got n={n}, batch={batch}")
 
     def __mul__(self, x):
+        # The planned case -- a contiguous device tensor of the plan's type and
+        # shape, on its device, which is current -- goes straight to the C
+        # entry: the general path's lookups and stream objects made a
+        # 4096-point call 12.4 us of host time, against 8 us on the device.
+        if self._torch_type is not None and type(x).__module__ == "torch" and x.dtype is self._torch_type \
+                and x.is_cuda and x.shape in self._shapes and x.is_contiguous():
+            import torch
+            plan, index = self._plan, self.device
+            if plan.handle is not None and x.get_device() == index and torch.cuda.current_device() == index:
+                y = torch.empty_like(x)
+                check(_lib.LIB.cfft_execute(plan.handle, x.data_ptr(), y.data_ptr(), self.direction,
+                                            _stream_handle(index)))
+                return y
         self._check(x)
         return _run(x, self.direction, self.flag)
 
