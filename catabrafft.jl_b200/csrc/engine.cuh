@@ -1,20 +1,18 @@
 // engine.cuh -- device side of the B200 1D complex FFT.
 //
-// One transform (or a tile of sub-transforms) is staged in shared memory and
-// every radix pass runs there; HBM is touched once on the way in and once on
-// the way out.  Two work shapes share the same in-place Stockham core:
+// Helpers shared by every kernel, the n = 4096 register kernel, and the FOUR
+// kernels, which run convolutions (ComplexF64 Rader beyond one CTA, and a range
+// of Bluestein lengths) of length M = N1*N2 split over a thread-block cluster
+// of C CTAs: column FFTs (length N1) in each CTA, twiddle w_M^(i2*k1),
+// exchange through distributed shared memory, row FFTs (length N2).  C = 1 is
+// the single-CTA four-step.  (Other lengths: passes.cuh, pow2.cuh, mixc.cuh,
+// convc.cuh.)  Every radix pass of FOUR runs in shared memory.
 //
-//   ROWS     V whole transforms per CTA (small n), one row each.
-//   FOUR     one transform of length M = N1*N2 split over a thread-block
-//            cluster of C CTAs: column FFTs (length N1) in each CTA, twiddle
-//            w_M^(i2*k1), exchange through distributed shared memory, row
-//            FFTs (length N2).  C = 1 is the single-CTA four-step.
-//
-// Rader (prime n) and Bluestein (other non-smooth n) are fused into ROWS and
-// FOUR: the prologue builds the zero-padded convolution input (generator
-// permutation or chirp), the convolution runs as FFT_M -> pointwise multiply
-// by a precomputed FP64 spectrum -> FFT_M of the conjugate, and the epilogue
-// applies the inverse permutation (+x0) or the output chirp.
+// Rader (prime n) and Bluestein (other non-smooth n) are fused into FOUR: the
+// prologue builds the zero-padded convolution input (generator permutation or
+// chirp), the convolution runs as FFT_M -> pointwise multiply by a precomputed
+// FP64 spectrum -> FFT_M of the conjugate, and the epilogue applies the
+// inverse permutation (+x0) or the output chirp.
 //
 // The Stockham pass is the reference's shell_layered pass
 // (src/radix_2_codelets.jl:402-447 and siblings): inputs x[q + s(p + k n1)],

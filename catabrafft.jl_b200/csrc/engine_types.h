@@ -75,9 +75,9 @@ struct KParams {
     int nx;                       // user transform length
     int M;                        // working FFT length (nx unless conv)
     int N1, N2, C;                // FOUR / pass split
-    int V;                        // ROWS: transforms per CTA; passes: tile width
+    int V;                        // LINE / LCONV: transforms per CTA; passes: tile width
     int PA, PC;                   // smem pitches (column layout / row layout)
-    int XP;                       // Rader x staging: row pitch (ROWS) or chunk (FOUR)
+    int XP;                       // Rader x staging: chunk (FOUR)
     int pre, post;                // pass prologue / epilogue
     union {                       // FOUR: column (N1) / row (N2) plans; passes.cuh: sub-transforms
         struct { SubPlan pa, pc; };

@@ -24,7 +24,7 @@ const void* cfft_pass_kernel64(int mode, bool batched);
 // nullptr; *single (if given) = 1 when it keeps one buffer for both layouts
 const void* cfft_static_four(int dtype, int N1, int N2, int C, const unsigned char* ca,
                              const unsigned char* cc, int* single = nullptr);
-// n = 4096 register kernel (KParams of a one-transform-per-CTA ROWS stage
+// n = 4096 register kernel (KParams of a one-transform-per-CTA LINE stage
 // plus t4 = the two-level table of w_4096) and its shared memory
 const void* cfft_r4096_kernel(int dtype);
 size_t cfft_r4096_smem(size_t elem_bytes);

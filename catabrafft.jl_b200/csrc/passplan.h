@@ -116,6 +116,10 @@ inline __host__ __device__ void sf_tw_entry(const SfPlan& S, int i, long long* e
 // shared memory per CTA: three ComplexF32 or two ComplexF64 CTAs per SM (the
 // register budgets of the kernels)
 inline size_t sf_budget(size_t e) { return (e == 8 ? 74 : 112) * (size_t)1024; }
+// ... and of a pass's tile: ComplexF64 tiles above 76 KB leave too little of an
+// SM's L1 to the loads in flight (10^6 x 64 1422 us at 112 KB, 1212 at 76, 1283
+// at 64; 999983 x 32 2246 / 2182 / 2219)
+inline size_t sf_pass_budget(size_t e) { return (e == 8 ? 74 : 76) * (size_t)1024; }
 // Pitches of a row tile, in elements: of a last-radix run, and of a row.
 // ROWPASS's later stages take V adjacent rows in adjacent lanes: B lanes (16
 // ComplexF32, 8 ComplexF64) share a wavefront, so from V = B rows an odd row
@@ -159,7 +163,7 @@ inline double sf_crowd(size_t smem, size_t e) {
 // cycles per useful element of a COLPASS / ROWPASS tile of width V
 inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bool row) {
     const size_t smem = row ? sf_row_smem(S, V, e, false) : sf_col_smem(S, V, e);
-    if (smem > sf_budget(e)) return 1e9 + (double)smem;
+    if (smem > sf_pass_budget(e)) return 1e9 + (double)smem;
     const int ks = SF_THREADS / V;
     double c = sf_start();
     for (int s = 0; s < S.np; s++) {
@@ -199,7 +203,7 @@ inline double sf_pass_cost(const SfPlan& S, long long count, size_t e, bool row)
 // stage fused with the first one's last
 inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e) {
     const size_t smem = sf_row_smem(S, V, e, true);
-    if (smem > sf_budget(e)) return 1e9 + (double)smem;
+    if (smem > sf_pass_budget(e)) return 1e9 + (double)smem;
     double c = sf_start();
     for (int s = 0; s < S.np; s++) {
         const int rounds = (V * (S.L / S.r[s]) + SF_THREADS - 1) / SF_THREADS;

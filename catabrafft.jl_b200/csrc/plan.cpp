@@ -2,7 +2,7 @@
 //
 // Host-side counterpart of CatabraFFT.jl's dispatcher (src/kernel.jl:72-199),
 // planner (src/radix_plan.jl) and plan object (src/spells.jl).  Strategy:
-//   n 7-smooth          -> Stockham on the device (ROWS / FOUR / two HBM passes)
+//   n 7-smooth          -> Stockham on the device (one CTA, a cluster, or two HBM passes)
 //   n prime             -> Rader (src/prime.jl): generator permutation, cyclic
 //                          convolution of length n-1 through a zero-padded
 //                          smooth FFT of length M >= 2n-3, inverse permutation
@@ -281,7 +281,7 @@ struct Stage {
 };
 
 struct Shape {
-    int mode = MODE_ROWS;    // ROWS, FOUR or GLOBAL(=MODE_COLPASS)
+    int mode = MODE_ROWS;    // ROWS (LINE / LCONV), FOUR (CLUS without a convolution), COLPASS (the HBM passes), ...
     int conv = CONV_NONE;
     int64_t M = 0;
     int N1 = 1, N2 = 1, C = 1, V = 1;
@@ -1162,6 +1162,20 @@ static int64_t scratch_budget(bool pow2 = false) {
     if (mb > 0 && mb <= (1LL << 20)) return (int64_t)mb << 20;
     return (int64_t)(pow2 ? 512 : 64) << 20;
 }
+// transforms per chunk of the generic passes, `one` bytes of intermediate each:
+// the whole batch up to 64 MB, else the fewest equal chunks of at most 512 MB,
+// at least two (the scratch then stays within half the data).  Measured on B200
+// by chunk size 64 / 128 / 256 / 512 MB: 10^6 x 64 ComplexF32 783 / 722 / 664 /
+// 631 us, 4096 x 3^9 814 / 794 / 745 / 713, 999983 x 32 1740 / 1508 / 1347 /
+// 1266, ComplexF64 999983 x 32 2848 / 2591 / 2376 / 2245 -- a launch's last wave
+// and start cost more than reading the intermediate back from HBM
+static int64_t pass_chunk(int64_t batch, int64_t one) {
+    if (getenv("CFFT_SCRATCH_MB")) return std::min<int64_t>(batch, std::max<int64_t>(1, scratch_budget() / one));
+    if (batch * one <= ((int64_t)64 << 20)) return batch;
+    const int64_t most = std::max<int64_t>(1, ((int64_t)512 << 20) / one);
+    int64_t n = std::max<int64_t>(2, (batch + most - 1) / most);
+    return std::max<int64_t>(1, (batch + n - 1) / n);
+}
 
 static int plan_build(cfft_plan_s* P, const Shape& sh) {
     P->shape = sh;
@@ -1654,15 +1668,21 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     if (rc) return rc;
     kp.N1 = (int)N1;
     kp.N2 = (int)N2;
-    // chunk the batch so the scratch of one chunk stays within ~64 MB (L2 sized)
-    int64_t chunk = std::max<int64_t>(1, scratch_budget() / (int64_t)(M * e));
-    chunk = std::min<int64_t>(chunk, P->batch);
-    P->chunk = chunk;
-    P->scratch_bytes = (size_t)chunk * M * e;
+    int64_t chunk = pass_chunk(P->batch, M * (int64_t)e);
     if (!P->shared_scratch) {
-        CUDA_TRY(lib_malloc(&P->scratch[0], P->scratch_bytes));
+        // where the device cannot hold that scratch, smaller chunks down to 64 MB
+        cudaError_t ce;
+        for (;;) {
+            ce = lib_malloc(&P->scratch[0], (size_t)chunk * M * e);
+            if (ce != cudaErrorMemoryAllocation || chunk * M * (int64_t)e <= ((int64_t)64 << 20) || chunk == 1) break;
+            cudaGetLastError();
+            chunk = (chunk + 1) / 2;
+        }
+        CUDA_TRY(ce);
         P->allocs.push_back(P->scratch[0]);
     }
+    P->chunk = chunk;
+    P->scratch_bytes = (size_t)chunk * M * e;
     auto add = [&](int mode, int pre, int post, int in_sel, int out_sel) {
         Stage s;
         s.kp = kp;
