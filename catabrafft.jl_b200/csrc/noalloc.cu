@@ -199,11 +199,11 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
     KParams col = kp, row = kp;
     col.mode = MODE_COLPASS;
     size_t smem_col = 0, smem_row = 0;
-    sf_stage(col, e, &smem_col);
+    sf_stage(col, e, &smem_col, true);
     col.pre = PRE_NONE;
     col.post = POST_TWIDDLE;
     row.mode = MODE_ROWPASS;
-    sf_stage(row, e, &smem_row);
+    sf_stage(row, e, &smem_row, true);
 
     const long long chunk = std::max<long long>(1, (long long)(kScratchBytes / ((size_t)n * e)));
     for (long long b0 = 0; b0 < batch; b0 += chunk) {

@@ -48,7 +48,7 @@ inline void sf_search(int rem, int maxr, int depth, double cost, int* cur, int* 
 // 0 stands for d = 1
 inline unsigned sf_magic(int d) { return d == 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
 // fills L, np, r and the table layout; false if L has no sequence
-inline bool sf_plan(int L, SfPlan& S, int maxr = 16) {
+inline bool sf_plan(int L, SfPlan& S, int maxr = 16, bool line = false) {
     S = SfPlan();
     S.L = L;
     if (L < 1) return false;
@@ -61,6 +61,16 @@ inline bool sf_plan(int L, SfPlan& S, int maxr = 16) {
     double c = 1e30;
     sf_search(L, maxr, 0, 0.0, cur, best, &n, &c);
     if (n > SF_MAXS) return false;
+    if (line && n == 1) {
+        // a row of one butterfly is read a row per lane: two stages where L
+        // factors, whose lanes read adjacent elements
+        for (int a = 4; a >= 2 && n == 1; a--)
+            if (L % a == 0 && L / a >= a) {
+                best[0] = L / a;
+                best[1] = a;
+                n = 2;
+            }
+    }
     S.np = n < 2 ? 2 : n;
     if (n == 1) {
         S.r[0] = (unsigned char)best[0];
@@ -116,9 +126,11 @@ inline __host__ __device__ void sf_tw_entry(const SfPlan& S, int i, long long* e
 // shared memory per CTA: three ComplexF32 or two ComplexF64 CTAs per SM (the
 // register budgets of the kernels)
 inline size_t sf_budget(size_t e) { return (e == 8 ? 74 : 112) * (size_t)1024; }
-// ... and of a pass's tile: ComplexF64 tiles above 76 KB leave too little of an
-// SM's L1 to the loads in flight (10^6 x 64 1422 us at 112 KB, 1212 at 76, 1283
-// at 64; 999983 x 32 2246 / 2182 / 2219)
+// ... and of a pass's tile in a launch of its own: ComplexF64 tiles above 76 KB
+// leave too little of an SM's L1 to the loads in flight (10^6 x 64 1422 us at
+// 112 KB, 1212 at 76, 1283 at 64; 999983 x 32 2246 / 2182 / 2219).  The work
+// queue's items keep the larger tiles: each pays the queue's overhead (1000
+// mixed lengths 5785 us against 6580)
 inline size_t sf_pass_budget(size_t e) { return (e == 8 ? 74 : 76) * (size_t)1024; }
 // Pitches of a row tile, in elements: of a last-radix run, and of a row.
 // ROWPASS's later stages take V adjacent rows in adjacent lanes: B lanes (16
@@ -161,9 +173,9 @@ inline double sf_crowd(size_t smem, size_t e) {
     return total > 130.0 ? 1.0 + 0.12 * (total - 130.0) / 68.0 : 1.0;
 }
 // cycles per useful element of a COLPASS / ROWPASS tile of width V
-inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bool row) {
+inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bool row, size_t budget) {
     const size_t smem = row ? sf_row_smem(S, V, e, false) : sf_col_smem(S, V, e);
-    if (smem > sf_pass_budget(e)) return 1e9 + (double)smem;
+    if (smem > budget) return 1e9 + (double)smem;
     const int ks = SF_THREADS / V;
     double c = sf_start();
     for (int s = 0; s < S.np; s++) {
@@ -181,11 +193,11 @@ inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bo
     return c / ((double)V * S.L) * (double)(tiles * V) / (double)count;
 }
 // the width with the least cost (at most 64)
-inline int sf_tile(const SfPlan& S, long long count, size_t e, bool row, double* cost = nullptr) {
+inline int sf_tile(const SfPlan& S, long long count, size_t e, bool row, size_t budget, double* cost = nullptr) {
     int best = 1;
     double bc = 1e300;
     for (int V = 1; V <= 64 && V <= count; V++) {
-        const double c = sf_tile_cost(S, V, count, e, row);
+        const double c = sf_tile_cost(S, V, count, e, row, budget);
         if (c < bc) {
             bc = c;
             best = V;
@@ -196,14 +208,14 @@ inline int sf_tile(const SfPlan& S, long long count, size_t e, bool row, double*
 }
 inline double sf_pass_cost(const SfPlan& S, long long count, size_t e, bool row) {
     double c;
-    sf_tile(S, count, e, row, &c);
+    sf_tile(S, count, e, row, sf_budget(e), &c);
     return c;
 }
 // MIDPASS: whole rows, contiguous on both sides, the second transform's first
 // stage fused with the first one's last
-inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e) {
+inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e, size_t budget) {
     const size_t smem = sf_row_smem(S, V, e, true);
-    if (smem > sf_pass_budget(e)) return 1e9 + (double)smem;
+    if (smem > budget) return 1e9 + (double)smem;
     double c = sf_start();
     for (int s = 0; s < S.np; s++) {
         const int rounds = (V * (S.L / S.r[s]) + SF_THREADS - 1) / SF_THREADS;
@@ -212,11 +224,11 @@ inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e
     const long long tiles = (count + V - 1) / V;
     return c / ((double)V * S.L) * (double)(tiles * V) / (double)count;
 }
-inline int sf_mid_rows(const SfPlan& S, long long count, size_t e, double* cost = nullptr) {
+inline int sf_mid_rows(const SfPlan& S, long long count, size_t e, size_t budget, double* cost = nullptr) {
     int best = 1;
     double bc = 1e300;
     for (int V = 1; V <= 32 && V <= count; V++) {
-        const double c = sf_mid_tile_cost(S, V, count, e);
+        const double c = sf_mid_tile_cost(S, V, count, e, budget);
         if (c < bc) {
             bc = c;
             best = V;
@@ -224,11 +236,6 @@ inline int sf_mid_rows(const SfPlan& S, long long count, size_t e, double* cost 
     }
     if (cost) *cost = bc;
     return best;
-}
-inline double sf_mid_cost(const SfPlan& S, long long count, size_t e) {
-    double c;
-    sf_mid_rows(S, count, e, &c);
-    return c;
 }
 // LINE: V whole rows; lanes of the first and middle stages walk a row, those
 // of the last one step by the first digit's pitch (odd)
@@ -290,11 +297,13 @@ inline int sf_lconv_rows(const SfPlan& S, long long batch, size_t e, double* cos
     return best;
 }
 // tile, pitches and shared memory of a pass (mode, N1, N2, sa, sc set)
-inline void sf_stage(KParams& k, size_t e, size_t* smem) {
+// (own: in a launch of its own)
+inline void sf_stage(KParams& k, size_t e, size_t* smem, bool own) {
+    const size_t budget = own ? sf_pass_budget(e) : sf_budget(e);
     const bool mid = k.mode == MODE_MIDPASS;
-    if (k.mode == MODE_COLPASS) k.V = sf_tile(k.sa, k.N2, e, false);
-    else if (mid) k.V = sf_mid_rows(k.sc, k.N1, e);
-    else k.V = sf_tile(k.sc, k.N1, e, true);
+    if (k.mode == MODE_COLPASS) k.V = sf_tile(k.sa, k.N2, e, false, budget);
+    else if (mid) k.V = sf_mid_rows(k.sc, k.N1, e, budget);
+    else k.V = sf_tile(k.sc, k.N1, e, true, budget);
     k.mv = sf_magic(k.V);
     k.ks = SF_THREADS / k.V;
     k.qp = sf_qp(k.sc, k.V, e, mid);

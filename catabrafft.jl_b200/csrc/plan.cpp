@@ -384,7 +384,7 @@ static const SfPlan* sf_line(int64_t L, int dtype) {
         for (int l = 1; l <= kLineMax; l++)
             for (int d = 0; d < 2; d++) {
                 SfPlan& S = t[d * (kLineMax + 1) + l];
-                if (!is_smooth7(l) || !sf_plan(l, S, d ? 20 : 16)) S.L = 0;
+                if (!is_smooth7(l) || !sf_plan(l, S, d ? 20 : 16, true)) S.L = 0;
             }
         return t;
     }();
@@ -554,7 +554,8 @@ static double sf_cost(int64_t L, int64_t count, size_t e, int kind) {
                 const size_t el = i < 3 ? 8 : 16;
                 const SfPlan* S = sf_get(l);
                 if (!S) continue;
-                x.V = i % 3 == 2 ? sf_mid_rows(*S, 1 << 16, el, &x.c) : sf_tile(*S, 1 << 16, el, i % 3 == 1, &x.c);
+                x.V = i % 3 == 2 ? sf_mid_rows(*S, 1 << 16, el, sf_budget(el), &x.c)
+                                     : sf_tile(*S, 1 << 16, el, i % 3 == 1, sf_budget(el), &x.c);
             }
         }
         return t;
@@ -1689,7 +1690,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         s.kp.mode = mode;
         s.kp.pre = pre;
         s.kp.post = post;
-        sf_stage(s.kp, e, &s.smem);
+        sf_stage(s.kp, e, &s.smem, !P->shared_scratch);
         s.threads = CFFT_THREADS;
         s.cluster = 1;
         s.in_sel = in_sel;
@@ -1886,7 +1887,7 @@ static void wisdom_store(const WisdomKey& k, const std::string& sig) {
 // in its own first and last kernel.  The register kernels keep contiguous
 // data of the plan's type: their ComplexF16 and strided plans widen / gather
 // in a sweep of their own (measured faster there: 4096 x 2^16 ComplexF32
-// runs 1.76 ms on the register passes, 3.49 ms as generic two-pass).
+// runs 1.8 ms on the register passes, 2.3 ms on the stage kernels' two).
 static bool io_fusable(const cfft_plan_s* P) {
     for (const auto& st : P->stages) {
         const int m = st.kp.mode;
@@ -3080,7 +3081,7 @@ int cfft_plan_create_many(cfft_plan* plan, int64_t n, int64_t batch, int dtype, 
         s.kp.N2 = (int)batch;
         s.kp.pre = PRE_NONE;
         s.kp.post = POST_STORE;
-        sf_stage(s.kp, e, &s.smem);
+        sf_stage(s.kp, e, &s.smem, true);
         s.cols = true;
         s.fn = cfft_kernel_for(MODE_COLS, dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64);
         if ((s.kp.V * e >= 32 || s.kp.V == batch) && s.smem <= sf_budget(e) &&

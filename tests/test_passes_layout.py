@@ -192,6 +192,13 @@ class Line(Row):
 
     def __init__(self, L):
         super().__init__(L)
+        if len(self.r) == 2 and self.r[1] == 1:        # one butterfly a row: two stages where L factors
+            for a in (4, 3, 2):
+                if L % a == 0 and L // a >= a:
+                    self.r = [a, L // a]
+                    break
+            self.rl = self.r[-1]
+            self.qp = self.rl | 1
         self.nb0 = L // self.r[0]
         self.q0 = 0 if len(self.r) < 3 or (self.nb0 // self.rl * self.qp) % 2 else 1
         self.qw = L // self.rl * self.qp + self.r[0] * self.q0
@@ -201,7 +208,7 @@ class Line(Row):
         return self.at(t) + t // self.nb0 * self.q0
 
 
-@pytest.mark.parametrize("L", LENGTHS + [8, 120, 2160, 3840, 8192, 8748, 6561, 7776])
+@pytest.mark.parametrize("L", LENGTHS + [3, 6, 7, 8, 9, 12, 14, 15, 120, 2160, 3840, 8192, 8748, 6561, 7776])
 def test_line_stages_are_the_dft(L):
     rng = np.random.default_rng(L + 2)
     x = rng.standard_normal(L) + 1j * rng.standard_normal(L)
