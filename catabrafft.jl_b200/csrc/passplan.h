@@ -211,9 +211,14 @@ inline double sf_pass_cost(const SfPlan& S, long long count, size_t e, bool row)
     sf_tile(S, count, e, row, sf_budget(e), &c);
     return c;
 }
+// MIDPASS and LCONV fuse the last stage with the second transform's first one
+// (mid_center), which has no radix-1 form: a length of one radix, whose
+// sequence is (L, 1), is no row of a convolution
+inline bool sf_mid_fits(const SfPlan& S) { return S.r[S.np - 1] >= 2; }
 // MIDPASS: whole rows, contiguous on both sides, the second transform's first
 // stage fused with the first one's last
 inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e, size_t budget) {
+    if (!sf_mid_fits(S)) return 1e300;
     const size_t smem = sf_row_smem(S, V, e, true);
     if (smem > budget) return 1e9 + (double)smem;
     double c = sf_start();

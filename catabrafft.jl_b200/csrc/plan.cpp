@@ -412,7 +412,7 @@ static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch
     double best = 1e300;
     for (int64_t m = M; m <= M + M / 50 && m <= kLineMax; m++) {
         const SfPlan* S = sf_line(m, dtype);
-        if (!S || S->r[S->np - 1] < 2 || sf_lconv_smem(*S, 1, e) > sf_budget(e)) continue;
+        if (!S || !sf_mid_fits(*S) || sf_lconv_smem(*S, 1, e) > sf_budget(e)) continue;
         double c;
         const int V = sf_lconv_rows(*S, batch, e, &c);
         if (c >= best) continue;
@@ -604,6 +604,7 @@ static bool conv_shape(int64_t M, int dtype, Shape& sh) {
         for (int tries = 0; tries < 2 && N2 <= kSfMax; tries++, N2++) {
             while (N2 <= kSfMax && !sf_get(N2)) N2++;
             if (N2 > kSfMax) break;
+            if (!sf_mid_fits(*sf_get(N2))) continue;
             const double sc = (double)(N1 * N2) * (2.0 * sf_cost(N1, N2, e, 0) + sf_cost(N2, N1, e, 2));
             if (sc < bests) { bests = sc; b1 = N1; b2 = N2; }
         }
@@ -1665,6 +1666,8 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     if (rc) return rc;
     rc = make_sfplan(P, N2, kp.sc);
     if (rc) return rc;
+    if (sh.conv != CONV_NONE && !sf_mid_fits(kp.sc))
+        return fail(CFFT_ERR_UNSUPPORTED, "convolution rows of one radix: " + std::to_string(N2));
     rc = make_twolevel(P, M, kp.t4);
     if (rc) return rc;
     kp.N1 = (int)N1;

@@ -1,0 +1,58 @@
+"""The host rules of the stage kernels (csrc/passplan.h), compiled here and
+called: which lengths a kernel takes, without a GPU."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from _pkg import PKG_DIR
+
+MAXS = 6
+
+
+class SfPlan(ctypes.Structure):
+    """engine_types.h"""
+    _fields_ = [("L", ctypes.c_int), ("np", ctypes.c_int), ("r", ctypes.c_ubyte * (MAXS + 2)),
+                ("off", ctypes.c_ushort * MAXS), ("boff", ctypes.c_ushort * MAXS),
+                ("twlen", ctypes.c_int), ("twall", ctypes.c_int),
+                ("mnb", ctypes.c_uint * MAXS), ("mper", ctypes.c_uint * MAXS), ("mr", ctypes.c_uint * MAXS),
+                ("tw", ctypes.c_void_p)]
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    so = tmp_path_factory.mktemp("probe") / "passplan_probe.so"
+    nvcc = os.path.realpath(shutil.which(os.environ.get("NVCC", "nvcc")))
+    cuda = os.path.join(os.path.dirname(os.path.dirname(nvcc)), "include")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "passplan_probe.cpp")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", cuda, "-I", os.path.join(PKG_DIR, "csrc"),
+                    src, "-o", str(so)], check=True)
+    lib = ctypes.CDLL(str(so))
+    lib.probe_mid_cost.restype = ctypes.c_double
+    lib.probe_mid_cost.argtypes = [ctypes.POINTER(SfPlan), ctypes.c_longlong, ctypes.c_int]
+    assert lib.probe_plan_bytes() == ctypes.sizeof(SfPlan)
+    return lib
+
+
+def plan(rules, L, maxr=16, line=False):
+    S = SfPlan()
+    return S if rules.probe_plan(L, maxr, int(line), ctypes.byref(S)) else None
+
+
+def test_convolution_rows_end_in_a_radix(rules):
+    # mid_center has no radix-1 form: a row length whose sequence ends in 1 (one
+    # radix) must not be priced as a row of a convolution
+    single = 0
+    for L in range(2, 4097):
+        S = plan(rules, L)
+        if S is None:
+            continue
+        costs = [rules.probe_mid_cost(ctypes.byref(S), 1 << 16, e) for e in (8, 16)]
+        if S.r[S.np - 1] < 2:
+            single += 1
+            assert min(costs) >= 1e9, (L, costs)
+        else:
+            assert max(costs) < 1e9, (L, costs)
+    assert single == 13          # 2 .. 10, 12, 14, 15 and 16
