@@ -82,6 +82,30 @@ static cudaError_t lib_free_host(void* p) {
     g_live_allocs.fetch_sub(1);
     return cudaFreeHost(p);
 }
+// a temporary in stream order (a cudaMalloc / cudaFree pair waits for the
+// device), or a plain allocation where the device has no memory pools
+template <class T> static cudaError_t lib_malloc_ordered(T** p, size_t bytes, cudaStream_t st, bool* ordered) {
+    *ordered = true;
+    if (alloc_injected_failure()) {
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
+    cudaError_t e = cudaMallocAsync((void**)p, bytes, st);
+    if (e == cudaErrorNotSupported) {
+        cudaGetLastError();
+        *ordered = false;
+        e = cudaMalloc((void**)p, bytes);
+    }
+    if (e == cudaSuccess) g_live_allocs.fetch_add(1);
+    else *p = nullptr;
+    return e;
+}
+static cudaError_t lib_free_ordered(void* p, cudaStream_t st, bool ordered) {
+    if (!ordered) return lib_free(p);
+    if (!p) return cudaSuccess;
+    g_live_allocs.fetch_sub(1);
+    return cudaFreeAsync(p, st);
+}
 
 #define CUDA_TRY(call)                                                                     \
     do {                                                                                   \
@@ -1077,15 +1101,15 @@ static int conv_spectrum_rows(cfft_plan_s* P, const std::string& key, int64_t N1
         // stream-ordered: a cudaMalloc / cudaFree pair per length was half of
         // the time to plan a batch of many lengths
         double2* v = nullptr;
-        if (alloc_injected_failure() || cudaMallocAsync((void**)&v, (size_t)M * sizeof(double2), 0) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(CFFT_ERR_NOMEM, "convolution spectrum: temporary buffer");
-        }
-        cudaError_t ce = gen(v);
+        bool ordered;
+        cudaError_t ce = lib_malloc_ordered(&v, (size_t)M * sizeof(double2), 0, &ordered);
+        if (ce != cudaSuccess) cudaGetLastError();
+        CUDA_TRY(ce);
+        ce = gen(v);
         int r = CFFT_OK;
         if (ce == cudaSuccess) r = plan_execute(F, v, v, CFFT_FORWARD, 0);
         if (ce == cudaSuccess && !r) ce = cfft_spec_center((double2*)dp, v, N1, S, 1.0 / (double)M, 0);
-        cudaFreeAsync(v, 0);
+        lib_free_ordered(v, 0, ordered);
         CUDA_TRY(ce);
         return r;
     }, &d);
