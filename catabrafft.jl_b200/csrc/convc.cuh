@@ -41,8 +41,8 @@ __device__ __forceinline__ double2 convc_w(const TwoLevel& t, unsigned e) {
 // the y index of c[c + C (t + 256 k)] or -1, spec = B (natural order, FP64),
 // t4 = two-level table of w_4096, t4n = two-level table of w_M.
 // Shared memory: buf (16 R4096_PL elements), w_4096 table (129 FP64), the
-// CTA's partial sum of x[1:] (FP64), the block reduction scratch (32) and,
-// in CTA 0, the total for y[0].
+// CTA's partial sum of x[1:] (FP64), the block reduction scratch (32), in CTA
+// 0 the total for y[0], and x[0].
 template <typename V, int C>
 __device__ __forceinline__ void convc_rader_body(const KParams& p, unsigned char* smem) {
     cg::cluster_group cl = cg::this_cluster();
@@ -53,7 +53,7 @@ __device__ __forceinline__ void convc_rader_body(const KParams& p, unsigned char
     double2* tlo = after16(buf + 16 * R4096_PL);
     double2* thi = tlo + 64;
     double2* part = thi + 65;                   // this CTA's sum of its x[1:] share
-    double2* red = part + 1;                    // block_sum scratch (32 entries), then y[0]'s sum
+    double2* red = part + 1;                    // block_sum scratch (32 entries), y[0]'s sum, x[0]
     {
         const int t = opaque_tid();
         if (t < 64) tlo[t ^ (t >> 3)] = p.t4.lo[t];
@@ -81,7 +81,12 @@ __device__ __forceinline__ void convc_rader_body(const KParams& p, unsigned char
             acc.y += d.y;
         }
         const double2 s = block_sum(acc, red);  // barriers inside: tables staged too
-        if (t == 0) *part = s;
+        // x[0] is kept here too: in place, a CTA that is ahead overwrites it with
+        // y[0] while others have still to add it
+        if (t == 0) {
+            *part = s;
+            red[33] = tod(load_in(p, x[0]));
+        }
     }
     // 2. F_c, stored in natural order
     fft4096_regs(v, buf, tlo, thi, opaque_tid());
@@ -143,9 +148,8 @@ __device__ __forceinline__ void convc_rader_body(const KParams& p, unsigned char
     fft4096_regs(v, buf, tlo, thi, opaque_tid());
     {
         const int t = opaque_tid();
-        const V* x = (const V*)p.in + (long long)tr * p.in_dist;
         V* y = (V*)p.out + (long long)tr * p.out_dist;
-        const V x0 = load_in(p, x[0]);
+        const V x0 = fromd<V>(red[33]);
         const int* ic = p.iperm + c * 4096 + t;
 #pragma unroll
         for (int k3 = 0; k3 < 16; k3++) {

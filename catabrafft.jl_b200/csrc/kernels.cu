@@ -391,9 +391,9 @@ const void* cfft_convc_kernel(int dtype, int C, int mb) {
     return convc_for<float2, 3>(C);
 }
 size_t cfft_convc_smem(size_t elem_bytes) {
-    // planes, w_4096 table (129), partial sum (1), reduction scratch (32) and
-    // the total for y[0] (1), FP64
-    return ((16 * R4096_PL * elem_bytes + 15) & ~(size_t)15) + (129 + 1 + 33) * sizeof(double2);
+    // planes, w_4096 table (129), partial sum (1), reduction scratch (32), the
+    // total for y[0] (1) and x[0] (1), FP64
+    return ((16 * R4096_PL * elem_bytes + 15) & ~(size_t)15) + (129 + 1 + 34) * sizeof(double2);
 }
 
 // mixed-radix lengths n = C L on a cluster of C register L-point CTAs
