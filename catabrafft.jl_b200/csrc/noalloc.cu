@@ -96,6 +96,65 @@ __global__ void k_noalloc_tables(V* twA, SfPlan A, V* twC, SfPlan Cc, double2* l
         if (i < nhi) hi[i] = omega_dev((long long)i * nlo, M);
     }
 }
+// split of n, tiles and shared memory of its two passes (parameter blocks
+// without pointers, direction or batch)
+struct Split {
+    long long n = 0;
+    size_t e = 0;
+    KParams col, row;
+    size_t smem_col = 0, smem_row = 0;
+};
+// by the planner's rule: factors <= 4096 and 7-smooth, the least cost of the two
+// passes.  Pricing every divisor pair takes up to 0.4 ms of host time (30240:
+// 87 pairs), several times the transform, so the last lengths keep theirs in a
+// fixed table, a slot by length
+bool find_split(long long n, size_t e, Split& sp) {
+    static std::mutex mu;
+    static Split kept[32];
+    Split& slot = kept[(size_t)(n * 2 + (e == 8)) * 2654435761u % 32];
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (slot.n == n && slot.e == e) {
+            sp = slot;
+            return true;
+        }
+    }
+    long long N1 = -1;
+    double best = 1e8;
+    SfPlan pa, pc;
+    for (long long a = 2; a <= 4096; a++) {
+        if (n % a) continue;
+        const long long b = n / a;
+        if (b < 2 || b > 4096) continue;
+        SfPlan ta, tc;
+        if (!sf_plan((int)a, ta) || !sf_plan((int)b, tc)) continue;
+        const double sc = sf_pass_cost(ta, b, e, false) + sf_pass_cost(tc, a, e, true);
+        if (sc < best) { best = sc; N1 = a; pa = ta; pc = tc; }
+    }
+    if (N1 < 0) return false;
+    sp.n = n;
+    sp.e = e;
+    KParams kp;
+    memset(&kp, 0, sizeof kp);
+    kp.conv = CONV_NONE;
+    kp.nx = (int)n;
+    kp.M = (int)n;
+    kp.N1 = (int)N1;
+    kp.N2 = (int)(n / N1);
+    kp.C = 1;
+    kp.sa = pa;
+    kp.sc = pc;
+    sp.col = sp.row = kp;
+    sp.col.mode = MODE_COLPASS;
+    sp.col.pre = PRE_NONE;
+    sp.col.post = POST_TWIDDLE;
+    sf_stage(sp.col, e, &sp.smem_col, true);
+    sp.row.mode = MODE_ROWPASS;
+    sf_stage(sp.row, e, &sp.smem_row, true);
+    std::lock_guard<std::mutex> lk(mu);
+    slot = sp;
+    return true;
+}
 }  // namespace
 
 extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, const void* d_in,
@@ -111,23 +170,11 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
                             "n exceeds the fixed scratch (2^21 ComplexF64 / 2^22 ComplexF32 elements)");
     if (((uintptr_t)d_in % e) || ((uintptr_t)d_out % e))
         return noalloc_fail(CFFT_ERR_INVALID, "buffers must be aligned to the element size");
-    // the planner's split rule (factors <= 4096 and 7-smooth, best score)
-    long long N1 = -1;
-    double best = 1e8;
-    SfPlan pa, pc;
-    for (long long a = 2; a <= 4096; a++) {
-        if (n % a) continue;
-        const long long b = n / a;
-        if (b < 2 || b > 4096) continue;
-        SfPlan ta, tc;
-        if (!sf_plan((int)a, ta) || !sf_plan((int)b, tc)) continue;
-        const double sc = sf_pass_cost(ta, b, e, false) + sf_pass_cost(tc, a, e, true);
-        if (sc < best) { best = sc; N1 = a; pa = ta; pc = tc; }
-    }
-    if (N1 < 0)
+    Split sp;
+    if (!find_split(n, e, sp))
         return noalloc_fail(CFFT_ERR_UNSUPPORTED,
                             "n must be 7-smooth with a split n = N1*N2, N1, N2 <= 4096");
-    const long long N2 = n / N1;
+    const SfPlan &pa = sp.col.sa, &pc = sp.col.sc;
 
     int dev = 0;
     cudaError_t ce = cudaGetDevice(&dev);
@@ -178,32 +225,17 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
     ce = cudaGetLastError();
     if (ce != cudaSuccess) return noalloc_fail(CFFT_ERR_CUDA, "table kernel launch", ce);
 
-    KParams kp;
-    memset(&kp, 0, sizeof kp);
-    kp.conv = CONV_NONE;
-    kp.nx = (int)n;
-    kp.M = (int)n;
-    kp.N1 = (int)N1;
-    kp.N2 = (int)N2;
-    kp.C = 1;
-    kp.dir = direction;
-    kp.scale = (direction == CFFT_INVERSE) ? 1.0 / (double)n : 1.0;
-    kp.t4.lo = lo;
-    kp.t4.hi = hi;
-    kp.t4.bits = bits;
-    kp.t4.N = (int)n;
-    pa.tw = twA;
-    pc.tw = twC;
-    kp.sa = pa;
-    kp.sc = pc;
-    KParams col = kp, row = kp;
-    col.mode = MODE_COLPASS;
-    size_t smem_col = 0, smem_row = 0;
-    sf_stage(col, e, &smem_col, true);
-    col.pre = PRE_NONE;
-    col.post = POST_TWIDDLE;
-    row.mode = MODE_ROWPASS;
-    sf_stage(row, e, &smem_row, true);
+    KParams &col = sp.col, &row = sp.row;
+    for (KParams* kp : {&col, &row}) {
+        kp->dir = direction;
+        kp->scale = (direction == CFFT_INVERSE) ? 1.0 / (double)n : 1.0;
+        kp->t4.lo = lo;
+        kp->t4.hi = hi;
+        kp->t4.bits = bits;
+        kp->t4.N = (int)n;
+        kp->sa.tw = twA;
+        kp->sc.tw = twC;
+    }
 
     const long long chunk = std::max<long long>(1, (long long)(kScratchBytes / ((size_t)n * e)));
     for (long long b0 = 0; b0 < batch; b0 += chunk) {
@@ -217,9 +249,9 @@ extern "C" int cfft_fft_twopass_noalloc(int64_t n, int64_t batch, int dtype, con
         row.out = (char*)d_out + (size_t)b0 * n * e;
         row.in_dist = n;
         row.out_dist = n;
-        ce = cfft_launch_fn(fcol, col, (unsigned)(nb * ((N2 + col.V - 1) / col.V)), CFFT_THREADS, smem_col, 1, st);
+        ce = cfft_launch_fn(fcol, col, (unsigned)(nb * ((col.N2 + col.V - 1) / col.V)), CFFT_THREADS, sp.smem_col, 1, st);
         if (ce == cudaSuccess)
-            ce = cfft_launch_fn(frow, row, (unsigned)(nb * ((N1 + row.V - 1) / row.V)), CFFT_THREADS, smem_row, 1, st);
+            ce = cfft_launch_fn(frow, row, (unsigned)(nb * ((row.N1 + row.V - 1) / row.V)), CFFT_THREADS, sp.smem_row, 1, st);
         if (ce != cudaSuccess) return noalloc_fail(CFFT_ERR_CUDA, "kernel launch", ce);
     }
     return CFFT_OK;
