@@ -301,6 +301,17 @@ inline int sf_lconv_rows(const SfPlan& S, long long batch, size_t e, double* cos
     if (cost) *cost = bc;
     return best;
 }
+// Strided plans whose transforms lie side by side: as columns of tiles (COLS)
+// only from 4.5 MB on, else as LINE's strided rows.  Whole segments save more
+// with size, but a 2D transform that runs its other axis in LINE then runs two
+// large kernels in turn, each finding the instruction caches without it: 2.5 to
+// 4.5 us a pair.  Both axes of a ComplexF32 image on B200, with COLS / with LINE
+// alone: 128 x 128 8.2 / 5.3 us, 256 x 256 11.3 / 6.8, 512 x 512 (2 MB) 11.0 /
+// 9.3, 640 x 640 (3.1) 13.4 / 13.0, 768 x 768 (4.5) 13.5 / 15.2, 1000 x 1000 18.7
+// / 23.0; ComplexF64 512 x 512 (4) 12.2 / 10.5, 640 x 640 (6.3) 15.8 / 16.4
+inline bool sf_cols_pays(long long n, long long count, size_t e) {
+    return (double)n * (double)count * (double)e >= 4.5 * (1 << 20);
+}
 // tile, pitches and shared memory of a pass (mode, N1, N2, sa, sc set)
 // (own: in a launch of its own)
 inline void sf_stage(KParams& k, size_t e, size_t* smem, bool own) {

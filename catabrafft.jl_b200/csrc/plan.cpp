@@ -3097,8 +3097,9 @@ int cfft_plan_create_many(cfft_plan* plan, int64_t n, int64_t batch, int dtype, 
     P->odist = odist;
     // transforms side by side (distance 1, rows at the stride): they are the
     // columns of one COLPASS tile row, so every access is a segment of V
-    // elements (LINE would gather its rows one element per sector)
+    // elements (LINE gathers its rows one element per sector)
     if (idist == 1 && odist == 1 && istride >= batch && ostride >= batch && P->stages.size() == 1 &&
+        sf_cols_pays(n, batch, elem_bytes(dtype)) &&
         P->stages[0].kp.mode == MODE_LINE && P->stages[0].smem_batched == 0 && batch <= 0x7fffffffLL) {
         Stage s = P->stages[0];
         const size_t e = elem_bytes(dtype);
@@ -3112,8 +3113,10 @@ int cfft_plan_create_many(cfft_plan* plan, int64_t n, int64_t batch, int dtype, 
         s.cols = true;
         s.fn = cfft_kernel_for(MODE_COLS, dtype == CFFT_C128 ? CFFT_DT_C128 : CFFT_DT_C64);
         if ((s.kp.V * e >= 32 || s.kp.V == batch) && s.smem <= sf_budget(e) &&
-            cfft_prepare_fn(s.fn, s.smem, 1) == cudaSuccess)
+            cfft_prepare_fn(s.fn, s.smem, 1) == cudaSuccess) {
             P->stages[0] = s;
+            P->desc = "cols(V=" + std::to_string(s.kp.V) + ")+" + P->desc;
+        }
     }
     if (io_fusable(P)) {
         // the first kernel gathers as it loads, the last scatters as it stores

@@ -11,4 +11,5 @@ double probe_mid_cost(const SfPlan* S, long long count, int e) {
     sf_mid_rows(*S, count, (size_t)e, sf_budget((size_t)e), &c);
     return c;
 }
+int probe_cols_pays(long long n, long long count, int e) { return sf_cols_pays(n, count, (size_t)e); }
 }

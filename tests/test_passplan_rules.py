@@ -32,6 +32,7 @@ def rules(tmp_path_factory):
     lib = ctypes.CDLL(str(so))
     lib.probe_mid_cost.restype = ctypes.c_double
     lib.probe_mid_cost.argtypes = [ctypes.POINTER(SfPlan), ctypes.c_longlong, ctypes.c_int]
+    lib.probe_cols_pays.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
     assert lib.probe_plan_bytes() == ctypes.sizeof(SfPlan)
     return lib
 
@@ -56,3 +57,11 @@ def test_convolution_rows_end_in_a_radix(rules):
         else:
             assert max(costs) < 1e9, (L, costs)
     assert single == 13          # 2 .. 10, 12, 14, 15 and 16
+
+
+def test_small_images_stay_on_one_kernel(rules):
+    # both axes of a small image in LINE: a second kernel for the columns costs
+    # more than its whole segments save
+    for n, m, e, cols in ((64, 64, 8, 0), (256, 256, 8, 0), (256, 256, 16, 0), (512, 512, 8, 0), (2000, 256, 8, 0),
+                          (768, 768, 8, 1), (640, 640, 16, 1), (1000, 1000, 8, 1), (2160, 3840, 8, 1), (4096, 4096, 16, 1)):
+        assert rules.probe_cols_pays(n, m, e) == cols, (n, m, e)
