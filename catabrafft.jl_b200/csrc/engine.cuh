@@ -332,9 +332,9 @@ __device__ __forceinline__ double2 r4096_w(const double2* lo, const double2* hi,
 // f(k, b^k) for k = 1 .. R - 1 in order: FP64 products in two chains (even and
 // odd k, both stepping by b^2), so that half as many wait for one another, for
 // one more product and eight registers.  Against one chain, B200: 4096 x 16384
-// ComplexF64 385 -> 370 us, 8192 x 4096 294 -> 282, 16384 x 2048 363 -> 358; in
-// the row pass and the column DFTs of pow2.cuh and in mixc.cuh one chain stayed
-// 1 - 3 % faster.
+// ComplexF64 385 -> 370 us, 8192 x 4096 294 -> 282; in the row pass and the column
+// DFTs of pow2.cuh and in mixc.cuh one chain stayed 1 - 3 % faster, and so it did
+// where those registers cost a CTA per SM (p2cl_body).
 template <int R, class F> __device__ __forceinline__ void fp64_powers(double2 b, F f) {
     double2 odd = b;
     f(1, odd);
@@ -361,12 +361,14 @@ template <int R, class F> __device__ __forceinline__ void fp64_powers(double2 b,
 template <typename V, bool TWO>
 __device__ __forceinline__ void r4096_tw_store(V (&v)[16], V* dst, int stride, const double2* lo,
                                                const double2* hi, unsigned e0) {
-    dst[0] = v[0];
-    const double2 b = r4096_w(lo, hi, e0);
     if constexpr (TWO) {
+        dst[0] = v[0];
+        const double2 b = r4096_w(lo, hi, e0);
         fp64_powers<16>(b, [&](int k, double2 w) { dst[k * stride] = cmul(v[k], fromd<V>(w)); });
     } else {
+        const double2 b = r4096_w(lo, hi, e0);
         double2 w = b;
+        dst[0] = v[0];
 #pragma unroll
         for (int k = 1; k < 16; k++) {
             dst[k * stride] = cmul(v[k], fromd<V>(w));

@@ -389,7 +389,12 @@ __device__ __forceinline__ void p2cl_body(const KParams& p, unsigned char* smem,
         for (int k = 0; k < 16; k++) v[k] = load_in(p, __ldg(x + (long long)C * 256 * k));
         __syncthreads();                        // tables staged
     }
-    fft4096_regs(v, buf, tlo, thi, opaque_tid());
+    // two chains of powers (fp64_powers) for ComplexF64 8192 only.  In ComplexF32
+    // they take 96 registers instead of 80, so two CTAs per SM instead of three
+    // (8192 x 2048 107 us, one chain 86; 16384 x 2048 216 / 186); in ComplexF64 16384
+    // x 40 is slower with them (13.1 / 12.7) and x 2048 faster (344 / 353)
+    constexpr bool TWO = sizeof(V) == 16 && C == 2;
+    fft4096_regs<V, TWO>(v, buf, tlo, thi, opaque_tid());
     {
         const int t = opaque_tid();
 #pragma unroll
@@ -407,7 +412,16 @@ __device__ __forceinline__ void p2cl_body(const KParams& p, unsigned char* smem,
             for (int q = 0; q < C; q++) f[q] = cl.map_shared_rank(buf, q)[k];
             // w_n^(q k) as FP64 powers of one table value, rounded once
             const double2 wk = cmul(__ldg(p.t4n.lo + (k & mask)), __ldg(p.t4n.hi + (k >> p.t4n.bits)));
-            fp64_powers<C>(wk, [&](int q, double2 w) { f[q] = cmul(f[q], fromd<V>(w)); });
+            if constexpr (TWO) {
+                fp64_powers<C>(wk, [&](int q, double2 w) { f[q] = cmul(f[q], fromd<V>(w)); });
+            } else {
+                double2 w = wk;
+#pragma unroll
+                for (int q = 1; q < C; q++) {
+                    f[q] = cmul(f[q], fromd<V>(w));
+                    if (q + 1 < C) w = cmul(w, wk);
+                }
+            }
             dft<C>(f);
 #pragma unroll
             for (int q = 0; q < C; q++) stg_stream(out + k + 4096 * q, store_out(p, f[q]));
