@@ -8,6 +8,7 @@
 #include "engine_types.h"
 
 static const int SF_THREADS = 256;    // CTA size of the pass kernels
+static const int SF_SMS = 148;        // a B200's SMs, the only device this is built for
 
 // Radix sequence of L (7-smooth, L >= 2): the fewest stages first (a stage is
 // a shared-memory round trip and a barrier), then the least arithmetic, in
@@ -172,8 +173,20 @@ inline double sf_crowd(size_t smem, size_t e) {
     const double total = (double)smem * (e == 8 ? 3 : 2) / 1024.0;
     return total > 130.0 ? 1.0 + 0.12 * (total - 130.0) / 68.0 : 1.0;
 }
+// A pass of nb transforms (0: many) of `tiles` tiles each costs its tiles, or as
+// much as 200 (ComplexF64: 148) of them: fewer leave SMs idle, and then narrower
+// tiles, each with fewer rounds, are faster however many they are.  ComplexF32 on
+// B200, without this bound / with 148 / 200 / 296: 117649 x 1 22.4 / 10.4 / 10.3 /
+// 10.4 us (15.4 before the stage kernels), 100000 x 8 17.0 / 15.3 / 13.8 / 13.8;
+// ComplexF64 59049 x 4 17.3 / 13.7 / 13.3 / 13.2, 177147 x 4 23.1 / 23.2 / 25.1 /
+// 27.0, 40009 x 1 27.0 / 19.1 / 19.3 / 19.2
+inline double sf_launch(long long tiles, long long nb, size_t e) {
+    const double least = e == 8 ? 200.0 : SF_SMS;
+    return nb > 0 && (double)(tiles * nb) < least ? least / (double)nb : (double)tiles;
+}
 // cycles per useful element of a COLPASS / ROWPASS tile of width V
-inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bool row, size_t budget) {
+inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bool row, size_t budget,
+                           long long nb = 0) {
     const size_t smem = row ? sf_row_smem(S, V, e, false) : sf_col_smem(S, V, e);
     if (smem > budget) return 1e9 + (double)smem;
     const int ks = SF_THREADS / V;
@@ -190,14 +203,15 @@ inline double sf_tile_cost(const SfPlan& S, int V, long long count, size_t e, bo
     const double sectors = (double)((seg + 31) / 32 + (whole ? 0 : 1)) * 32.0 / (double)seg;
     c *= 1.0 + 0.25 * (sectors - 1.0) + (seg < 64 ? 0.3 : seg < 128 ? 0.1 : 0.0);
     const long long tiles = (count + V - 1) / V;
-    return c / ((double)V * S.L) * (double)(tiles * V) / (double)count;
+    return c / (double)S.L * sf_launch(tiles, nb, e) / (double)count;
 }
 // the width with the least cost (at most 64)
-inline int sf_tile(const SfPlan& S, long long count, size_t e, bool row, size_t budget, double* cost = nullptr) {
+inline int sf_tile(const SfPlan& S, long long count, size_t e, bool row, size_t budget, double* cost = nullptr,
+                   long long nb = 0) {
     int best = 1;
     double bc = 1e300;
     for (int V = 1; V <= 64 && V <= count; V++) {
-        const double c = sf_tile_cost(S, V, count, e, row, budget);
+        const double c = sf_tile_cost(S, V, count, e, row, budget, nb);
         if (c < bc) {
             bc = c;
             best = V;
@@ -217,7 +231,7 @@ inline double sf_pass_cost(const SfPlan& S, long long count, size_t e, bool row)
 inline bool sf_mid_fits(const SfPlan& S) { return S.r[S.np - 1] >= 2; }
 // MIDPASS: whole rows, contiguous on both sides, the second transform's first
 // stage fused with the first one's last
-inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e, size_t budget) {
+inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e, size_t budget, long long nb = 0) {
     if (!sf_mid_fits(S)) return 1e300;
     const size_t smem = sf_row_smem(S, V, e, true);
     if (smem > budget) return 1e9 + (double)smem;
@@ -227,13 +241,14 @@ inline double sf_mid_tile_cost(const SfPlan& S, int V, long long count, size_t e
         c += rounds * (s == S.np - 1 ? sf_round(S.r[s], 2) : 2.0 * sf_round(S.r[s], 1));
     }
     const long long tiles = (count + V - 1) / V;
-    return c / ((double)V * S.L) * (double)(tiles * V) / (double)count;
+    return c / (double)S.L * sf_launch(tiles, nb, e) / (double)count;
 }
-inline int sf_mid_rows(const SfPlan& S, long long count, size_t e, size_t budget, double* cost = nullptr) {
+inline int sf_mid_rows(const SfPlan& S, long long count, size_t e, size_t budget, double* cost = nullptr,
+                       long long nb = 0) {
     int best = 1;
     double bc = 1e300;
     for (int V = 1; V <= 32 && V <= count; V++) {
-        const double c = sf_mid_tile_cost(S, V, count, e, budget);
+        const double c = sf_mid_tile_cost(S, V, count, e, budget, nb);
         if (c < bc) {
             bc = c;
             best = V;
@@ -257,7 +272,7 @@ inline size_t sf_line_smem(const SfPlan& S, int V, size_t e) { return (size_t)sf
 // transforms per CTA: the model's cost of the whole batch, waves of CTAs on
 // 148 SMs x (three ComplexF32 or two ComplexF64)
 inline int sf_line_rows(const SfPlan& S, long long batch, size_t e) {
-    const long long slots = 148 * (e == 8 ? 3 : 2);
+    const long long slots = SF_SMS * (e == 8 ? 3 : 2);
     int best = 1;
     double bc = 1e300;
     for (int V = 1; V <= 1024 && V <= batch; V++) {
@@ -280,7 +295,7 @@ inline size_t sf_lconv_smem(const SfPlan& S, int V, size_t e) {
     return ((size_t)sf_qw(S, V, e, true) * V * e + 15) / 16 * 16 + (size_t)V * 32;
 }
 inline int sf_lconv_rows(const SfPlan& S, long long batch, size_t e, double* cost = nullptr) {
-    const long long slots = 148 * (e == 8 ? 3 : 2);
+    const long long slots = SF_SMS * (e == 8 ? 3 : 2);
     int best = 1;
     double bc = 1e300;
     for (int V = 1; V <= 256 && V <= batch; V++) {
@@ -313,13 +328,13 @@ inline bool sf_cols_pays(long long n, long long count, size_t e) {
     return (double)n * (double)count * (double)e >= 4.5 * (1 << 20);
 }
 // tile, pitches and shared memory of a pass (mode, N1, N2, sa, sc set)
-// (own: in a launch of its own)
-inline void sf_stage(KParams& k, size_t e, size_t* smem, bool own) {
+// (own: in a launch of its own, of nb transforms; 0: many)
+inline void sf_stage(KParams& k, size_t e, size_t* smem, bool own, long long nb = 0) {
     const size_t budget = own ? sf_pass_budget(e) : sf_budget(e);
     const bool mid = k.mode == MODE_MIDPASS;
-    if (k.mode == MODE_COLPASS) k.V = sf_tile(k.sa, k.N2, e, false, budget);
-    else if (mid) k.V = sf_mid_rows(k.sc, k.N1, e, budget);
-    else k.V = sf_tile(k.sc, k.N1, e, true, budget);
+    if (k.mode == MODE_COLPASS) k.V = sf_tile(k.sa, k.N2, e, false, budget, nullptr, nb);
+    else if (mid) k.V = sf_mid_rows(k.sc, k.N1, e, budget, nullptr, nb);
+    else k.V = sf_tile(k.sc, k.N1, e, true, budget, nullptr, nb);
     k.mv = sf_magic(k.V);
     k.ks = SF_THREADS / k.V;
     k.qp = sf_qp(k.sc, k.V, e, mid);

@@ -1717,7 +1717,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         s.kp.mode = mode;
         s.kp.pre = pre;
         s.kp.post = post;
-        sf_stage(s.kp, e, &s.smem, !P->shared_scratch);
+        sf_stage(s.kp, e, &s.smem, !P->shared_scratch, P->shared_scratch ? 0 : chunk);
         s.threads = CFFT_THREADS;
         s.cluster = 1;
         s.in_sel = in_sel;

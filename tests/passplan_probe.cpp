@@ -12,4 +12,7 @@ double probe_mid_cost(const SfPlan* S, long long count, int e) {
     return c;
 }
 int probe_cols_pays(long long n, long long count, int e) { return sf_cols_pays(n, count, (size_t)e); }
+int probe_tile(const SfPlan* S, long long count, int e, int row, long long nb) {
+    return sf_tile(*S, count, (size_t)e, row != 0, sf_pass_budget((size_t)e), nullptr, nb);
+}
 }

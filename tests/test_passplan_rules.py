@@ -33,6 +33,7 @@ def rules(tmp_path_factory):
     lib.probe_mid_cost.restype = ctypes.c_double
     lib.probe_mid_cost.argtypes = [ctypes.POINTER(SfPlan), ctypes.c_longlong, ctypes.c_int]
     lib.probe_cols_pays.argtypes = [ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int]
+    lib.probe_tile.argtypes = [ctypes.POINTER(SfPlan), ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_longlong]
     assert lib.probe_plan_bytes() == ctypes.sizeof(SfPlan)
     return lib
 
@@ -65,3 +66,19 @@ def test_small_images_stay_on_one_kernel(rules):
     for n, m, e, cols in ((64, 64, 8, 0), (256, 256, 8, 0), (256, 256, 16, 0), (512, 512, 8, 0), (2000, 256, 8, 0),
                           (768, 768, 8, 1), (640, 640, 16, 1), (1000, 1000, 8, 1), (2160, 3840, 8, 1), (4096, 4096, 16, 1)):
         assert rules.probe_cols_pays(n, m, e) == cols, (n, m, e)
+
+
+@pytest.mark.parametrize("e", [8, 16])
+def test_a_few_transforms_get_many_tiles(rules, e):
+    # a pass over few transforms must not leave SMs idle for wide tiles of several
+    # rounds: 343 rows made 22 tiles or fewer
+    for L, count, nb in ((343, 343, 1), (625, 625, 1), (81, 729, 1), (81, 729, 2), (160, 225, 1), (400, 500, 1)):
+        S = plan(rules, L)
+        for row in (0, 1):
+            few = rules.probe_tile(ctypes.byref(S), count, e, row, nb)
+            many = rules.probe_tile(ctypes.byref(S), count, e, row, 0)
+            assert 1 <= few <= many
+            rounds = max(-(-(L // r) // (256 // few)) for r in list(S.r)[:S.np])
+            assert -(-count // few) * nb >= 40 or rounds == 1, (L, count, nb, row, few, many)
+            # enough transforms: the width for many
+            assert rules.probe_tile(ctypes.byref(S), count, e, row, 1000) == many
