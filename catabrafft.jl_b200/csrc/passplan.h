@@ -341,23 +341,41 @@ inline void sf_stage(KParams& k, size_t e, size_t* smem, bool own, long long nb 
     k.qw = sf_qw(k.sc, k.V, e, mid);
     *smem = k.mode == MODE_COLPASS ? sf_col_smem(k.sa, k.V, e) : sf_row_smem(k.sc, k.V, e, mid);
 }
-// CLUS: shared memory and cost per element of an N1 x N2 split on C CTAs
+// CLUS: shared memory of an N1 x N2 split on C CTAs
 inline size_t sf_clus_smem(const SfPlan& a, const SfPlan& c, int C, size_t e) {
     return ((size_t)a.L * (c.L / C) + (size_t)(a.L / C) * sf_qw(c, a.L / C, e, false)) * e;
 }
-inline double sf_clus_cost(const SfPlan& a, const SfPlan& c, int C, size_t e, int threads) {
-    const int W = c.L / C, R1 = a.L / C;
-    if (W > threads || R1 > threads) return 1e9;
-    const int kc = threads / W, kr = threads / R1;
+// cycles of a CTA of CLUS, with its segments' sectors and its barriers
+inline double sf_clus_cycles(const SfPlan& a, const SfPlan& c, int C, size_t e, int threads) {
+    const int W = c.L / C, R1 = a.L / C, kc = threads / W, kr = threads / R1;
     double t = sf_start() + 2000.0;
     for (int s = 0; s < a.np; s++) t += sf_round(a.r[s], 1) * ((a.L / a.r[s] + kc - 1) / kc);
     for (int s = 0; s < c.np; s++) {
         const int nb = c.L / c.r[s];
         t += sf_round(c.r[s], 1) * (s == c.np - 1 ? (nb + kr - 1) / kr : (R1 * nb + threads - 1) / threads);
     }
-    if (sf_clus_smem(a, c, C, e) > 112 * 1024) t *= 1.6;
     for (long long seg : {W * (long long)e, R1 * (long long)e})
         t *= seg < 32 ? 1.6 : seg < 64 ? 1.2 : seg < 128 ? 1.05 : 1.0;
     if (W < 32) t *= 1.2;          // the exchange writes runs of W elements
-    return t * (1.0 + 0.02 * C + (C > 8 ? 0.3 : 0.0)) / ((double)a.L * W);
+    return t * (1.0 + 0.02 * C + (C > 8 ? 0.3 : 0.0));
+}
+// ... per element, of many transforms
+inline double sf_clus_cost(const SfPlan& a, const SfPlan& c, int C, size_t e, int threads) {
+    if (c.L / C > threads || a.L / C > threads) return 1e9;
+    const double t = sf_clus_cycles(a, c, C, e, threads);
+    return (sf_clus_smem(a, c, C, e) > 112 * 1024 ? 1.6 * t : t) / ((double)a.L * (c.L / C));
+}
+// Time of `batch` transforms in cycles.  Up to 148 CTAs take a CTA's own time
+// however few they are, so that a few transforms take as many CTAs as shorten
+// them; more share SMs (at least 1.35 times as long, 2.1 times at 296, two to an
+// SM) and then run in waves.  By cost per element 8 x 19683 ComplexF64 took
+// clusters of 3 (18.4 us; 10.3 on clusters of 9, 14.7 before the stage kernels).
+// Above 148 CTAs fewer are as good: 40 x 9000 10.7 us on clusters of 3, 11.7 on 5;
+// 40 x 9604 12.6 on 2, 17.2 on 7; 40 x 10000 11.7 on 4, 12.3 on 2
+inline double sf_clus_time(const SfPlan& a, const SfPlan& c, int C, size_t e, int threads, long long batch) {
+    const double t = sf_clus_cycles(a, c, C, e, threads);
+    if (batch * C <= SF_SMS) return t;
+    const bool one = sf_clus_smem(a, c, C, e) > 112 * 1024;
+    const double w = (double)batch * C / (one ? 148.0 : 296.0);
+    return t * std::max(1.35, (one ? 1.68 : 2.1) * (w < 1.0 ? w : w < 4.0 ? std::ceil(w) : w + 0.5));
 }

@@ -470,9 +470,9 @@ static size_t four_smem_bytes(int64_t M, int64_t twA, int64_t twC, int64_t bufsz
     return b;
 }
 
-// CLUS shapes of a smooth length, best first
+// CLUS shapes of a smooth length for `batch` transforms (0: many), best first
 static int clus_threads(int dtype) { return dtype == CFFT_C128 ? CFFT_CLUS64 : CFFT_CLUS32; }
-static void clus_candidates(int64_t M, int dtype, std::vector<Shape>& out) {
+static void clus_candidates(int64_t M, int dtype, int64_t batch, std::vector<Shape>& out) {
     const size_t e = elem_bytes(dtype);
     std::vector<Shape> v;
     for (int64_t N1 = 4; N1 <= kSfMax; N1++) {
@@ -498,13 +498,17 @@ static void clus_candidates(int64_t M, int dtype, std::vector<Shape>& out) {
         }
     }
     std::sort(v.begin(), v.end(), [](const Shape& a, const Shape& b) { return a.score < b.score; });
+    if (batch > 0) {
+        for (Shape& sh : v) sh.score = sf_clus_time(*sf_get(sh.N1), *sf_get(sh.N2), sh.C, e, clus_threads(dtype), batch);
+        std::stable_sort(v.begin(), v.end(), [](const Shape& a, const Shape& b) { return a.score < b.score; });
+    }
     if (v.size() > 8) v.resize(8);
     out.insert(out.end(), v.begin(), v.end());
 }
 
-static void four_candidates(int64_t M, int64_t nx, int conv, int dtype, std::vector<Shape>& out) {
+static void four_candidates(int64_t M, int64_t nx, int conv, int dtype, int64_t batch, std::vector<Shape>& out) {
     size_t e = elem_bytes(dtype);
-    if (conv == CONV_NONE) return clus_candidates(M, dtype, out);
+    if (conv == CONV_NONE) return clus_candidates(M, dtype, batch, out);
     for (int64_t N1 = 2; N1 <= 4096; N1++) {
         if (M % N1) continue;
         int64_t N2 = M / N1;
@@ -794,7 +798,8 @@ static bool twopass_shape(int64_t n, int conv, int64_t M, int dtype, Shape& g) {
     return true;
 }
 
-static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch) {
+// (shared: a plan of one transform among many others in flight)
+static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch, bool shared = false) {
     std::vector<Shape> v;
     int conv;
     int64_t M;
@@ -804,25 +809,34 @@ static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch) 
         sh.conv = conv;
         v.push_back(sh);
     }
-    if (M > 64) four_candidates(M, n, conv, dtype, v);
+    // (a few ComplexF32 transforms take the clusters of many: never slower than
+    // before the stage kernels, as a few ComplexF64 ones were)
+    if (M > 64) four_candidates(M, n, conv, dtype, shared || dtype == CFFT_C64 ? 0 : batch, v);
     Shape g;
     if ((v.empty() || M >= 16384 || (conv != CONV_NONE && M >= 8192)) && twopass_shape(n, conv, M, dtype, g)) {
         // beyond a cluster, or in place of one.  Measured on B200: a batch of
         // 32 MB or more of smooth transforms runs faster as two passes than
         // on clusters (ComplexF64 60480 x 256 317 against 530 us, 24000 x 512
-        // 200 / 253; ComplexF32 48000 x 256 134 / 153, 24000 x 1024 211 / 222),
-        // a few of them faster on clusters, one launch and no intermediate
-        // (60480 x 1 17 / 26, 24000 x 32 ComplexF32 15 / 20; 64 x 19683 21 /
-        // 24); from 2^15 points ComplexF32 clusters no longer win either way.
-        // Otherwise second in line, so that MEASURE / ENCHANT time both
+        // 200 / 253; ComplexF32 48000 x 256 134 / 153, 24000 x 1024 211 / 222);
+        // a few stay on a cluster, one launch (ComplexF64 19683 x 8 10.9 us, two
+        // passes 12.4); from 2^15 points ComplexF32 clusters no longer win either
+        // way.  Otherwise second in line, so that MEASURE / ENCHANT time both
         const bool pow2 = (M & (M - 1)) == 0;
         const bool big = (double)batch * (double)M * (double)elem_bytes(dtype) >= 2.0 * (1 << 20);
+        // ComplexF64 clusters of large CTAs (one to an SM) from 24000 points: of
+        // fewer than ten they are slower than two passes (48000 x 1 17.6 / 10.7
+        // us, 59049 x 1 18.7 / 12.4, 30000 x 16 16.8 / 14.5, x 24 17.0 / 17.6), of
+        // ten or more they run one to a GPC, so that eight take two waves (77760 x
+        // 8 36.0 / 17.3).  Up to seven of those stay clusters, although the
+        // passes have overtaken them too (60480 x 1 16.6 / 11.0)
+        const bool large = conv == CONV_NONE && dtype == CFFT_C128 && M >= 24000 && !v.empty() &&
+                           v[0].mode == MODE_FOUR && v[0].smem > 112 * 1024 && (v[0].C < 10 || batch > 7);
         // convolutions (C64 20011 x 64 60 against 128 us on a cluster, C128
         // 20002 x 64 86 / 109, 10006 x 1 36 / 30); a ComplexF64 prime keeps
         // Rader's algorithm, whose twiddles follow the reference, while a
         // cluster holds it
         const bool cfirst = (conv == CONV_BLUE || (conv == CONV_RADER && dtype == CFFT_C64)) && (M >= 32768 || big);
-        const bool first = cfirst ||
+        const bool first = cfirst || large ||
                            (conv == CONV_NONE && (((dtype == CFFT_C64 || pow2) && M >= 32768) ||
                                                  (double)batch * (double)M * (double)elem_bytes(dtype) >= 32.0 * (1 << 20)));
         v.insert(v.begin() + (first ? 0 : std::min<size_t>(v.size(), 1)), g);
@@ -2126,7 +2140,7 @@ static void batch_free(cfft_batch_s* B) {
 // and serving forms)
 static int build_shared_plan(int64_t n, int dtype, int flags, int device, cfft_plan_s** out) {
     if (n > (1LL << 26)) return fail(CFFT_ERR_UNSUPPORTED, "length above 2^26");
-    auto cands = candidate_shapes(n, dtype, 1);
+    auto cands = candidate_shapes(n, dtype, 1, true);
     cfft_plan_s* P = new cfft_plan_s();
     P->n = n;
     P->batch = 1;

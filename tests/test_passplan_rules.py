@@ -7,7 +7,7 @@ import subprocess
 
 import pytest
 
-from _pkg import PKG_DIR
+from _pkg import PKG_DIR, load
 
 MAXS = 6
 
@@ -82,3 +82,11 @@ def test_a_few_transforms_get_many_tiles(rules, e):
             assert -(-count // few) * nb >= 40 or rounds == 1, (L, count, nb, row, few, many)
             # enough transforms: the width for many
             assert rules.probe_tile(ctypes.byref(S), count, e, row, 1000) == many
+
+
+@pytest.mark.parametrize("n,expect", [(19683, "four(C=9,"), (24000, "four(C=10,"), (59049, "twopass("), (48000, "twopass("),
+                                      (77760, "four(C=1")])
+def test_one_long_transform(n, expect):
+    # one ComplexF64 transform: as many CTAs as shorten it, or two passes where
+    # clusters of few large CTAs are slower
+    assert expect in load().describe_strategy(n), load().describe_strategy(n)
