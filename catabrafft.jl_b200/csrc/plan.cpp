@@ -812,6 +812,21 @@ static std::vector<Shape> candidate_shapes(int64_t n, int dtype, int64_t batch, 
     // (a few ComplexF32 transforms take the clusters of many: never slower than
     // before the stage kernels, as a few ComplexF64 ones were)
     if (M > 64) four_candidates(M, n, conv, dtype, shared || dtype == CFFT_C64 ? 0 : batch, v);
+    // a few long Rader convolutions run shorter on clusters of three CTAs or more
+    // than on one CTA each, while the clusters fit the device at once.  ComplexF64,
+    // LCONV against clusters on B200: 2707 x 1 37.1 / 27.9 us, x 64 37.6 / 31.1, x 90
+    // (360 CTAs) 37.6 / 60.5; 3301 x 90 (270) 42.4 / 37.2, x 128 43.3 / 73.3.  On
+    // clusters of two only with few stages: 2557 x 40 33.1 / 30.7, x 100 33.2 / 32.2;
+    // 2657 x 40 35.3 / 33.8, x 100 35.4 / 37.4; but 2503 x 1 32.2 / 33.6, 2411 x 1
+    // 32.8 / 41.0
+    if (conv == CONV_RADER && dtype == CFFT_C128 && !shared && v.size() > 1 && v[0].mode == MODE_ROWS &&
+        v[1].mode == MODE_FOUR) {
+        const size_t stages = v[1].ra.size() + v[1].rc.size() + (v[0].M == v[1].M ? 1 : 0);
+        // (of equal splits the one with shorter columns: 2801 x 1 27.3 us, 27.8)
+        for (size_t i = 2; i < v.size() && v[i].mode == MODE_FOUR && v[i].score == v[1].score; i++)
+            if (v[i].C == v[1].C && v[i].N1 < v[1].N1) std::swap(v[1], v[i]);
+        if (v[1].C >= 3 ? batch * v[1].C <= 280 : v[1].C == 2 && stages <= 5 && batch * 2 <= 148) std::swap(v[0], v[1]);
+    }
     Shape g;
     if ((v.empty() || M >= 16384 || (conv != CONV_NONE && M >= 8192)) && twopass_shape(n, conv, M, dtype, g)) {
         // beyond a cluster, or in place of one.  Measured on B200: a batch of

@@ -90,3 +90,10 @@ def test_one_long_transform(n, expect):
     # one ComplexF64 transform: as many CTAs as shorten it, or two passes where
     # clusters of few large CTAs are slower
     assert expect in load().describe_strategy(n), load().describe_strategy(n)
+
+
+@pytest.mark.parametrize("n,expect", [(2801, "four(C=4,N1=56,"), (3109, "four(C=5,"), (3301, "four(C=3,"), (2557, "four(C=2,"),
+                                      (2503, "rows(V=1)"), (2411, "rows(V=1)"), (1511, "rows(V=1)")])
+def test_one_long_prime(n, expect):
+    # one ComplexF64 prime: on a cluster where that is shorter than one CTA
+    assert expect in load().describe_strategy(n), load().describe_strategy(n)
