@@ -338,6 +338,7 @@ struct cfft_plan_s {
     int64_t chunk = 0;       // transforms per stage sequence (GLOBAL)
     void* scratch[2] = {nullptr, nullptr};
     size_t scratch_bytes = 0;
+    int64_t scratch_extra = 0;   // of them counted in g_pass_extra
     std::vector<void*> allocs;
     std::vector<DevPtr> tables;  // shared, cached tables
     bool shared_scratch = false; // scratch provided by a batch (not allocated here)
@@ -1232,6 +1233,26 @@ static int64_t pass_chunk(int64_t batch, int64_t one) {
     return std::max<int64_t>(1, (batch + n - 1) / n);
 }
 
+// Plans are cached by shape, so what their passes hold beyond 64 MB (or one
+// transform) is bounded for all live plans together: once 2 GB are out, further
+// plans take chunks of 64 MB
+static const int64_t kPassBase = (int64_t)64 << 20, kPassExtra = (int64_t)2 << 30;
+static std::atomic<int64_t> g_pass_extra{0};
+static void pass_extra_release(cfft_plan_s* P) {
+    g_pass_extra.fetch_sub(P->scratch_extra);
+    P->scratch_extra = 0;
+}
+// counts a chunk's extra bytes; false (nothing counted) beyond the bound
+static bool pass_extra_take(cfft_plan_s* P, int64_t chunk, int64_t one) {
+    const int64_t extra = std::max<int64_t>(0, chunk * one - std::max(kPassBase, one));
+    if (g_pass_extra.fetch_add(extra) + extra > kPassExtra && extra > 0) {
+        g_pass_extra.fetch_sub(extra);
+        return false;
+    }
+    P->scratch_extra = extra;
+    return true;
+}
+
 static int plan_build(cfft_plan_s* P, const Shape& sh) {
     P->shape = sh;
     P->stages.clear();
@@ -1725,15 +1746,21 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     if (rc) return rc;
     kp.N1 = (int)N1;
     kp.N2 = (int)N2;
-    int64_t chunk = pass_chunk(P->batch, M * (int64_t)e);
+    const int64_t one = M * (int64_t)e;
+    int64_t chunk = pass_chunk(P->batch, one);
     if (!P->shared_scratch) {
+        if (!getenv("CFFT_SCRATCH_MB") && !pass_extra_take(P, chunk, one)) chunk = std::max<int64_t>(1, kPassBase / one);
         // where the device cannot hold that scratch, smaller chunks down to 64 MB
         cudaError_t ce;
         for (;;) {
-            ce = lib_malloc(&P->scratch[0], (size_t)chunk * M * e);
-            if (ce != cudaErrorMemoryAllocation || chunk * M * (int64_t)e <= ((int64_t)64 << 20) || chunk == 1) break;
+            ce = lib_malloc(&P->scratch[0], (size_t)(chunk * one));
+            if (ce != cudaErrorMemoryAllocation || chunk * one <= kPassBase || chunk == 1) break;
             cudaGetLastError();
             chunk = (chunk + 1) / 2;
+        }
+        if (P->scratch_extra) {                 // what is held in the end
+            pass_extra_release(P);
+            pass_extra_take(P, chunk, one);
         }
         CUDA_TRY(ce);
         P->allocs.push_back(P->scratch[0]);
@@ -1795,6 +1822,7 @@ static void plan_free(cfft_plan_s* P) {
     P->stages.clear();
     P->scratch[0] = P->scratch[1] = nullptr;
     P->flow_ctr = nullptr;
+    pass_extra_release(P);
 }
 
 // in_dist / out_dist: elements between consecutive transforms of the caller's
