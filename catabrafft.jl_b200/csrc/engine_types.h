@@ -55,6 +55,15 @@ struct TwoLevel {                 // w_N^e = lo[e & mask] * hi[e >> bits]  (FP64
     int N;
 };
 
+// w^e of the real transforms' sweeps in FP64, rounded once but for its last
+// step: hi (1 + lo1), hi's rounding error kept in hr and lo1 = w^l - 1 small
+struct RootTable {
+    const double2* lo1;           // w^l - 1, l < 2^bits
+    const double2* hi;            // w^(h 2^bits)
+    const double2* hr;            // ... minus its rounded value
+    int bits;
+};
+
 enum { MODE_ROWS = 0, MODE_FOUR = 1, MODE_COLPASS = 2, MODE_ROWPASS = 3, MODE_P2COL = 4, MODE_P2ROW = 5,
        MODE_CONVC = 6, MODE_MIXC = 7, MODE_P2CL = 8, MODE_MIDPASS = 9, MODE_LINE = 10,
        MODE_CLUS = 11, MODE_LCONV = 12 };

@@ -109,10 +109,10 @@ cudaError_t cfft_spec_rowmajor(double2* dst, const double2* src, long long N1, l
 cudaError_t cfft_spec_center(double2* dst, const double2* src, long long N1, const SfPlan& S, double scale,
                              cudaStream_t st);
 // real-input transforms (real.cu)
-// (w: the two-level FP64 table of w_2N)
-cudaError_t cfft_r2c_post(void* out, long long N, const TwoLevel& w, long long batch, long long dist, int dtype,
+// (w: the table of w_2N)
+cudaError_t cfft_r2c_post(void* out, long long N, const RootTable& w, long long batch, long long dist, int dtype,
                           cudaStream_t st);
-cudaError_t cfft_c2r_pre(const void* in, void* z, long long N, const TwoLevel& w, long long batch,
+cudaError_t cfft_c2r_pre(const void* in, void* z, long long N, const RootTable& w, long long batch,
                          long long in_dist, double scale, int dtype, cudaStream_t st);
 cudaError_t cfft_r2c_widen(const void* x, void* s, long long n, long long batch, int dtype, cudaStream_t st);
 cudaError_t cfft_r2c_keep(const void* s, void* out, long long n, long long batch, int dtype, cudaStream_t st);

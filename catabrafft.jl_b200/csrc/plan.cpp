@@ -216,7 +216,7 @@ static int wave_G(const std::vector<int>& rad, int64_t L, int T) {
 
 // ------------------------------------------------------------- FP64 tables
 // exp(sign * 2 pi i m / N) with exact integer reduction, long double kernel
-static double2 omega(int64_t m, int64_t N, int sign) {
+static void omega_l(int64_t m, int64_t N, int sign, long double* re, long double* im) {
     m %= N;
     if (m < 0) m += N;
     // quadrant: theta = (pi/2) (q + r/N)
@@ -241,7 +241,13 @@ static double2 omega(int64_t m, int64_t N, int sign) {
         case 2: cc = -c; ss = -s; break;
         default: cc = s; ss = -c; break;
     }
-    return make_double2((double)cc, (double)(sign * ss));
+    *re = cc;
+    *im = sign * ss;
+}
+static double2 omega(int64_t m, int64_t N, int sign) {
+    long double c, s;
+    omega_l(m, N, sign, &c, &s);
+    return make_double2((double)c, (double)s);
 }
 // Julia's robust complex inverse (Smith's algorithm) for |z| near 1
 static double2 julia_inv(double2 z) {
@@ -1041,6 +1047,36 @@ static int make_twolevel(cfft_plan_s* P, int64_t N, TwoLevel& t) {
     t.hi = (const double2*)d + lo_n;
     t.bits = bits;
     t.N = (int)N;
+    return CFFT_OK;
+}
+// table of w_n^e, e <= n / 4, for the real transforms: at most 4097 high entries
+static int make_root(cfft_plan_s* P, int64_t n, RootTable& t) {
+    const int64_t last = n / 4;
+    int bits = 0;
+    while ((last >> bits) > 4096) bits++;
+    const int64_t lo_n = 1LL << bits, hi_n = (last >> bits) + 1;
+    const void* d = nullptr;
+    int rc = cached_table(P, "rt/" + std::to_string(n), [&](std::vector<unsigned char>& img) {
+        std::vector<double2> v(lo_n + 2 * hi_n);
+        long double c, s;
+        for (int64_t a = 0; a < lo_n; a++) {
+            // w^a - 1 = 2i sin(x/2) e^(ix/2): no cancellation
+            omega_l(a, 2 * n, -1, &c, &s);
+            v[a] = make_double2((double)(-2 * s * s), (double)(2 * s * c));
+        }
+        for (int64_t b = 0; b < hi_n; b++) {
+            omega_l(b * lo_n, n, -1, &c, &s);
+            const double2 h = make_double2((double)c, (double)s);
+            v[lo_n + b] = h;
+            v[lo_n + hi_n + b] = make_double2((double)(c - h.x), (double)(s - h.y));
+        }
+        put(img, v);
+    }, &d);
+    if (rc) return rc;
+    t.lo1 = (const double2*)d;
+    t.hi = t.lo1 + lo_n;
+    t.hr = t.hi + hi_n;
+    t.bits = bits;
     return CFFT_OK;
 }
 
@@ -3729,7 +3765,7 @@ struct cfft_rplan_s {
     int64_t n = 0, batch = 0;
     int dtype = 0;
     cfft_plan_s* P = nullptr;
-    TwoLevel w = {};             // even n: table of w_n
+    RootTable w = {};            // even n: table of w_n
     void* scratch = nullptr;     // odd n: batch * n complex
     void* d_real = nullptr;      // host entry: device copies of the two sides
     void* d_cplx = nullptr;
@@ -3749,7 +3785,7 @@ int cfft_rfft_plan_create(cfft_rplan* plan, int64_t n, int64_t batch, int dtype,
     R->dtype = dtype;
     const bool even = (n % 2 == 0);
     int rc = plan_create_impl(&R->P, even ? n / 2 : n, batch, dtype, flags);
-    if (rc == CFFT_OK && even) rc = make_twolevel(R->P, n, R->w);
+    if (rc == CFFT_OK && even) rc = make_root(R->P, n, R->w);
     if (rc == CFFT_OK && !even) {
         if (lib_malloc(&R->scratch, (size_t)n * batch * elem_bytes(dtype)) != cudaSuccess) {
             cudaGetLastError();

@@ -21,11 +21,24 @@
 #include "kernels.h"
 
 // One thread per pair (k, N - k), k = 0 .. N/2: both of its elements are read
-// and written once.  w^k comes from the two-level FP64 table of w (lanes read
-// adjacent low entries and one high entry), and w^(N-k) = -conj(w^k), since
-// w^N = -1.  These sweeps are bandwidth bound: evaluating both twiddles of a
+// and written once.  w^k comes from a two-level FP64 table of w (lanes read
+// adjacent or the same entries), and w^(N-k) = -conj(w^k), since w^N = -1.  These sweeps are bandwidth bound: evaluating both twiddles of a
 // pair by sincospi, with 64-bit quotients per element, took 150 us for
 // 1024 x 24000 ComplexF32 (2.6 TB/s).
+// A product of two rounded table entries was off by up to 1.9e-16, sincospi by
+// 1.5e-16; this sum, whose last addition alone rounds at full size, by half an
+// ulp, 0.56e-16 (ComplexF32, without hi's rounding error: by 1.1e-16).
+template <typename V> __device__ __forceinline__ double2 root(const RootTable& w, int e) {
+    const double2 h = __ldg(w.hi + (e >> w.bits));
+    const double2 l = __ldg(w.lo1 + (e & ((1 << w.bits) - 1)));
+    double x = h.x * l.x - h.y * l.y, y = h.x * l.y + h.y * l.x;
+    if constexpr (sizeof(V) == 16) {
+        const double2 r = __ldg(w.hr + (e >> w.bits));
+        x += r.x;
+        y += r.y;
+    }
+    return make_double2(h.x + x, h.y + y);
+}
 // pair i of a launch -> transform t, pair k (half = N/2 + 1 pairs each)
 __device__ __forceinline__ bool pair_index(long long half, long long total, long long* t, int* k) {
     const long long base = (long long)blockIdx.x * blockDim.x;
@@ -45,7 +58,7 @@ __device__ __forceinline__ bool pair_index(long long half, long long total, long
     return base + threadIdx.x < total;
 }
 template <typename V>
-__global__ void __launch_bounds__(256) k_r2c_post(V* out, int N, TwoLevel w, long long half, long long total,
+__global__ void __launch_bounds__(256) k_r2c_post(V* out, int N, RootTable w, long long half, long long total,
                                                   long long dist) {
     long long t;
     int k;
@@ -62,13 +75,13 @@ __global__ void __launch_bounds__(256) k_r2c_post(V* out, int N, TwoLevel w, lon
     const double2 fe = make_double2(0.5 * (A.x + B.x), 0.5 * (A.y + B.y));
     // (A - B) / 2i = (Im(A - B) / 2, -Re(A - B) / 2)
     const double2 fo = make_double2(0.5 * (A.y - B.y), -0.5 * (A.x - B.x));
-    const double2 a = cmul(tw_two(w, (unsigned)k), fo);
+    const double2 a = cmul(root<V>(w, k), fo);
     X[k] = fromd<V>(make_double2(fe.x + a.x, fe.y + a.y));
     if (j != k) X[j] = fromd<V>(make_double2(fe.x - a.x, a.y - fe.y));
 }
 
 template <typename V>
-__global__ void __launch_bounds__(256) k_c2r_pre(const V* in, V* z, int N, TwoLevel w, long long half,
+__global__ void __launch_bounds__(256) k_c2r_pre(const V* in, V* z, int N, RootTable w, long long half,
                                                  long long total, long long in_dist, double scale) {
     long long t;
     int k;
@@ -83,7 +96,7 @@ __global__ void __launch_bounds__(256) k_c2r_pre(const V* in, V* z, int N, TwoLe
     const int j = N - k;
     const double2 A = tod(X[k]), B = conjv(tod(X[j]));
     const double2 fe = make_double2(A.x + B.x, A.y + B.y);
-    const double2 fo = cmul(make_double2(A.x - B.x, A.y - B.y), conjv(tw_two(w, (unsigned)k)));
+    const double2 fo = cmul(make_double2(A.x - B.x, A.y - B.y), conjv(root<V>(w, k)));
     // fe + i fo, and of N - k: conj(fe) + i conj(fo)
     Z[k] = fromd<V>(make_double2(scale * (fe.x - fo.y), scale * (fe.y + fo.x)));
     if (j != k) Z[j] = fromd<V>(make_double2(scale * (fe.x + fo.y), scale * (fo.x - fe.y)));
@@ -129,7 +142,7 @@ static unsigned grid_for(long long work) {
     return (unsigned)(g < 1 ? 1 : (g > 8192 ? 8192 : g));
 }
 
-cudaError_t cfft_r2c_post(void* out, long long N, const TwoLevel& w, long long batch, long long dist, int dtype,
+cudaError_t cfft_r2c_post(void* out, long long N, const RootTable& w, long long batch, long long dist, int dtype,
                           cudaStream_t st) {
     const long long half = N / 2 + 1, total = half * batch, grid = (total + 255) / 256;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -139,7 +152,7 @@ cudaError_t cfft_r2c_post(void* out, long long N, const TwoLevel& w, long long b
         k_r2c_post<float2><<<(unsigned)grid, 256, 0, st>>>((float2*)out, (int)N, w, half, total, dist);
     return cudaGetLastError();
 }
-cudaError_t cfft_c2r_pre(const void* in, void* z, long long N, const TwoLevel& w, long long batch,
+cudaError_t cfft_c2r_pre(const void* in, void* z, long long N, const RootTable& w, long long batch,
                          long long in_dist, double scale, int dtype, cudaStream_t st) {
     const long long half = N / 2 + 1, total = half * batch, grid = (total + 255) / 256;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
