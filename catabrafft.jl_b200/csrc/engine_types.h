@@ -107,11 +107,10 @@ struct KParams {
     void* out;
     long long in_dist, out_dist;  // elements between consecutive transforms
     int batch;                    // transforms in this launch
-    int units;                    // CTAs (ROWS/FOUR clusters) or tiles per transform
     int dir;                      // 0 forward, 1 inverse (scaled), 2 backward
     double scale;                 // 1/nx for dir 1, else 1
     // multiply-shift reciprocals (see fdiv) of the layout's divisors
-    unsigned long long mW, mN2, mR1, mX, mM, mL;
+    unsigned long long mW, mN2, mR1;
     int blk0;                     // first block of this parameter block in its launch
     unsigned char in_user, out_user;  // batched launches: in/out relative to the caller's buffers
     unsigned char in_fmt, out_fmt;    // IO_*: how in / out hold the caller's elements

@@ -311,7 +311,10 @@ struct Stage {
 };
 
 struct Shape {
-    int mode = MODE_ROWS;    // ROWS (LINE / LCONV), FOUR (CLUS without a convolution), COLPASS (the HBM passes), ...
+    // the family of a shape, not always the kernel's KParams.mode: MODE_ROWS is
+    // one CTA (LINE, or LCONV with a convolution), MODE_FOUR a cluster (CLUS, or
+    // with a convolution the FOUR kernels), MODE_COLPASS the HBM passes
+    int mode = MODE_ROWS;
     int conv = CONV_NONE;
     int64_t M = 0;
     int N1 = 1, N2 = 1, C = 1, V = 1;
@@ -1243,11 +1246,10 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
     }, &kp.spec);
 }
 
-// bytes of intermediate one chunk of a two-pass plan may use: 64 MB for the
-// generic passes (the intermediate then stays in the 126 MB L2) and 512 MB
-// for the power-of-two register passes (measured on B200 at 1 GiB batches:
-// fewer, longer persistent launches beat L2 residency by 7-20 %);
-// CFFT_SCRATCH_MB overrides both (read at plan creation)
+// bytes of intermediate a chunk may use under CFFT_SCRATCH_MB (read at plan
+// creation); without it 512 MB for the power-of-two register passes (measured on
+// B200 at 1 GiB batches: fewer, longer persistent launches beat L2 residency by
+// 7-20 %), while the generic passes follow pass_chunk
 static int64_t scratch_budget(bool pow2 = false) {
     const char* v = getenv("CFFT_SCRATCH_MB");
     const long long mb = v ? atoll(v) : 0;
@@ -1480,7 +1482,6 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         return CFFT_OK;
     }
     if (sh.mode == MODE_ROWS) {
-        kp.mode = MODE_ROWS;
         kp.V = sh.V;
         rc = make_sfplan(P, sh.M, kp.sc, true);
         if (rc) return rc;
@@ -1594,7 +1595,6 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
         kp.mW = magic(sh.N2 / sh.C);
         kp.mN2 = magic(sh.N2);
         kp.mR1 = magic(sh.N1 / sh.C);
-        kp.mX = magic(std::max(kp.XP, 1));
         rc = make_subplan(P, sh.N1, sh.ra, sh.N2 / sh.C, kp.pa, P->dtype == CFFT_C64);
         if (rc) return rc;
         rc = make_subplan(P, sh.N2, sh.rc, sh.N1 / sh.C, kp.pc, P->dtype == CFFT_C64);
@@ -3816,8 +3816,8 @@ int cfft_rfft_execute(cfft_rplan plan, const void* d_real, void* d_complex, void
     if (n % 2 == 0) {
         if (((uintptr_t)d_real % e) != 0 || ((uintptr_t)d_complex % e) != 0)
             return fail(CFFT_ERR_INVALID, "buffers must be aligned to the complex element size");
-        // chunk by chunk where the complex plan is: the sweep then finds the
-        // chunk's outputs in L2
+        // the sweep after each chunk of the complex plan (up to 512 MB: only
+        // small ones are still in L2)
         for (int64_t b0 = 0; b0 < R->batch; b0 += R->P->chunk) {
             const int64_t nb = std::min(R->P->chunk, R->batch - b0);
             char* out = (char*)d_complex + (size_t)b0 * h * e;
