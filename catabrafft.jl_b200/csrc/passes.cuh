@@ -37,10 +37,10 @@
 // earlier form staged the tile by cp.async and ran all stages from shared
 // memory with runtime divisions per wave: it spent twice the instructions
 // (issue slots are what bounds these kernels: 40 % ALU at 12 % of DRAM).
-// Measured on B200, before -> after, per launch of the whole plan: ComplexF32
-// 10^6 x 64 1367 -> 844 us, 3^10 x 512 528 -> 359, prime 999983 x 32 (a
-// four-pass convolution before) 3972 -> 1973, 100003 x 128 2039 -> 660;
-// ComplexF64 10^6 x 64 2537 -> 1541, 999983 x 32 8314 -> 3363.
+// Measured on B200, before it and now, per launch of the whole plan: ComplexF32
+// 10^6 x 64 1321 -> 659 us, 3^10 x 512 510 -> 309, prime 999983 x 32 (a four-pass
+// convolution before) 3822 -> 1329, 100003 x 128 1981 -> 494; ComplexF64 10^6 x 64
+// 2475 -> 1202, 999983 x 32 8172 -> 2267.
 // What a stage does per butterfly of radix R: R loads and R stores at a fixed
 // stride, one DFT_R codelet, R - 1 table twiddles (exactly rounded, read
 // through L1), and one or two small integer quotients.
@@ -57,7 +57,8 @@
 
 // R as a compile-time constant for each radix the planner uses (sf_search in
 // passplan.h); SF_SWITCH_LINE adds 18 and 20 for ComplexF32 (V of the enclosing
-// template) in LINE and LCONV
+// template) in LINE and COLS, and radix 1.  (SF_SWITCH_CONV, LCONV's, has that
+// case too: it is never reached, but without it the compiler spills twice as much)
 #define SF_CASES(CALL)              \
     case 2: CALL(2); break;         \
     case 3: CALL(3); break;         \
@@ -83,6 +84,12 @@
         case 18: if constexpr (sizeof(V) == 8) { CALL(18); } break; \
         case 20: if constexpr (sizeof(V) == 8) { CALL(20); } break; \
         default: CALL(16); break;                                 \
+    }
+#define SF_SWITCH_CONV(r, CALL)     \
+    switch (r) {                    \
+        SF_CASES(CALL)              \
+        case 1: CALL(1); break;     \
+        default: CALL(16); break;   \
     }
 #define SF_SWITCH_LAST(r, CALL)     \
     if ((r) == 1) { CALL(1); }      \
@@ -719,30 +726,30 @@ template <typename V> __device__ __forceinline__ void lconv_body(const KParams& 
         }
     }
 #define SF_CALL(R) lconv_first<V, R>(p, buf, t0, rows)
-    SF_SWITCH_LINE(S.r[0], SF_CALL)
+    SF_SWITCH_CONV(S.r[0], SF_CALL)
 #undef SF_CALL
     __syncthreads();
     int Ls = S.L / S.r[0];
     for (int s = 1; s < S.np - 1; s++) {
 #define SF_CALL(R) row_mid<V, R, false, false>(p, buf, s, Ls, rows)
-        SF_SWITCH_LINE(S.r[s], SF_CALL)
+        SF_SWITCH_CONV(S.r[s], SF_CALL)
 #undef SF_CALL
         __syncthreads();
         Ls /= S.r[s];
     }
 #define SF_CALL(R) mid_center<V, R, true>(p, buf, 0, rows)
-    SF_SWITCH_LINE(S.r[S.np - 1], SF_CALL)
+    SF_SWITCH_CONV(S.r[S.np - 1], SF_CALL)
 #undef SF_CALL
     __syncthreads();
     for (int s = S.np - 2; s >= 1; s--) {
         Ls *= S.r[s];
 #define SF_CALL(R) row_mid<V, R, false, true>(p, buf, s, Ls, rows)
-        SF_SWITCH_LINE(S.r[s], SF_CALL)
+        SF_SWITCH_CONV(S.r[s], SF_CALL)
 #undef SF_CALL
         __syncthreads();
     }
 #define SF_CALL(R) lconv_last<V, R>(p, buf, x0, t0, rows)
-    SF_SWITCH_LINE(S.r[0], SF_CALL)
+    SF_SWITCH_CONV(S.r[0], SF_CALL)
 #undef SF_CALL
     if (p.conv == CONV_RADER)
         for (int r = opaque_tid(); r < rows; r += CFFT_THREADS)

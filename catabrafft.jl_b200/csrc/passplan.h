@@ -16,9 +16,14 @@ static const int SF_SMS = 148;        // a B200's SMs, the only device this is b
 // layout keeps contiguous span a half-warp (the other way round a 24000-point
 // two-pass plan took 225 us against 212).  One stage becomes two (L, 1), as
 // the kernels always run a first and a last one.  Radices go up to maxr: 20 for
-// ComplexF32 in LINE and LCONV (50000 x 360 as 18 x 20 63 us, as 6 x 6 x 10
-// 86), 16 elsewhere (in the HBM passes 18 and 20 measured from 5 % faster to
-// 10 % slower, and 21 to 27 spill at 80 registers and lose 15 - 25 %).
+// ComplexF32 in LINE, at 8 bytes of spill (50000 x 360 as 18 x 20 63 us, as 6 x 6
+// x 10 86; of 28 lengths from 162 to 8000 all are 2 - 38 % faster with them at
+// full batches but 3600, 13 % slower), and so in COLS, which repeats LINE's
+// arithmetic (884 bytes of spill stores, 260 without; from 24 % faster, 400 x
+// 3000, to 6 % slower, 6000 x 1000); 16 elsewhere: in LCONV 18 and 20 spill 816
+// bytes (144 without) and are slower throughout, 181 x 1 13.6 us (6.2 without),
+// 3001 x 1 33.1 (23.2), x 4000 437 (376); in the HBM passes they measured from 5 %
+// faster to 10 % slower, and 21 to 27 spill at 80 registers and lose 15 - 25 %
 inline double sf_radix_cost(int r) {
     // real additions and multiplications per point of the codelets
     switch (r) {

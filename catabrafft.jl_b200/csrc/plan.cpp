@@ -411,8 +411,8 @@ static const SfPlan* sf_get(int64_t L) {
     }();
     return L >= 1 && L <= kSfMax && tab[L].L ? &tab[L] : nullptr;
 }
-// ... and of every length LINE and LCONV use
-static const SfPlan* sf_line(int64_t L, int dtype) {
+// ... and of every length LINE (wide: ComplexF32 radices up to 20) and LCONV use
+static const SfPlan* sf_line(int64_t L, int dtype, bool wide) {
     static const std::vector<SfPlan> tab = [] {
         std::vector<SfPlan> t(2 * (kLineMax + 1));
         for (int l = 1; l <= kLineMax; l++)
@@ -423,7 +423,7 @@ static const SfPlan* sf_line(int64_t L, int dtype) {
         return t;
     }();
     if (L < 1 || L > kLineMax) return nullptr;
-    const SfPlan* S = &tab[(dtype == CFFT_C128 ? 0 : kLineMax + 1) + L];
+    const SfPlan* S = &tab[(dtype == CFFT_C128 || !wide ? 0 : kLineMax + 1) + L];
     return S->L ? S : nullptr;
 }
 static std::vector<int> sf_radices(const SfPlan& S) { return std::vector<int>(S.r, S.r + S.np); }
@@ -434,7 +434,7 @@ static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch
     if (M > kLineMax) return false;
     sh.mode = MODE_ROWS;
     if (conv == CONV_NONE) {
-        const SfPlan* S = sf_line(M, dtype);
+        const SfPlan* S = sf_line(M, dtype, true);
         if (!S || sf_line_smem(*S, 1, e) > sf_budget(e)) return false;
         sh.M = M;
         // one row a CTA where the n = 4096 register kernel runs it
@@ -445,7 +445,7 @@ static bool rows_shape(int64_t M, int64_t nx, int conv, int dtype, int64_t batch
     }
     double best = 1e300;
     for (int64_t m = M; m <= M + M / 50 && m <= kLineMax; m++) {
-        const SfPlan* S = sf_line(m, dtype);
+        const SfPlan* S = sf_line(m, dtype, false);
         if (!S || !sf_mid_fits(*S) || sf_lconv_smem(*S, 1, e) > sf_budget(e)) continue;
         double c;
         const int V = sf_lconv_rows(*S, batch, e, &c);
@@ -1013,12 +1013,12 @@ static int make_subplan(cfft_plan_s* P, int64_t L, const std::vector<int>& rad, 
     }, &sp.tw);
 }
 // sub-transform of the passes with its twiddle blocks (SfPlan.off / .boff)
-static int make_sfplan(cfft_plan_s* P, int64_t L, SfPlan& S, bool line = false) {
-    const SfPlan* q = line ? sf_line(L, P->dtype) : sf_get(L);
+static int make_sfplan(cfft_plan_s* P, int64_t L, SfPlan& S, bool line = false, bool wide = false) {
+    const SfPlan* q = line ? sf_line(L, P->dtype, wide) : sf_get(L);
     if (!q) return fail(CFFT_ERR_UNSUPPORTED, "no radix sequence for " + std::to_string(L));
     S = *q;
     const int dtype = P->dtype;
-    return cached_table(P, "sf/" + std::to_string(dtype) + (line ? "l/" : "/") + std::to_string(L), [&](std::vector<unsigned char>& img) {
+    return cached_table(P, "sf/" + std::to_string(dtype) + (line ? wide ? "l/" : "c/" : "/") + std::to_string(L), [&](std::vector<unsigned char>& img) {
         std::vector<double2> w(std::max(1, q->twall));
         for (int i = 0; i < q->twall; i++) {
             long long e;
@@ -1220,7 +1220,7 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
         const int* iperm = kp.iperm;
         *spec_key = "sr/" + tag + "/" + std::to_string(exact);
         if (sh.mode == MODE_ROWS)
-            return conv_spectrum_rows(P, *spec_key + "/c" + std::to_string(P->dtype), 1, *sf_line(M, P->dtype), [&](double2* v) {
+            return conv_spectrum_rows(P, *spec_key + "/c" + std::to_string(P->dtype), 1, *sf_line(M, P->dtype, false), [&](double2* v) {
                 return cfft_gen_rader_b(v, iperm, n, M, exact, winv, 0);
             }, &kp.spec);
         return conv_spectrum(P, *spec_key, M, [&](double2* v) {
@@ -1238,7 +1238,7 @@ static int make_conv_tables(cfft_plan_s* P, const Shape& sh, KParams& kp, std::s
     const double2* ch = kp.chirp;
     if (sh.mode == MODE_COLPASS || sh.mode == MODE_ROWS)
         return conv_spectrum_rows(P, "sc/" + tag + "/" + std::to_string(P->dtype) + "/" + std::to_string(sh.mode == MODE_ROWS ? 1 : sh.N1),
-                                  sh.mode == MODE_ROWS ? 1 : sh.N1, sh.mode == MODE_ROWS ? *sf_line(sh.M, P->dtype) : *sf_get(sh.N2),
+                                  sh.mode == MODE_ROWS ? 1 : sh.N1, sh.mode == MODE_ROWS ? *sf_line(sh.M, P->dtype, false) : *sf_get(sh.N2),
                                   [&](double2* v) { return cfft_gen_bluestein_b(v, ch, n, M, 0); }, &kp.spec);
     *spec_key = "sb/" + tag;
     return conv_spectrum(P, *spec_key, M, [&](double2* v) {
@@ -1483,7 +1483,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     }
     if (sh.mode == MODE_ROWS) {
         kp.V = sh.V;
-        rc = make_sfplan(P, sh.M, kp.sc, true);
+        rc = make_sfplan(P, sh.M, kp.sc, true, sh.conv == CONV_NONE);
         if (rc) return rc;
         if (sh.conv == CONV_NONE) {
             // V rows per CTA in register stages (passes.cuh), or the persistent

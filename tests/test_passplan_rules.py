@@ -97,3 +97,12 @@ def test_one_long_transform(n, expect):
 def test_one_long_prime(n, expect):
     # one ComplexF64 prime: on a cluster where that is shorter than one CTA
     assert expect in load().describe_strategy(n), load().describe_strategy(n)
+
+
+def test_convolutions_use_radices_up_to_16():
+    # 18 and 20 pay in LINE; in LCONV they made every convolution slower
+    m = load()
+    for n in (163, 181, 1511, 2503, 2506, 3001, 4001):
+        d = m.describe_strategy(n, "complex64")
+        assert "rows(" in d and max(int(x) for x in d[d.rindex("[") + 1:-1].split(",")) <= 16, d
+    assert m.describe_strategy(360, "complex64").endswith("[18,20]")
