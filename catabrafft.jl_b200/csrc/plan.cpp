@@ -1012,19 +1012,34 @@ static int make_subplan(cfft_plan_s* P, int64_t L, const std::vector<int>& rad, 
         }
     }, &sp.tw);
 }
-// sub-transform of the passes with its twiddle blocks (SfPlan.off / .boff)
-static int make_sfplan(cfft_plan_s* P, int64_t L, SfPlan& S, bool line = false, bool wide = false) {
-    const SfPlan* q = line ? sf_line(L, P->dtype, wide) : sf_get(L);
+// roots w_L^e, e < L: half of them by omega, the others their conjugates
+static std::vector<double2> roots_of(int64_t L) {
+    std::vector<double2> w(L);
+    for (int64_t e = 0; 2 * e <= L; e++) {
+        w[e] = omega(e, L, -1);
+        if (e > 0) w[L - e] = make_double2(w[e].x, -w[e].y);
+    }
+    return w;
+}
+// sub-transform of the passes with its twiddle blocks: the forward ones, and for
+// a convolution's rows (conv) the second transform's too (SfPlan.off / .boff).
+// Every entry is a root of L.  One sine and cosine per entry of both blocks made
+// planning a large part of a first call: 4096 points 0.97 ms
+static int make_sfplan(cfft_plan_s* P, int64_t L, SfPlan& S, bool line, bool conv) {
+    const SfPlan* q = line ? sf_line(L, P->dtype, !conv) : sf_get(L);
     if (!q) return fail(CFFT_ERR_UNSUPPORTED, "no radix sequence for " + std::to_string(L));
     S = *q;
     const int dtype = P->dtype;
-    return cached_table(P, "sf/" + std::to_string(dtype) + (line ? wide ? "l/" : "c/" : "/") + std::to_string(L), [&](std::vector<unsigned char>& img) {
-        std::vector<double2> w(std::max(1, q->twall));
-        for (int i = 0; i < q->twall; i++) {
+    const std::string key = "sf/" + std::to_string(dtype) + (line ? "l" : "p") + (conv ? "c/" : "/") + std::to_string(L);
+    return cached_table(P, key, [&](std::vector<unsigned char>& img) {
+        const int len = conv ? q->twall : q->twlen;
+        const std::vector<double2> root = roots_of(L);
+        std::vector<double2> w(std::max(1, len), make_double2(1, 0));
+        for (int i = 0; i < len; i++) {
             long long e;
             int N;
             sf_tw_entry(*q, i, &e, &N);
-            w[i] = omega(e, N, -1);
+            w[i] = root[e % N * (L / N)];
         }
         if (dtype == CFFT_C128) {
             put(img, w);
@@ -1483,7 +1498,7 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     }
     if (sh.mode == MODE_ROWS) {
         kp.V = sh.V;
-        rc = make_sfplan(P, sh.M, kp.sc, true, sh.conv == CONV_NONE);
+        rc = make_sfplan(P, sh.M, kp.sc, true, sh.conv != CONV_NONE);
         if (rc) return rc;
         if (sh.conv == CONV_NONE) {
             // V rows per CTA in register stages (passes.cuh), or the persistent
@@ -1540,9 +1555,9 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     }
     if (sh.mode == MODE_FOUR && sh.conv == CONV_NONE) {
         const int T = clus_threads(P->dtype), R1 = sh.N1 / sh.C;
-        rc = make_sfplan(P, sh.N1, kp.sa);
+        rc = make_sfplan(P, sh.N1, kp.sa, false, false);
         if (rc) return rc;
-        rc = make_sfplan(P, sh.N2, kp.sc);
+        rc = make_sfplan(P, sh.N2, kp.sc, false, false);
         if (rc) return rc;
         rc = make_twolevel(P, sh.M, kp.t4);
         if (rc) return rc;
@@ -1772,9 +1787,9 @@ static int plan_build(cfft_plan_s* P, const Shape& sh) {
     }
     // HBM passes (passes.cuh) over one intermediate
     const int64_t N1 = sh.N1, N2 = sh.N2, M = sh.M;
-    rc = make_sfplan(P, N1, kp.sa);
+    rc = make_sfplan(P, N1, kp.sa, false, false);
     if (rc) return rc;
-    rc = make_sfplan(P, N2, kp.sc);
+    rc = make_sfplan(P, N2, kp.sc, false, sh.conv != CONV_NONE);
     if (rc) return rc;
     if (sh.conv != CONV_NONE && !sf_mid_fits(kp.sc))
         return fail(CFFT_ERR_UNSUPPORTED, "convolution rows of one radix: " + std::to_string(N2));
