@@ -82,30 +82,6 @@ static cudaError_t lib_free_host(void* p) {
     g_live_allocs.fetch_sub(1);
     return cudaFreeHost(p);
 }
-// a temporary in stream order (a cudaMalloc / cudaFree pair waits for the
-// device), or a plain allocation where the device has no memory pools
-template <class T> static cudaError_t lib_malloc_ordered(T** p, size_t bytes, cudaStream_t st, bool* ordered) {
-    *ordered = true;
-    if (alloc_injected_failure()) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-    }
-    cudaError_t e = cudaMallocAsync((void**)p, bytes, st);
-    if (e == cudaErrorNotSupported) {
-        cudaGetLastError();
-        *ordered = false;
-        e = cudaMalloc((void**)p, bytes);
-    }
-    if (e == cudaSuccess) g_live_allocs.fetch_add(1);
-    else *p = nullptr;
-    return e;
-}
-static cudaError_t lib_free_ordered(void* p, cudaStream_t st, bool ordered) {
-    if (!ordered) return lib_free(p);
-    if (!p) return cudaSuccess;
-    g_live_allocs.fetch_sub(1);
-    return cudaFreeAsync(p, st);
-}
 
 #define CUDA_TRY(call)                                                                     \
     do {                                                                                   \
@@ -1137,12 +1113,14 @@ static int cached_dev_table(cfft_plan_s* P, const std::string& key0, size_t byte
     return CFFT_OK;
 }
 
-// smooth FP64 plans (batch 1) that transform convolution kernel vectors,
-// cached per (device, M)
+// Building a convolution's spectrum uses a cached smooth FP64 plan (batch 1) per
+// (device, M) and a buffer, both shared by all threads: a build holds g_spec_mu
+// from looking them up to the end of its work on the default stream
 static std::mutex g_spec_mu;
 static std::map<std::pair<int, int64_t>, cfft_plan_s*> g_spec_plans;
+static std::map<int, DevPtr> g_spec_tmp;
+static const size_t kSpecTmpKeep = (size_t)32 << 20;
 static int spectrum_plan(int dev, int64_t M, cfft_plan_s** out) {
-    std::lock_guard<std::mutex> lk(g_spec_mu);
     auto it = g_spec_plans.find({dev, M});
     if (it != g_spec_plans.end()) { *out = it->second; return CFFT_OK; }
     cfft_plan_s* S = nullptr;
@@ -1155,14 +1133,15 @@ static int spectrum_plan(int dev, int64_t M, cfft_plan_s** out) {
 // spectrum = FFT_M(b') / M in FP64, b' generated in place by `gen`
 template <class G>
 static int conv_spectrum(cfft_plan_s* P, const std::string& key, int64_t M, G gen, const double2** out) {
-    cfft_plan_s* S = nullptr;
-    int rc = spectrum_plan(P->device, M, &S);
-    if (rc) return rc;
     const void* d = nullptr;
-    rc = cached_dev_table(P, key, (size_t)M * sizeof(double2), [&](void* dp) -> int {
+    std::lock_guard<std::mutex> lk(g_spec_mu);
+    int rc = cached_dev_table(P, key, (size_t)M * sizeof(double2), [&](void* dp) -> int {
+        cfft_plan_s* S = nullptr;
+        int r = spectrum_plan(P->device, M, &S);
+        if (r) return r;
         double2* v = (double2*)dp;
         CUDA_TRY(gen(v));
-        int r = plan_execute(S, v, v, CFFT_FORWARD, 0);
+        r = plan_execute(S, v, v, CFFT_FORWARD, 0);
         if (r) return r;
         CUDA_TRY(cfft_scale(v, M, 1.0 / (double)M, 0));
         return CFFT_OK;
@@ -1172,30 +1151,35 @@ static int conv_spectrum(cfft_plan_s* P, const std::string& key, int64_t M, G ge
 }
 
 // the spectrum in MIDPASS's order (mid_center), which alone is kept: the
-// natural-order one is built in a temporary buffer
+// natural-order one is built in a buffer, kept up to 32 MB until cfft_empty_cache
+// (an allocation per length was half of the time to plan a batch of many lengths)
 template <class G>
 static int conv_spectrum_rows(cfft_plan_s* P, const std::string& key, int64_t N1, const SfPlan& S, G gen,
                               const double2** out) {
     const int64_t M = N1 * S.L;
-    cfft_plan_s* F = nullptr;
-    int rc = spectrum_plan(P->device, M, &F);
-    if (rc) return rc;
+    const size_t bytes = (size_t)M * sizeof(double2);
     const void* d = nullptr;
-    rc = cached_dev_table(P, key, (size_t)M * sizeof(double2), [&](void* dp) -> int {
-        // stream-ordered: a cudaMalloc / cudaFree pair per length was half of
-        // the time to plan a batch of many lengths
-        double2* v = nullptr;
-        bool ordered;
-        cudaError_t ce = lib_malloc_ordered(&v, (size_t)M * sizeof(double2), 0, &ordered);
-        if (ce != cudaSuccess) cudaGetLastError();
-        CUDA_TRY(ce);
-        ce = gen(v);
-        int r = CFFT_OK;
-        if (ce == cudaSuccess) r = plan_execute(F, v, v, CFFT_FORWARD, 0);
-        if (ce == cudaSuccess && !r) ce = cfft_spec_center((double2*)dp, v, N1, S, 1.0 / (double)M, 0);
-        lib_free_ordered(v, 0, ordered);
-        CUDA_TRY(ce);
-        return r;
+    std::lock_guard<std::mutex> lk(g_spec_mu);
+    int rc = cached_dev_table(P, key, bytes, [&](void* dp) -> int {
+        cfft_plan_s* F = nullptr;
+        int r = spectrum_plan(P->device, M, &F);
+        if (r) return r;
+        DevPtr big;                             // freed below, which waits for the device
+        DevPtr& tmp = bytes <= kSpecTmpKeep ? g_spec_tmp[P->device] : big;
+        if (!tmp || tmp->bytes < bytes) {
+            tmp.reset();
+            const size_t step = bytes <= kSpecTmpKeep / 8 ? kSpecTmpKeep / 8 : kSpecTmpKeep;
+            if (bytes > kSpecTmpKeep || dev_alloc(step, &tmp) != CFFT_OK) {
+                r = dev_alloc(bytes, &tmp);
+                if (r) return r;
+            }
+        }
+        double2* v = (double2*)tmp->p;
+        CUDA_TRY(gen(v));
+        r = plan_execute(F, v, v, CFFT_FORWARD, 0);
+        if (r) return r;
+        CUDA_TRY(cfft_spec_center((double2*)dp, v, N1, S, 1.0 / (double)M, 0));
+        return CFFT_OK;
     }, &d);
     *out = (const double2*)d;
     return rc;
@@ -3447,6 +3431,7 @@ int cfft_empty_cache(void) {
     }
     {
         std::lock_guard<std::mutex> lk(g_spec_mu);
+        g_spec_tmp.clear();
         for (auto& kv : g_spec_plans) {
             plan_free(kv.second);
             delete kv.second;
