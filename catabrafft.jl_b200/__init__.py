@@ -86,6 +86,9 @@ class _Plan:
         h = ctypes.c_void_p()
         check(_lib.LIB.cfft_plan_create(ctypes.byref(h), n, batch, dtype, flags))
         self.handle = h
+        # device memory that its executions share (ComplexF16 plans may hold a working copy)
+        self.scratch = dtype == C32 or _lib.LIB.cfft_plan_workspace_bytes(h) > 0
+        self.stream = None            # the one that uses it (_for_stream)
 
     def describe(self) -> str:
         buf = ctypes.create_string_buffer(512)
@@ -110,14 +113,36 @@ def _current_device(x=None) -> int:
     return 0
 
 
-def _get_plan(n, batch, dtype, flags, device) -> _Plan:
-    key = (device, n, batch, dtype, flags)
-    with _cache_lock:
-        p = _plans.get(key)
-        if p is None:
-            p = _Plan(n, batch, dtype, flags, device)
-            _plans[key] = p
+def _for_stream(cache, key, stream, make):
+    """The cached plan of `key` for work on `stream` (None: not known yet).  A plan
+    with scratch belongs to the first stream that runs it; another stream gets a
+    plan of its own, as two executions at once would share the scratch.  A
+    stream under capture, where nothing can be allocated, takes the first one.
+    The caller holds _cache_lock."""
+    p = cache.get(key)
+    if p is None:
+        p = cache[key] = make()
+    if stream is None or not p.scratch:
         return p
+    if p.stream is None:
+        p.stream = stream
+    if p.stream != stream:
+        if stream != "host":
+            import torch
+            if torch.cuda.is_current_stream_capturing():
+                return p
+        key = (*key, "stream", stream)
+        p = cache.get(key)
+        if p is None:
+            p = cache[key] = make()
+            p.stream = stream
+    return p
+
+
+def _get_plan(n, batch, dtype, flags, device, stream=None) -> _Plan:
+    with _cache_lock:
+        return _for_stream(_plans, (device, n, batch, dtype, flags), stream,
+                           lambda: _Plan(n, batch, dtype, flags, device))
 
 
 def _shape(x):
@@ -140,9 +165,9 @@ def _run(x, direction: int, flags: int = NO_FLAG, out=None):
             y = torch.empty_like(xc) if out is None else out
             if batch == 0:
                 return y
-            plan = _get_plan(n, batch, dt, flags, x.device.index)
             stream = torch.cuda.current_stream(x.device).cuda_stream
             with torch.cuda.device(x.device):
+                plan = _get_plan(n, batch, dt, flags, x.device.index, stream)
                 check(_lib.LIB.cfft_execute(plan.handle, ctypes.c_void_p(xc.data_ptr()),
                                             ctypes.c_void_p(y.data_ptr()), direction,
                                             ctypes.c_void_p(stream)))
@@ -159,7 +184,7 @@ def _run(x, direction: int, flags: int = NO_FLAG, out=None):
     y = np.empty_like(a) if out is None else out
     if batch == 0:
         return y
-    plan = _get_plan(n, batch, dt, flags, 0)
+    plan = _get_plan(n, batch, dt, flags, 0, "host")
     check(_lib.LIB.cfft_execute_host(plan.handle, a.ctypes.data_as(ctypes.c_void_p),
                                      y.ctypes.data_as(ctypes.c_void_p), direction))
     return y
@@ -192,20 +217,16 @@ def _run_axis(x, direction: int, axis: int):
         y = torch.empty_like(xc)
         dt = _dtype_code(xc.dtype)
         e = 16 if dt == C128 else 8
-        key = ("many", xc.device.index, n, inner, dt)
-        with _cache_lock:
-            h = _plans.get(key)
-            if h is None:
-                hp = ctypes.c_void_p()
-                check(_lib.LIB.cfft_plan_create_many(ctypes.byref(hp), n, inner, dt, NO_FLAG, inner, 1, inner, 1))
-                h = _ManyPlan(hp)
-                _plans[key] = h
-        stream = ctypes.c_void_p(torch.cuda.current_stream(xc.device).cuda_stream)
+        stream = torch.cuda.current_stream(xc.device).cuda_stream
         with torch.cuda.device(xc.device):
+            with _cache_lock:
+                h = _for_stream(_plans, ("many", xc.device.index, n, inner, dt), stream,
+                                lambda: _ManyPlan(n, inner, dt))
             for o in range(outer):
                 off = o * n * inner * e
                 check(_lib.LIB.cfft_execute(h.handle, ctypes.c_void_p(xc.data_ptr() + off),
-                                            ctypes.c_void_p(y.data_ptr() + off), direction, stream))
+                                            ctypes.c_void_p(y.data_ptr() + off), direction,
+                                            ctypes.c_void_p(stream)))
         return y
     if _is_torch(x):
         import torch
@@ -215,8 +236,17 @@ def _run_axis(x, direction: int, axis: int):
 
 
 class _ManyPlan:
-    def __init__(self, handle):
-        self.handle = handle
+    """`inner` strided transforms side by side."""
+
+    def __init__(self, n, inner, dtype):
+        h = ctypes.c_void_p()
+        check(_lib.LIB.cfft_plan_create_many(ctypes.byref(h), n, inner, dtype, NO_FLAG, inner, 1, inner, 1))
+        self.handle = h
+        buf = ctypes.create_string_buffer(512)
+        check(_lib.LIB.cfft_plan_describe(h, buf, 512))
+        # (unfused strided plans gather into a working copy)
+        self.scratch = buf.value.startswith(b"strided+") or _lib.LIB.cfft_plan_workspace_bytes(h) > 0
+        self.stream = None
 
     def destroy(self):
         if self.handle:
@@ -324,10 +354,11 @@ class Spell:
             import torch
             plan, index = self._plan, self.device
             if plan.handle is not None and x.get_device() == index and torch.cuda.current_device() == index:
-                y = torch.empty_like(x)
-                check(_lib.LIB.cfft_execute(plan.handle, x.data_ptr(), y.data_ptr(), self.direction,
-                                            _stream_handle(index)))
-                return y
+                stream = _stream_handle(index)
+                if not plan.scratch or plan.stream == stream:
+                    y = torch.empty_like(x)
+                    check(_lib.LIB.cfft_execute(plan.handle, x.data_ptr(), y.data_ptr(), self.direction, stream))
+                    return y
         self._check(x)
         return _run(x, self.direction, self.flag)
 
@@ -548,6 +579,7 @@ class _RPlan:
         h = ctypes.c_void_p()
         check(_lib.LIB.cfft_rfft_plan_create(ctypes.byref(h), n, batch, dtype, flags))
         self.handle, self.n, self.batch, self.dtype = h, n, batch, dtype
+        self.scratch, self.stream = True, None      # (its complex plan's, or the widened copy of odd lengths)
 
     def destroy(self):
         if self.handle:
@@ -555,14 +587,9 @@ class _RPlan:
             self.handle = None
 
 
-def _get_rplan(n, batch, dtype, flags, device):
-    key = (device, n, batch, dtype, flags)
+def _get_rplan(n, batch, dtype, flags, device, stream):
     with _cache_lock:
-        p = _rplans.get(key)
-        if p is None:
-            p = _RPlan(n, batch, dtype, flags)
-            _rplans[key] = p
-        return p
+        return _for_stream(_rplans, (device, n, batch, dtype, flags), stream, lambda: _RPlan(n, batch, dtype, flags))
 
 
 def _rrun(x, n, direction, flags=NO_FLAG):
@@ -579,9 +606,10 @@ def _rrun(x, n, direction, flags=NO_FLAG):
         if xc.dim() == 2:
             shp = (rows,) + shp
         y = torch.empty(shp, dtype=cdt if fwd else rdt, device=xc.device)
-        plan = _get_rplan(n, rows, dt, flags, xc.device.index)
-        stream = ctypes.c_void_p(torch.cuda.current_stream(xc.device).cuda_stream)
+        raw = torch.cuda.current_stream(xc.device).cuda_stream
+        stream = ctypes.c_void_p(raw)
         with torch.cuda.device(xc.device):
+            plan = _get_rplan(n, rows, dt, flags, xc.device.index, raw)
             if fwd:
                 check(_lib.LIB.cfft_rfft_execute(plan.handle, ctypes.c_void_p(xc.data_ptr()),
                                                  ctypes.c_void_p(y.data_ptr()), stream))
@@ -606,7 +634,7 @@ def _rrun(x, n, direction, flags=NO_FLAG):
         shp = (rows,) + shp
     y = np.empty(shp, dtype=(np.complex128 if dt == C128 else np.complex64) if fwd
                  else (np.float64 if dt == C128 else np.float32))
-    plan = _get_rplan(n, rows, dt, flags, 0)
+    plan = _get_rplan(n, rows, dt, flags, 0, "host")
     check(_lib.LIB.cfft_rfft_execute_host(plan.handle, a.ctypes.data_as(ctypes.c_void_p),
                                           y.ctypes.data_as(ctypes.c_void_p), direction))
     return y

@@ -351,6 +351,8 @@ struct cfft_plan_s {
     bool io_fused = false;
     int in_fmt = IO_PLAIN, out_fmt = IO_PLAIN;
     void* half_dev = nullptr;    // host entry: device copy of the ComplexF16 data
+    bool owned = false;          // cfft_fft's cache: the stream that runs it (plans with scratch)
+    void* owner = nullptr;
     int* flow_ctr = nullptr;     // dataflow plans: ticket, abort flag, per-transform counters (2 + 2 batch ints)
 };
 
@@ -3107,6 +3109,8 @@ static int serve_create_impl(cfft_server_s* S, int dtype, int64_t max_inflight_b
 // ------------------------------------------------------------------- C ABI
 static std::mutex g_cache_mu;
 static std::map<std::tuple<int, int64_t, int64_t, int, int>, cfft_plan_s*> g_cache;
+// plans with scratch belong to the first stream that runs them; those of others
+static std::map<std::tuple<int, int64_t, int64_t, int, int, void*>, cfft_plan_s*> g_cache_streams;
 
 extern "C" {
 
@@ -3415,6 +3419,26 @@ int cfft_fft(int64_t n, int64_t batch, int dtype, int flags, const void* d_in, v
             if (rc) return rc;
             g_cache[key] = P;
         }
+        if (P->scratch[0] || P->half_work) {
+            if (!P->owned) {
+                P->owned = true;
+                P->owner = stream;
+            }
+            // (nothing can be allocated under capture, which takes the first one)
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            if (P->owner != stream &&
+                cudaStreamIsCapturing((cudaStream_t)stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
+                auto skey = std::make_tuple(dev, n, batch, dtype, flags, stream);
+                auto is = g_cache_streams.find(skey);
+                if (is != g_cache_streams.end()) {
+                    P = is->second;
+                } else {
+                    int rc = plan_create_impl(&P, n, batch, dtype, flags);
+                    if (rc) return rc;
+                    g_cache_streams[skey] = P;
+                }
+            }
+        }
     }
     return cfft_execute(P, d_in, d_out, direction, stream);
 }
@@ -3428,6 +3452,11 @@ int cfft_empty_cache(void) {
             delete kv.second;
         }
         g_cache.clear();
+        for (auto& kv : g_cache_streams) {
+            plan_free(kv.second);
+            delete kv.second;
+        }
+        g_cache_streams.clear();
     }
     {
         std::lock_guard<std::mutex> lk(g_spec_mu);
