@@ -89,7 +89,9 @@ int cfft_plan_create_many(cfft_plan* plan, int64_t n, int64_t batch, int dtype, 
 int cfft_plan_destroy(cfft_plan plan);
 
 /* One-call form with an internal plan cache keyed by (n, batch, dtype,
- * flags), mirroring fft_kernel!'s cached lookup (src/kernel.jl:72-100). */
+ * flags), mirroring fft_kernel!'s cached lookup (src/kernel.jl:72-100).  Plans
+ * with scratch are kept per stream (a stream under capture takes the first
+ * one's), so that calls on several streams do not share it. */
 int cfft_fft(int64_t n, int64_t batch, int dtype, int flags, const void* d_in, void* d_out,
              int direction, void* stream);
 
