@@ -87,7 +87,7 @@
     }
 // ComplexF64 takes LINE's switch, where 18 and 20 are empty cases: with the same
 // registers and spills the compiler's code without them measured slower (97 x 1
-// 7.2 us, 6.3 with; 2018 x 128 16.7, 16.2; at most 1 % the other way, 2503 x 8)
+// 7.2 us, 6.3 with; 2018 x 128 16.7, 16.2; 2503 x 8 the other way, 32.1, 32.7)
 #define SF_SWITCH_CONV(r, CALL)     \
     if constexpr (sizeof(V) == 16) { SF_SWITCH_LINE(r, CALL) } \
     else switch (r) {               \
